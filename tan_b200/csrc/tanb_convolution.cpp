@@ -1443,7 +1443,7 @@ int32_t init_impl(tanb_convolution* v, uint32_t method, uint32_t L, uint32_t B, 
   }
   std::memset(v->h_stage, 0, stage_bytes);
   std::vector<float2> tw(2 * Bs);
-  tanb::make_twiddles(2 * B, tw.data());
+  tanb::make_plan_twiddles(log2B, tw.data());
   e = cudaMemcpyAsync(v->d_tw, tw.data(), tw.size() * sizeof(float2), cudaMemcpyHostToDevice, v->stream);
   if (e == cudaSuccess) e = cudaEventRecord(v->ev_stage, v->stream);
   if (e == cudaSuccess) e = cudaEventRecord(v->ev_ir, v->stream);

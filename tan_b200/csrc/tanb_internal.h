@@ -85,7 +85,7 @@ struct DevState {
   float2* fdl;    // delay line      [C][P][B]  (slot (cur + i) mod P holds X_{k-i})
   float* prev;    // previous input  [C][B]     (overlap-save history)
   float2* tail;   // tails           [C][2][B]  ([0]: active IR, [1]: pending IR)
-  const float2* tw;  // W_N^j, N = 2B, j in [0, N)
+  const float2* tw;  // twiddles of the B-point register transform (2B entries)
   int* err;       // device-visible error word (host-mapped); nonzero after a
                   // bounded wait in a kernel gave up (kErr* codes)
   int wait_limit = kBulkWaitLimit;  // polls of a bounded wait for a pipeline
@@ -252,5 +252,9 @@ cudaError_t prepare_kernels();
 // Fills the twiddle table W_N^j = exp(-2 pi i j / N) on the host, computed in
 // double and rounded to float, exact at multiples of pi/2.
 void make_twiddles(int N, float2* out);
+
+// Fills the table of the M = 2^log2M register transform (tanb_fft_reg.cuh):
+// 2M entries, values of make_twiddles(2M) in the order the passes read them.
+void make_plan_twiddles(int log2M, float2* out);
 
 }  // namespace tanb

@@ -14,11 +14,13 @@
 // (tan/tanlibrary/src/TrueAudioNext/convolution/ConvolutionImpl.cpp:2380-2643);
 // overlap-save needs no overlap buffer and gives the exact new-IR output on a
 // swap block from the same delay line.
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <utility>
+#include <vector>
 
-#include "tanb_fft.cuh"
+#include "tanb_fft_reg.cuh"
 #include "tanb_internal.h"
 
 namespace tanb {
@@ -106,232 +108,121 @@ struct CtlDesc {
 };
 
 
+// R2C of each IR partition: z[n] = (h[t0 + 2n], h[t0 + 2n + 1]) for n < M / 2,
+// zero above, through register passes (tanb_fft_reg.cuh). THREADS / T transforms
+// run side by side in a CTA and each group of T threads takes several partitions
+// of its channel in turn, so that the stage twiddles are loaded into registers
+// once and the next partition's samples while the present one is transformed.
+// The kernel is bound by the shared-memory pipe and the barriers rather than by
+// the 12 bytes a sample it moves: with one partition per group, twiddles in
+// shared memory and CTA-wide barriers it took 22 us for 8192 partitions of 512
+// (50 MB).
 template <int LOG2M>
-__global__ void __launch_bounds__(FftShape<LOG2M>::T)
-    ir_spectrum_kernel(DevState s, IrRows ir, const int* __restrict__ chans, const ChanCtl* __restrict__ ctl) {
-  using S = FftShape<LOG2M>;
-  constexpr int M = S::M, T = S::T;
-  extern __shared__ float2 sm[];
-  const int part = blockIdx.x;
-  const int row = blockIdx.y;
-  const int c = chans[row];
-  const int slot = ctl[c].slot_new;
-  const float* h = ir.ptrs ? ir.ptrs[row] : ir.base + (size_t)row * ir.stride;
-  const long long t0 = (long long)part * M;  // first sample of this partition
-  for (int n = threadIdx.x; n < M; n += T) {
-    const long long t = t0 + 2 * n;
-    float2 v = make_float2(0.f, 0.f);
-    if (n < M / 2) {
-      if (t < ir.n) v.x = h[t];
-      if (t + 1 < ir.n) v.y = h[t + 1];
-    }
-    sm[n] = v;
-  }
-  __syncthreads();
-  fft_inplace<LOG2M, false>(sm, s.tw);
-  float2* H = s.H + h_index(s, c, slot, part);
-  for (int k = threadIdx.x; k <= M / 2; k += T) {
-    if (k == 0) {
-      H[0] = rfft_post_dc(sm[0]);
-    } else {
-      const int km = M - k;
-      const float2 a = sm[k], b = sm[km];
-      H[k] = rfft_post(a, b, __ldg(s.tw + k));
-      if (km != k) H[km] = rfft_post(b, a, __ldg(s.tw + km));
-    }
-  }
-}
-
-// 8-point DFT in registers (forward): two 4-point DFTs of the even and odd
-// inputs, combined with W_8^q.
-__device__ __forceinline__ void dft4_fwd(float2& a, float2& b, float2& c, float2& d) {
-  const float2 t0 = c_add(a, c), t1 = c_sub(a, c), t2 = c_add(b, d), t3 = c_sub(b, d);
-  const float2 it3 = make_float2(-t3.y, t3.x);
-  a = c_add(t0, t2);
-  c = c_sub(t0, t2);
-  b = c_sub(t1, it3);
-  d = c_add(t1, it3);
-}
-__device__ __forceinline__ void dft8_fwd(float2* v) {
-  float2 e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6], o0 = v[1], o1 = v[3], o2 = v[5], o3 = v[7];
-  dft4_fwd(e0, e1, e2, e3);
-  dft4_fwd(o0, o1, o2, o3);
-  const float r = 0.70710678118654752f;  // cos(pi/4)
-  const float2 w1 = make_float2((o1.x + o1.y) * r, (o1.y - o1.x) * r);     // o1 * W_8
-  const float2 w2 = make_float2(o2.y, -o2.x);                               // o2 * W_8^2 = -i
-  const float2 w3 = make_float2((o3.y - o3.x) * r, (-o3.y - o3.x) * r);    // o3 * W_8^3
-  v[0] = c_add(e0, o0);
-  v[4] = c_sub(e0, o0);
-  v[1] = c_add(e1, w1);
-  v[5] = c_sub(e1, w1);
-  v[2] = c_add(e2, w2);
-  v[6] = c_sub(e2, w2);
-  v[3] = c_add(e3, w3);
-  v[7] = c_sub(e3, w3);
-}
-
-// IR partition spectra with radix-8 Stockham stages in registers: M / 8
-// threads per partition, one shared-memory pass per stage instead of two for
-// radix 4 (8192 transforms of 512 points: 32 us against 45 us). When log2 M is
-// not a multiple of 3, a radix-2 or radix-4 stage comes first; it reads the
-// row directly, where the upper half of the frame is zero. Shared memory is
-// padded by one slot per 8 so that the strided stage stores spread over the
-// banks. Same inputs, twiddle table and output as ir_spectrum_kernel.
-//
-// Up to M = 1024 a CTA transforms G partitions side by side (256 threads) and
-// first gathers each stage's twiddles into shared memory, ordered so that a
-// warp reads consecutive entries: read from the table in global memory, the
-// stages' scattered twiddle loads kept the L1 pipe 93% busy (29 us for 8192
-// transforms of 512 points, which move 50 MB). The values are the table's, so
-// the spectra are the same bit for bit.
-template <int LOG2M>
-struct IrR8Shape {
-  static constexpr int M = 1 << LOG2M, T = M / 8;
-  static constexpr int R0 = LOG2M % 3;
-  static constexpr int NS0 = R0 == 0 ? 8 : (R0 == 1 ? 2 : 4);  // span after the first stage
-  static constexpr bool TWS = T <= 128;                // stage twiddles in shared memory
-  static constexpr int G = TWS ? 256 / T : 1;          // partitions per CTA
-  static constexpr int THREADS = G * T;
-  // the stages' twiddles W^(r k tstep), r = 1..7, k < Ns, stored [stage][r - 1][k]
-  // so that a warp's lanes (consecutive k) read consecutive entries
-  static constexpr int stage_entries() {
-    int n = 0;
-    for (int ns = NS0; ns < M; ns *= 8) n += 7 * ns;
-    return n;
-  }
-  static constexpr int TWN = stage_entries();
+struct IrShape {
+  using F = RegFft<LOG2M>;
+  static constexpr int G = F::T >= 256 ? 1 : 256 / F::T;  // groups (partitions side by side) per CTA
+  static constexpr int THREADS = G * F::T;
+  static constexpr bool PP = LOG2M <= 12;                 // two exchange buffers (8192 points: one)
+  static constexpr bool WREG = F::E == 8;                 // all twiddles in registers
+  static constexpr int SMEM = G * (PP ? 2 : 1) * F::PM * (int)sizeof(float2);
 };
 
+// Barrier of the T threads of one group: a warp or part of one, a named barrier
+// of whole warps, or the whole CTA.
+template <int T, int G>
+__device__ __forceinline__ void group_sync() {
+  if constexpr (T < 32) {
+    const unsigned lane = threadIdx.x & 31u;
+    __syncwarp(((1u << T) - 1u) << (lane / T * T));
+  } else if constexpr (T == 32) {
+    __syncwarp();
+  } else if constexpr (G > 1) {
+    asm volatile("bar.sync %0, %1;" ::"r"((int)threadIdx.x / T + 1), "n"(T) : "memory");
+  } else {
+    __syncthreads();
+  }
+}
+
 template <int LOG2M>
-__global__ void __launch_bounds__(IrR8Shape<LOG2M>::THREADS)
-    ir_spectrum_r8_kernel(DevState s, IrRows ir, const int* __restrict__ chans, const ChanCtl* __restrict__ ctl) {
-  using Sh = IrR8Shape<LOG2M>;
-  constexpr int M = Sh::M, T = Sh::T, G = Sh::G, R0 = Sh::R0;  // first stage radix 2^R0 (1: none)
-  constexpr int PADDED = M + M / 8;
-  __shared__ float2 sm_all[G * PADDED];
-  __shared__ float2 tw_st[Sh::TWS ? Sh::TWN : 1];
-  auto pad = [](int i) { return i + (i >> 3); };
-  const int grp = (G > 1) ? (int)threadIdx.x / T : 0;
-  const int j = (G > 1) ? (int)threadIdx.x % T : (int)threadIdx.x;
-  float2* sm = sm_all + grp * PADDED;
-  const int part = blockIdx.x * G + grp;
-  const bool live = part < s.P;
+__global__ void __launch_bounds__(IrShape<LOG2M>::THREADS)
+    ir_spectrum_kernel(DevState s, IrRows ir, const int* __restrict__ chans, const ChanCtl* __restrict__ ctl) {
+  using Sh = IrShape<LOG2M>;
+  using F = RegFft<LOG2M>;
+  constexpr int M = F::M, T = F::T, E = F::E, G = Sh::G, RL = F::RL, NPAIR = E / 2;
+  extern __shared__ __align__(16) float2 sm[];
+  auto sync = [] { group_sync<T, G>(); };
+  const int grp = (int)threadIdx.x / T, t = (int)threadIdx.x % T;
+  float2* buf0 = sm + (Sh::PP ? 2 : 1) * grp * F::PM;
+  float2* buf1 = Sh::PP ? buf0 + F::PM : buf0;
   const int row = blockIdx.y;
   const int c = chans[row];
   const int slot = ctl[c].slot_new;
   const float* h = ir.ptrs ? ir.ptrs[row] : ir.base + (size_t)row * ir.stride;
-  const long long t0 = (long long)part * M;
   const float2* tw = s.tw;
-  if constexpr (Sh::TWS) {
-    // gathered once per CTA from the table; made visible by the barrier after
-    // the first stage
-    int base = 0;
-    for (int ns = Sh::NS0; ns < M; ns *= 8) {
-      const int tstep = (2 * M) / (8 * ns);
-      for (int q = threadIdx.x; q < 7 * ns; q += Sh::THREADS) {
-        const int r = 1 + q / ns, k = q % ns;
-        tw_st[base + q] = __ldg(s.tw + r * k * tstep);
-      }
-      base += 7 * ns;
-    }
+  float2 w[Sh::WREG ? F::TWT : 1];
+  if constexpr (Sh::WREG) {
+    reg_twiddles<LOG2M, 1>(w, tw, t);
+    if constexpr (F::NP > 2) reg_twiddles<LOG2M, 2>(w + F::tw_base(2), tw, t);
   }
-  // z[n] = (h[t0 + 2n], h[t0 + 2n + 1]) for n < M / 2, zero above (and for a
-  // group past the last partition, which runs the stages for their barriers)
-  const bool h8 = (reinterpret_cast<uintptr_t>(h) & 7) == 0;  // t is even: pairs load as one float2
-  auto load = [&](int n) {
-    float2 v = make_float2(0.f, 0.f);
-    if (live && n < M / 2) {
-      const long long t = t0 + 2 * n;
-      if (h8 && t + 1 < ir.n) {
-        v = __ldg(reinterpret_cast<const float2*>(h + t));
+  float2 wp[NPAIR];
+#pragma unroll
+  for (int p = 0; p < NPAIR; ++p) wp[p] = tw[reg_out_index<LOG2M>(t, p / (RL / 2) * RL + p % (RL / 2))];
+  const bool h8 = (reinterpret_cast<uintptr_t>(h) & 7) == 0;  // sample pairs load as one float2
+  // inputs below M / 2 of partition `part` (the rest of the frame is zero)
+  auto load = [&](int part, float2 (&x)[NPAIR]) {
+#pragma unroll
+    for (int p = 0; p < NPAIR; ++p) {
+      const int n = reg_in_index<LOG2M>(t, p / (F::R0 / 2) * F::R0 + p % (F::R0 / 2));
+      const long long at = (long long)part * M + 2 * n;
+      x[p] = make_float2(0.f, 0.f);
+      if (h8 && at + 1 < ir.n) {
+        x[p] = __ldg(reinterpret_cast<const float2*>(h + at));
       } else {
-        if (t < ir.n) v.x = h[t];
-        if (t + 1 < ir.n) v.y = h[t + 1];
+        if (at < ir.n) x[p].x = h[at];
+        if (at + 1 < ir.n) x[p].y = h[at + 1];
       }
     }
-    return v;
   };
-  constexpr int NS0 = Sh::NS0;
-  float2 v[8];
-  if constexpr (R0 == 0) {
-    // radix-8 stage with Ns = 1: inputs j + r M / 8, zero for r >= 4
+  int part = blockIdx.x * G + grp;
+  const int step = gridDim.x * G;
+  float2 x[NPAIR];
+  if (part < s.P) load(part, x);
+  for (; part < s.P; part += step) {
+    float2 v[E];
 #pragma unroll
-    for (int r = 0; r < 8; ++r) v[r] = load(j + r * T);
-    dft8_fwd(v);
+    for (int i = 0; i < E; ++i)
+      v[i] = (i % F::R0 < F::R0 / 2) ? x[i / F::R0 * (F::R0 / 2) + i % F::R0] : make_float2(0.f, 0.f);
+    if (part + step < s.P) load(part + step, x);
+    reg_fft<LOG2M, false, Sh::WREG>(v, w, tw, buf0, buf1, t, sync);
+    // the upper half meets the lower one of the bin pairs in the next buffer
+    float2* pb = (F::NP & 1) ? buf0 : buf1;
 #pragma unroll
-    for (int q = 0; q < 8; ++q) sm[pad((j << 3) + q)] = v[q];
-  } else if constexpr (R0 == 1) {
-    // radix 2, Ns = 1: butterflies b = j + e T (M / 2 of them) pair z[b] with
-    // z[b + M / 2] = 0, so both outputs are z[b]
+    for (int i = 0; i < E; ++i)
+      if (i % RL >= RL / 2) pb[F::pad(reg_out_index<LOG2M>(t, i))] = v[i];
+    sync();
+    float2* H = s.H + h_index(s, c, slot, part);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int b = j + e * T;
-      const float2 a = load(b);
-      sm[pad(2 * b)] = a;
-      sm[pad(2 * b + 1)] = a;
-    }
-  } else {
-    // radix 4, Ns = 1: butterflies b = j + e T (M / 4 of them) on z[b],
-    // z[b + M / 4] and two zeros: (a + c, a - i c, a - c, a + i c)
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int b = j + e * T;
-      const float2 a = load(b), cc = load(b + M / 4);
-      sm[pad(4 * b)] = c_add(a, cc);
-      sm[pad(4 * b + 1)] = make_float2(a.x + cc.y, a.y - cc.x);
-      sm[pad(4 * b + 2)] = c_sub(a, cc);
-      sm[pad(4 * b + 3)] = make_float2(a.x - cc.y, a.y + cc.x);
-    }
-  }
-  __syncthreads();
-  auto stage = [&](const int Ns, const int tbase) {
-    const int k = j & (Ns - 1);
-    const int tstep = (2 * M) / (8 * Ns);
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-      const float2 x = sm[pad(j + r * T)];
-      if (r == 0) {
-        v[r] = x;
-      } else if constexpr (Sh::TWS) {
-        v[r] = c_mul(x, tw_st[tbase + (r - 1) * Ns + k]);
+    for (int p = 0; p < NPAIR; ++p) {
+      const int i = p / (RL / 2) * RL + p % (RL / 2);
+      const int k = reg_out_index<LOG2M>(t, i);
+      const float2 b = pb[F::pad(k == 0 ? M / 2 : M - k)];
+      if (k == 0) {
+        H[0] = x_post_dc(v[i]);
+        H[M / 2] = x_post_mid(b);
       } else {
-        v[r] = c_mul(x, __ldg(tw + r * k * tstep));
+        float2 Xk, Xm;
+        x_post(v[i], b, wp[p], Xk, Xm);
+        H[k] = Xk;
+        H[M - k] = Xm;
       }
     }
-    __syncthreads();
-    dft8_fwd(v);
-    const int d = ((j - k) << 3) + k;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) sm[pad(d + q * Ns)] = v[q];
-    __syncthreads();
-  };
-  // Powers of 8 unroll the stages (compile-time spans and twiddle strides);
-  // the others keep one loop body, which ptxas fits without spilling.
-  if constexpr (R0 == 0) {
-    int tb = 0;
-#pragma unroll
-    for (int Ns = NS0; Ns < M; Ns <<= 3) {
-      stage(Ns, tb);
-      tb += 7 * Ns;
-    }
-  } else {
-    int tb = 0;
-#pragma unroll 1
-    for (int Ns = NS0; Ns < M; Ns <<= 3) {
-      stage(Ns, tb);
-      tb += 7 * Ns;
-    }
-  }
-  if (!live) return;
-  float2* H = s.H + h_index(s, c, slot, part);
-  for (int k = j; k <= M / 2; k += T) {
-    if (k == 0) {
-      H[0] = rfft_post_dc(sm[0]);
-    } else {
-      const int km = M - k;
-      const float2 a = sm[pad(k)], b = sm[pad(km)];
-      H[k] = rfft_post(a, b, __ldg(s.tw + k));
-      if (km != k) H[km] = rfft_post(b, a, __ldg(s.tw + km));
+    if constexpr (!Sh::PP) {
+      sync();
+    } else if constexpr ((F::NP & 1) != 0) {
+      // an odd number of uses: the next partition starts with the other buffer
+      float2* b = buf0;
+      buf0 = buf1;
+      buf1 = b;
     }
   }
 }
@@ -341,7 +232,7 @@ __global__ void __launch_bounds__(IrR8Shape<LOG2M>::THREADS)
 __device__ __forceinline__ float2 crossfade_pair(float2 o, float2 yn, int i, float step, int M) {
   const float a0 = step * (float)i, b0 = step * (float)(M - i);
   const float a1 = step * (float)(i + 1), b1 = step * (float)(M - i - 1);
-  return make_float2(yn.x * a0 + o.x * b0, yn.y * a1 + o.y * b1);
+  return make_float2(__fmaf_rn(yn.x, a0, __fmul_rn(o.x, b0)), __fmaf_rn(yn.y, a1, __fmul_rn(o.y, b1)));
 }
 
 // Fused PCM epilogue (MixEpi): the channel's output row is in epi.scratch; the
@@ -374,13 +265,31 @@ __device__ __forceinline__ void mix_epilogue(const MixEpi& epi, int c) {
   if (threadIdx.x == 0) epi.count[g] = 0u;  // every member has counted itself
 }
 
+// One block of one channel. Every global load of the prologue is issued before
+// any of them is used, so the block waits for one memory round trip: the frame
+// (caller rows may sit in pinned host memory, the longest latency), the
+// twiddles, the tail, partitions 0 and 1 and X_{k-1}. The transforms run as
+// register passes (tanb_fft_reg.cuh): a block of 512 meets six barriers, where
+// radix-4 stages in shared memory met 24.
+template <int LOG2M>
+struct HeadShape {
+  using F = RegFft<LOG2M>;
+  static constexpr bool PP = LOG2M <= 11;    // two exchange buffers
+  static constexpr bool WREG = LOG2M <= 12;  // all twiddles in registers
+  static constexpr bool PRE = LOG2M <= 12;   // tail and H_0 prefetched (8192: 512 threads, 128 registers each)
+  static constexpr int SMEM = (PP ? 3 : 2) * F::PM * (int)sizeof(float2);
+};
+
 template <int LOG2M, class D>
 __device__ __forceinline__ void head_body(const DevState& s, const D& desc, int cur, int parity, const MixEpi& epi) {
-  using S = FftShape<LOG2M>;
-  constexpr int M = S::M, T = S::T, KP = S::KP;
-  extern __shared__ float2 sm[];
-  float2* z = sm;       // old / only IR
-  float2* z2 = sm + M;  // new IR on a swap block
+  using F = RegFft<LOG2M>;
+  using Sh = HeadShape<LOG2M>;
+  constexpr int M = F::M, T = F::T, E = F::E, R0 = F::R0, RL = F::RL, NP = F::NP, NPAIR = E / 2;
+  extern __shared__ __align__(16) float2 sm[];
+  float2* bufs[2] = {sm, Sh::PP ? sm + F::PM : sm};
+  float2* zb = sm + (Sh::PP ? 2 : 1) * F::PM;  // the new IR's bins on a swap block
+  auto sync = [] { __syncthreads(); };
+  const int t = threadIdx.x;
   const int c = blockIdx.x;
   const ChanCtl cc = desc.get_ctl(c);
   if (!cc.run) return;
@@ -397,191 +306,174 @@ __device__ __forceinline__ void head_body(const DevState& s, const D& desc, int 
   const bool p1 = s.P > 1;
   const float2* xp = s.fdl + ((size_t)c * s.P + (cur + 1) % s.P) * M;
 
-  // Every global load of the prologue is issued before any of them is used,
-  // so the block waits for one memory round trip instead of one per phase:
-  // first the frame (caller rows may sit in pinned host memory, the longest
-  // latency), then the twiddles, then the tail, partitions 0 and 1 and X_{k-1}.
-  // frame [x_{k-1}, x_k] packed as complex pairs. 16-byte loads of two pairs
-  // when the caller's row allows (history rows and staging rows always do):
-  // half the requests, which counts when the row is read over the host bus.
-  const bool x_vec = x && (reinterpret_cast<uintptr_t>(x) & 7) == 0;
+  // The new half of the frame, M / 2 complex pairs, goes through shared memory:
+  // 16-byte loads when the caller's row allows (staging rows always do), half
+  // the requests, which counts when the row is read over the host bus.
   const int16_t* x16 = epi.active ? reinterpret_cast<const int16_t*>(x) : nullptr;
   const bool x_v4 = !x16 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;  // also when x is null
-  constexpr int E = M / T;
-  float2 zr[E];
+  float2 xr[NPAIR];
   if (x_v4) {
-    // pair index q = threadIdx.x + j * T holds z[2q], z[2q + 1]
 #pragma unroll
-    for (int j = 0; j < E / 2; ++j) {
-      const int q = threadIdx.x + j * T;
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (q < M / 4)
-        v = reinterpret_cast<const float4*>(prev)[q];
-      else if (x)
-        v = reinterpret_cast<const float4*>(x)[q - M / 4];
-      zr[2 * j] = make_float2(v.x, v.y);
-      zr[2 * j + 1] = make_float2(v.z, v.w);
+    for (int e = 0; e < NPAIR / 2; ++e) {
+      const float4 q = x ? reinterpret_cast<const float4*>(x)[t + e * T] : make_float4(0.f, 0.f, 0.f, 0.f);
+      xr[2 * e] = make_float2(q.x, q.y);
+      xr[2 * e + 1] = make_float2(q.z, q.w);
     }
   } else {
+    const bool x_vec = (reinterpret_cast<uintptr_t>(x) & 7) == 0;
 #pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const int n = threadIdx.x + e * T;
-      if (n < M / 2) {
-        zr[e] = reinterpret_cast<const float2*>(prev)[n];
-      } else if (!x) {
-        zr[e] = make_float2(0.f, 0.f);
-      } else if (x16) {
-        const int k = 2 * (n - M / 2);
-        zr[e] = make_float2(__fmul_rn((float)x16[k], epi.in_scale), __fmul_rn((float)x16[k + 1], epi.in_scale));
-      } else if (x_vec) {
-        zr[e] = reinterpret_cast<const float2*>(x)[n - M / 2];
-      } else {
-        const float* src = x + 2 * (n - M / 2);
-        zr[e] = make_float2(src[0], src[1]);
-      }
+    for (int e = 0; e < NPAIR; ++e) {
+      const int n = t + e * T;
+      if (x16) xr[e] = make_float2(__fmul_rn((float)x16[2 * n], epi.in_scale), __fmul_rn((float)x16[2 * n + 1], epi.in_scale));
+      else if (x_vec) xr[e] = reinterpret_cast<const float2*>(x)[n];
+      else xr[e] = make_float2(x[2 * n], x[2 * n + 1]);
     }
   }
-  // twiddles (staged in shared memory for small transforms), float4 loads
+  // the old half where pass 0 takes it
+  float2 v[E];
+#pragma unroll
+  for (int i = 0; i < E; ++i)
+    if (i % R0 < R0 / 2) v[i] = reinterpret_cast<const float2*>(prev)[reg_in_index<LOG2M>(t, i)];
   const float2* tw = s.tw;
-  float4 twr[S::TW_SMEM ? E : 1];
-  if constexpr (S::TW_SMEM) {
-#pragma unroll
-    for (int e = 0; e < E; ++e) twr[e] = __ldg(reinterpret_cast<const float4*>(s.tw) + threadIdx.x + e * T);
+  float2 w[Sh::WREG ? F::TWT : 1];
+  if constexpr (Sh::WREG) {
+    reg_twiddles<LOG2M, 1>(w, tw, t);
+    if constexpr (NP > 2) reg_twiddles<LOG2M, 2>(w + F::tw_base(2), tw, t);
   }
-  // tail and partition 0 of this thread's bin pairs, and the partition-1
-  // product's operands; they do not depend on the transform. At 1024 threads
-  // (64 registers each) the partition-1 product is taken as its operands
-  // arrive, so that the prefetch fits in registers.
-  constexpr bool kHoldP1 = T < 1024;
-  float2 pt[KP][2], ph[KP][2], px[kHoldP1 ? KP : 1][2], p1h[kHoldP1 ? KP : 1][2];
+  // tail (with partition 1's product) and partition 0 of this thread's bin
+  // pairs (k, M - k), k < M / 2, with bin M / 2 beside bin 0: they do not
+  // depend on the transform
+  auto pair_reg = [](int p) { return p / (RL / 2) * RL + p % (RL / 2); };
+  auto tail_of = [&](const float2* tl, const float2* hp, int k, int km, float2& a, float2& b) {
+    a = tl[k];
+    b = tl[km];
+    if (p1) {
+      a = (k == 0) ? c_mac_dc(a, xp[0], hp[M]) : c_mac(a, xp[k], hp[M + k]);
+      b = c_mac(b, xp[km], hp[M + km]);
+    }
+  };
+  float2 pt[Sh::PRE ? NPAIR : 1][2], ph[Sh::PRE ? NPAIR : 1][2], wp[Sh::PRE ? NPAIR : 1];
+  if constexpr (Sh::PRE) {
 #pragma unroll
-  for (int q = 0; q < KP; ++q) {
-    const int k = threadIdx.x + q * T;
-    if (k <= M / 2) {
-      const int km = (k == 0) ? 0 : M - k;
-      pt[q][0] = t0[k];
-      pt[q][1] = t0[km];
-      ph[q][0] = h0[k];
-      ph[q][1] = h0[km];
-      if constexpr (kHoldP1) {
-        if (p1) {
-          px[q][0] = xp[k];
-          px[q][1] = xp[km];
-          p1h[q][0] = h0[M + k];
-          p1h[q][1] = h0[M + km];
-        }
-      } else if (p1) {
-        pt[q][0] = (k == 0) ? c_mac_dc(pt[q][0], xp[0], h0[M]) : c_mac(pt[q][0], xp[k], h0[M + k]);
-        if (k != 0) pt[q][1] = c_mac(pt[q][1], xp[km], h0[M + km]);
-      }
+    for (int p = 0; p < NPAIR; ++p) {
+      const int k = reg_out_index<LOG2M>(t, pair_reg(p)), km = (k == 0) ? M / 2 : M - k;
+      tail_of(t0, h0, k, km, pt[p][0], pt[p][1]);
+      ph[p][0] = h0[k];
+      ph[p][1] = h0[km];
+      wp[p] = tw[k];
     }
   }
-  if constexpr (S::TW_SMEM) {
-    float2* tws = sm + 2 * M;
-#pragma unroll
-    for (int e = 0; e < E; ++e) reinterpret_cast<float4*>(tws)[threadIdx.x + e * T] = twr[e];
-    tw = tws;
-  }
+  float2* xs = Sh::PP ? bufs[1] : zb;  // free until after the next barrier
   if (x_v4) {
 #pragma unroll
-    for (int j = 0; j < E / 2; ++j)
-      reinterpret_cast<float4*>(z)[threadIdx.x + j * T] =
-          make_float4(zr[2 * j].x, zr[2 * j].y, zr[2 * j + 1].x, zr[2 * j + 1].y);
+    for (int e = 0; e < NPAIR / 2; ++e)
+      reinterpret_cast<float4*>(xs)[t + e * T] = make_float4(xr[2 * e].x, xr[2 * e].y, xr[2 * e + 1].x, xr[2 * e + 1].y);
   } else {
 #pragma unroll
-    for (int e = 0; e < E; ++e) z[threadIdx.x + e * T] = zr[e];
+    for (int e = 0; e < NPAIR; ++e) xs[t + e * T] = xr[e];
   }
-  if constexpr (kHoldP1) {
-    if (p1) {
+  sync();  // also: every thread has read its part of prev
 #pragma unroll
-      for (int q = 0; q < KP; ++q) {
-        const int k = threadIdx.x + q * T;
-        if (k <= M / 2) {
-          pt[q][0] = (k == 0) ? c_mac_dc(pt[q][0], px[q][0], p1h[q][0]) : c_mac(pt[q][0], px[q][0], p1h[q][0]);
-          if (k != 0) pt[q][1] = c_mac(pt[q][1], px[q][1], p1h[q][1]);
-        }
-      }
-    }
-  }
-  __syncthreads();
-  for (int q = threadIdx.x; q < M / 4; q += T)
-    reinterpret_cast<float4*>(prev)[q] = reinterpret_cast<const float4*>(z + M / 2)[q];
+  for (int e = 0; e < NPAIR / 2; ++e)
+    reinterpret_cast<float4*>(prev)[t + e * T] = reinterpret_cast<const float4*>(xs)[t + e * T];
+#pragma unroll
+  for (int i = 0; i < E; ++i)
+    if (i % R0 >= R0 / 2) v[i] = xs[reg_in_index<LOG2M>(t, i) - M / 2];
 
-  fft_inplace<LOG2M, false>(z, tw);
+  reg_fft<LOG2M, false, Sh::WREG>(v, w, tw, bufs[0], bufs[1], t, sync);
 
-  float2* F = s.fdl + ((size_t)c * s.P + cur) * M;
+  // the upper half of the bins through shared memory to the threads that hold
+  // their partners, and the products' upper halves back the same way
+  float2* F0 = s.fdl + ((size_t)c * s.P + cur) * M;
   const float inv_n = 1.0f / (float)(2 * M);
+  float2* pb = bufs[(NP - 1) & 1];
 #pragma unroll
-  for (int q = 0; q < KP; ++q) {
-    const int k = threadIdx.x + q * T;
-    if (k > M / 2) continue;
-    if (k == 0) {
-      const float2 X = rfft_post_dc(z[0]);
-      F[0] = X;
-      z[0] = irfft_pre_dc(c_mac_dc(pt[q][0], X, ph[q][0]), inv_n);
-      if (swap) {
-        const float2 u = p1 ? c_mac_dc(t1[0], xp[0], h1[M]) : t1[0];
-        z2[0] = irfft_pre_dc(c_mac_dc(u, X, h1[0]), inv_n);
-      }
+  for (int i = 0; i < E; ++i)
+    if (i % RL >= RL / 2) pb[F::pad(reg_out_index<LOG2M>(t, i))] = v[i];
+  sync();
+#pragma unroll
+  for (int p = 0; p < NPAIR; ++p) {
+    const int i = pair_reg(p);
+    const int k = reg_out_index<LOG2M>(t, i), km = (k == 0) ? M / 2 : M - k;
+    const float2 b = pb[F::pad(km)];
+    float2 tk, tm, hk, hm, wk;
+    if constexpr (Sh::PRE) {
+      tk = pt[p][0]; tm = pt[p][1]; hk = ph[p][0]; hm = ph[p][1]; wk = wp[p];
     } else {
-      const int km = M - k;
-      const float2 wk = tw[k], wm = tw[km];
-      const float2 a = z[k], b = z[km];
-      const float2 Xk = rfft_post(a, b, wk);
-      const float2 Xm = rfft_post(b, a, wm);
-      F[k] = Xk;
-      if (km != k) F[km] = Xm;
-      const float2 Ak = c_mac(pt[q][0], Xk, ph[q][0]);
-      const float2 Am = c_mac(pt[q][1], Xm, ph[q][1]);
-      z[k] = irfft_pre(Ak, Am, wk, inv_n);
-      if (km != k) z[km] = irfft_pre(Am, Ak, wm, inv_n);
-      if (swap) {
-        const float2 uk = p1 ? c_mac(t1[k], xp[k], h1[M + k]) : t1[k];
-        const float2 um = p1 ? c_mac(t1[km], xp[km], h1[M + km]) : t1[km];
-        const float2 Bk = c_mac(uk, Xk, h1[k]);
-        const float2 Bm = c_mac(um, Xm, h1[km]);
-        z2[k] = irfft_pre(Bk, Bm, wk, inv_n);
-        if (km != k) z2[km] = irfft_pre(Bm, Bk, wm, inv_n);
+      tail_of(t0, h0, k, km, tk, tm);
+      hk = h0[k]; hm = h0[km]; wk = tw[k];
+    }
+    float2 Xk, Xm, zk, zm;
+    if (k == 0) {
+      Xk = x_post_dc(v[i]);
+      Xm = x_post_mid(b);
+      zk = x_pre_dc(c_mac_dc(tk, Xk, hk), inv_n);
+      zm = x_pre_mid(c_mac(tm, Xm, hm), inv_n);
+    } else {
+      x_post(v[i], b, wk, Xk, Xm);
+      x_pre(c_mac(tk, Xk, hk), c_mac(tm, Xm, hm), wk, inv_n, zk, zm);
+    }
+    F0[k] = Xk;
+    F0[km] = Xm;
+    if constexpr (F::SYM) v[i] = zk;
+    else pb[F::pad(k)] = zk;
+    pb[F::pad(km)] = zm;
+    if (swap) {
+      float2 uk, um;
+      tail_of(t1, h1, k, km, uk, um);
+      if (k == 0) {
+        zk = x_pre_dc(c_mac_dc(uk, Xk, h1[0]), inv_n);
+        zm = x_pre_mid(c_mac(um, Xm, h1[km]), inv_n);
+      } else {
+        x_pre(c_mac(uk, Xk, h1[k]), c_mac(um, Xm, h1[km]), wk, inv_n, zk, zm);
       }
+      zb[F::pad(k)] = zk;
+      zb[F::pad(km)] = zm;
     }
   }
-  __syncthreads();
-  fft_inplace<LOG2M, true>(z, tw);
-  if (swap) fft_inplace<LOG2M, true>(z2, tw);
+  sync();
+  if constexpr (F::SYM) {
+#pragma unroll
+    for (int i = 0; i < E; ++i)
+      if (i % R0 >= R0 / 2) v[i] = pb[F::pad(reg_in_index<LOG2M>(t, i))];
+  } else {
+    reg_load<LOG2M, 0>(v, pb, t);
+  }
+  if constexpr (!Sh::PP) sync();
+  reg_fft<LOG2M, true, Sh::WREG>(v, w, tw, bufs[NP & 1], bufs[(NP + 1) & 1], t, sync);
 
   // overlap-save: samples [B, 2B) of the circular result are the output
-  if (!y) return;
   const float step = 1.0f / (float)M;
-  const bool y_vec = (reinterpret_cast<uintptr_t>(y) & 7) == 0;
-  if ((reinterpret_cast<uintptr_t>(y) & 15) == 0) {
-    // two output pairs (samples 4q .. 4q + 3) per 16-byte store
-    for (int q = threadIdx.x; q < M / 4; q += T) {
-      const int m = M / 2 + 2 * q;
-      float2 o0 = z[m], o1 = z[m + 1];
-      if (swap) {
-        o0 = crossfade_pair(o0, z2[m], 4 * q, step, M);
-        o1 = crossfade_pair(o1, z2[m + 1], 4 * q + 2, step, M);
-      }
-      reinterpret_cast<float4*>(y)[q] = make_float4(o0.x, o0.y, o1.x, o1.y);
+  if (swap) {
+    float2 o[E / 2];
+#pragma unroll
+    for (int p = 0; p < NPAIR; ++p) o[p] = v[pair_reg(p) + RL / 2];
+    reg_load<LOG2M, 0>(v, zb, t);
+    if constexpr (!Sh::PP) sync();
+    reg_fft<LOG2M, true, Sh::WREG>(v, w, tw, bufs[1], bufs[0], t, sync);
+#pragma unroll
+    for (int p = 0; p < NPAIR; ++p) {
+      const int i = pair_reg(p) + RL / 2;
+      v[i] = crossfade_pair(o[p], v[i], 2 * (reg_out_index<LOG2M>(t, i) - M / 2), step, M);
     }
-  } else {
-    for (int m = M / 2 + threadIdx.x; m < M; m += T) {
-      const int i = 2 * (m - M / 2);
-      float2 o = z[m];
-      if (swap) o = crossfade_pair(o, z2[m], i, step, M);
-      if (y_vec) {
-        reinterpret_cast<float2*>(y)[i / 2] = o;
-      } else {
-        y[i] = o.x;
-        y[i + 1] = o.y;
-      }
+  }
+  if (!y) return;
+  const bool y_vec = (reinterpret_cast<uintptr_t>(y) & 7) == 0;
+#pragma unroll
+  for (int p = 0; p < NPAIR; ++p) {
+    const int i = pair_reg(p) + RL / 2, n = reg_out_index<LOG2M>(t, i) - M / 2;
+    if (y_vec) {
+      reinterpret_cast<float2*>(y)[n] = v[i];
+    } else {
+      y[2 * n] = v[i].x;
+      y[2 * n + 1] = v[i].y;
     }
   }
   if (epi.active) mix_epilogue<M, T>(epi, c);
 }
 
 template <int LOG2M, class D>
-__global__ void __launch_bounds__(FftShape<LOG2M>::T)
+__global__ void __launch_bounds__(RegFft<LOG2M>::T)
     head_kernel(DevState s, const __grid_constant__ D desc, int cur, int parity, MixEpi epi, HeadSignal sig) {
   // The tail launched behind this kernel (the next block's partitions >= 2)
   // shares no data with it and may start at once.
@@ -792,7 +684,7 @@ constexpr int bulk_smem_bytes() {
 
 template <int LOG2M>
 cudaError_t set_attrs() {
-  const int smem = (FftShape<LOG2M>::TW_SMEM ? 4 : 2) * (1 << LOG2M) * (int)sizeof(float2);
+  constexpr int smem = HeadShape<LOG2M>::SMEM;
   cudaError_t e =
       cudaFuncSetAttribute(head_kernel<LOG2M, DevDesc>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
@@ -801,35 +693,37 @@ cudaError_t set_attrs() {
   e = cudaFuncSetAttribute(head_kernel<LOG2M, StgDesc>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute(ir_spectrum_kernel<LOG2M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (1 << LOG2M) * (int)sizeof(float2));
+                              IrShape<LOG2M>::SMEM);
 }
+
+// Partitions of an IR update that one group of threads takes in turn: enough to
+// pay for loading the twiddles, few enough that every SM has several CTAs.
+constexpr int kIrPartsPerGroup = 4;
 
 template <int LOG2M>
 cudaError_t launch_ir_t(const DevState& s, const IrRows& ir, const int* chans, int nch, const ChanCtl* ctl,
                         cudaStream_t st) {
-  using S = FftShape<LOG2M>;
-  if constexpr (LOG2M <= 12) {  // the padded buffer of 8192 points exceeds static shared memory
-    using R = IrR8Shape<LOG2M>;
-    ir_spectrum_r8_kernel<LOG2M><<<dim3((s.P + R::G - 1) / R::G, nch), R::THREADS, 0, st>>>(s, ir, chans, ctl);
-  } else {
-    ir_spectrum_kernel<LOG2M><<<dim3(s.P, nch), S::T, S::M * sizeof(float2), st>>>(s, ir, chans, ctl);
-  }
+  using R = IrShape<LOG2M>;
+  const long long groups = ((long long)s.P * nch + R::G - 1) / R::G;  // CTAs at one partition per group
+  const int iters = (int)std::max<long long>(1, std::min<long long>(kIrPartsPerGroup, groups / (148 * 2)));
+  const int gx = (s.P + R::G * iters - 1) / (R::G * iters);
+  ir_spectrum_kernel<LOG2M><<<dim3(gx, nch), R::THREADS, R::SMEM, st>>>(s, ir, chans, ctl);
   return cudaGetLastError();
 }
 
 template <int LOG2M>
 cudaError_t launch_head_t(const DevState& s, const BlockRef& d, int cur, int parity, cudaStream_t st,
                           const MixEpi& epi, const HeadSignal& sig) {
-  using S = FftShape<LOG2M>;
-  const size_t smem = (S::TW_SMEM ? 4 : 2) * S::M * sizeof(float2);
+  constexpr int T = RegFft<LOG2M>::T;
+  constexpr size_t smem = HeadShape<LOG2M>::SMEM;
   const int cv = pair_carveout(LOG2M);
   if (d.stage)
-    return launch_k(head_kernel<LOG2M, StgDesc>, dim3(s.C), dim3(S::T), smem, st, false, cv, s, StgDesc{*d.stage},
+    return launch_k(head_kernel<LOG2M, StgDesc>, dim3(s.C), dim3(T), smem, st, false, cv, s, StgDesc{*d.stage},
                     cur, parity, epi, sig);
   if (d.param)
-    return launch_k(head_kernel<LOG2M, ParDesc>, dim3(s.C), dim3(S::T), smem, st, false, cv, s, ParDesc{*d.param},
+    return launch_k(head_kernel<LOG2M, ParDesc>, dim3(s.C), dim3(T), smem, st, false, cv, s, ParDesc{*d.param},
                     cur, parity, epi, sig);
-  return launch_k(head_kernel<LOG2M, DevDesc>, dim3(s.C), dim3(S::T), smem, st, false, cv, s,
+  return launch_k(head_kernel<LOG2M, DevDesc>, dim3(s.C), dim3(T), smem, st, false, cv, s,
                   DevDesc{d.ctl, d.in, d.out}, cur, parity, epi, sig);
 }
 
@@ -961,6 +855,13 @@ void make_twiddles(int N, float2* out) {
     }
     out[j] = make_float2((float)cc, (float)(-ss));
   }
+}
+
+void make_plan_twiddles(int log2M, float2* out) {
+  const int M = 1 << log2M;
+  std::vector<float2> w(2 * M);
+  make_twiddles(2 * M, w.data());
+  for (int i = 0; i < 2 * M; ++i) out[i] = w[plan_twiddle_index(log2M, i)];
 }
 
 }  // namespace tanb

@@ -23,6 +23,7 @@
 #include <mutex>
 
 #include "../../include/tanb.h"
+#include "tanb_fft_reg.cuh"
 #include "tanb_internal.h"
 
 namespace {
@@ -58,11 +59,13 @@ cudaError_t scratch_base(unsigned char** out) {
 
 size_t up256(size_t x) { return (x + 255) / 256 * 256; }
 
-// W_N^j = exp(-2 pi i j / N), computed in double with the same quadrant
-// reduction as tanb::make_twiddles and rounded to float.
-__global__ void twiddle_kernel(float2* tw, int N) {
-  const int q4 = N / 4;
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < N; j += gridDim.x * blockDim.x) {
+// The table of tanb::make_plan_twiddles: entries exp(-2 pi i j / N), N = 2M,
+// computed in double with the same quadrant reduction as tanb::make_twiddles
+// and rounded to float.
+__global__ void twiddle_kernel(float2* tw, int log2M) {
+  const int N = 2 << log2M, q4 = N / 4;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
+    const int j = tanb::plan_twiddle_index(log2M, i);
     const int q = j / q4, r = j % q4;
     const double th = 2.0 * 3.14159265358979323846 * (double)r / (double)N;
     double s, c;
@@ -74,7 +77,7 @@ __global__ void twiddle_kernel(float2* tw, int N) {
       case 2: cc = -c; ss = -s; break;
       default: cc = s; ss = -c; break;
     }
-    tw[j] = make_float2((float)cc, (float)(-ss));
+    tw[i] = make_float2((float)cc, (float)(-ss));
   }
 }
 
@@ -172,7 +175,7 @@ extern "C" int32_t tanb_convolve_no_alloc(const float* in, const float* ir, floa
     if ((e = cudaMemcpy2DAsync(irp, P * B * sizeof(float), ir, ir_length * sizeof(float),
                                ir_length * sizeof(float), C, cudaMemcpyDeviceToDevice, st)) != cudaSuccess)
       break;
-    twiddle_kernel<<<(unsigned)((2 * B + 255) / 256), 256, 0, st>>>(tw, (int)(2 * B));
+    twiddle_kernel<<<(unsigned)((2 * B + 255) / 256), 256, 0, st>>>(tw, s.log2B);
     // IR spectra into slot 0
     describe_kernel<<<(unsigned)((C + 127) / 128), 128, 0, st>>>(ctl, in_rows, out_rows, chans, nullptr, nullptr,
                                                                  (int)C, samples, 0, 0);
