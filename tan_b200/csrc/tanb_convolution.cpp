@@ -149,6 +149,11 @@ struct tanb_convolution {
 
   cudaEvent_t ev_stage = nullptr, ev_ir = nullptr, ev_out = nullptr;
 
+  // calls over several blocks: spectra of the new blocks and of their outputs,
+  // [2][C][run_blocks][B] float2, allocated by the first such call
+  float2* d_run = nullptr;
+  int run_blocks = 0;
+
   // fused PCM pipeline (tanb_convolution_process_mix_pcm16), allocated on first use
   float* d_mix_scratch = nullptr;   // [C][B] channel outputs
   int* d_mix_table = nullptr;       // chan_group[C], gstart[C + 1], gchan[C], count[C]
@@ -268,6 +273,9 @@ void free_all(tanb_convolution* v) {
   v->d_head_count = nullptr;
   cudaFree(v->d_ir);
   cudaFree(v->d_uctl);
+  cudaFree(v->d_run);
+  v->d_run = nullptr;
+  v->run_blocks = 0;
   cudaFree(v->d_mix_scratch);
   cudaFree(v->d_mix_table);
   cudaFreeHost(v->h_clip);
@@ -685,6 +693,208 @@ cudaError_t ensure_mix(tanb_convolution* v, const PcmIO& pcm, tanb::MixEpi* epi)
   return cudaSuccess;
 }
 
+// Blocks of one many-block launch at most, and the device bytes of its
+// workspace at most (the rest of a call goes through further launches).
+constexpr int kRunMaxBlocks = 64;
+constexpr int kRunIrBlocks = 16;
+constexpr size_t kRunSmallBytes = 8u << 20;
+constexpr size_t kRunMaxBytes = 64u << 20;
+
+// Workspace for launches over up to `nb` blocks; returns the blocks it holds
+// (0: too large for the bound, or no memory: the call then runs block by block).
+// The device rows of IR updates (C x P x B floats, used by copies and transforms
+// on the same stream only) serve where they hold the whole launch, or enough
+// blocks of a large one (kRunIrBlocks) that a second launch sequence costs little;
+// calls of a few small channels are bound by the sequence's latency (two
+// sequences for 64 blocks of two channels took 93 us instead of 56).
+int ensure_run(tanb_convolution* v, size_t nb, float2** work) {
+  const int ir = std::min(v->P / 4, kRunMaxBlocks);  // 4 B floats per block and channel
+  const size_t per = 2 * (size_t)v->C * v->B * sizeof(float2);  // bytes per block
+  const int want = (int)std::min<size_t>({nb, (size_t)kRunMaxBlocks, kRunMaxBytes / per});
+  if (ir >= 2 && (want <= ir || (ir >= kRunIrBlocks && per * want > kRunSmallBytes))) {
+    *work = reinterpret_cast<float2*>(v->d_ir);
+    return ir;
+  }
+  if (want < 2) return 0;
+  if (want > v->run_blocks) {
+    // the old one may be in use by a launch in flight: freed after it
+    if (v->d_run && cudaStreamSynchronize(v->stream) != cudaSuccess) return 0;
+    cudaFree(v->d_run);
+    v->dev_bytes -= per * v->run_blocks;
+    v->d_run = nullptr;
+    v->run_blocks = 0;
+    if (cudaMalloc(&v->d_run, per * want) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return 0;
+    }
+    v->run_blocks = want;
+    v->dev_bytes += per * want;
+  }
+  *work = v->d_run;
+  return v->run_blocks;
+}
+
+// True when the input and output rows of a call over n samples per row are
+// apart, or every channel's output is its own input row: reading all inputs
+// before writing any output then gives what block-by-block processing gives.
+bool rows_apart(const float* const* in, float* const* out, int C, size_t n) {
+  uintptr_t il = UINTPTR_MAX, ih = 0, ol = UINTPTR_MAX, oh = 0;
+  bool same = true;
+  for (int c = 0; c < C; ++c) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(in[c]), b = reinterpret_cast<uintptr_t>(out[c]);
+    same = same && a == b;
+    if (a) {
+      il = std::min(il, a);
+      ih = std::max(ih, a + n * sizeof(float));
+    }
+    if (b) {
+      ol = std::min(ol, b);
+      oh = std::max(oh, b + n * sizeof(float));
+    }
+  }
+  if (il >= oh || ol >= ih) return true;
+  if (!same) return false;
+  // in place: the rows must not overlap one another
+  std::vector<uintptr_t> r;
+  for (int c = 0; c < C; ++c)
+    if (in[c]) r.push_back(reinterpret_cast<uintptr_t>(in[c]));
+  std::sort(r.begin(), r.end());
+  for (size_t j = 1; j < r.size(); ++j)
+    if (r[j] - r[j - 1] < n * sizeof(float)) return false;
+  return true;
+}
+
+// Blocks of the next of as few launches as `left` blocks need, alike in size.
+int even_share(size_t left, int cap) {
+  const size_t parts = (left + cap - 1) / cap;
+  return (int)((left + parts - 1) / parts);
+}
+
+struct RunCall {
+  Mem in_mem;
+  const float* const* in;
+  Mem out_mem;
+  float* const* out;
+  const uint32_t* flags;
+  size_t first;             // block of the call the launch starts at
+  const PinnedRows* pin_in;   // caller rows addressed in place
+  const PinnedRows* pin_out;
+  bool param, staged;
+  float2* work;             // X and Y of RunShape
+};
+
+// Up to `nb` blocks of a call as one launch sequence; *done: how many. Host rows
+// the kernels cannot address in place go through pinned staging: the IR staging
+// rows (free once ev_ir has passed: an IR update waits for it before it writes
+// them, and so does this) when they hold more blocks than Process's own.
+int32_t run_blocks(tanb_convolution* v, const RunCall& q, int nb, int* done, double* t_wait) {
+  const int B = v->B, C = v->C, P = v->P;
+  const bool stage_in = q.in_mem == Mem::Host && !q.pin_in, stage_out = q.out_mem == Mem::Host && !q.pin_out;
+  TANB_CUDA(cudaEventSynchronize(v->ev_stage));
+  if (v->staging_busy) {
+    TANB_CUDA(cudaEventSynchronize(v->ev_out));
+    v->staging_busy = false;
+  }
+  float* hin = v->stage_in(v->h_stage, 0, 0);
+  float* hout = v->h_out;
+  bool ir_stage = false;
+  if (stage_in || stage_out) {
+    const int own = kMaxBlocksPerChunk, ir = P / 2;
+    if (ir > own && nb > own) {
+      TANB_CUDA(cudaEventSynchronize(v->ev_ir));
+      nb = std::min(nb, ir);
+      hin = v->h_ir;
+      hout = v->h_ir + (size_t)C * nb * B;
+      ir_stage = true;
+    } else {
+      nb = std::min(nb, own);
+    }
+  }
+  std::vector<uint8_t>& run = v->scr_run;
+  std::vector<uint8_t>& flush = v->scr_flush;
+  for (int b = 0; b < nb; ++b) {
+    channel_flags(v, q.flags, run, flush);  // every channel runs; flushes only on the first block
+    if (b == 0)
+      for (int c = 0; c < C; ++c)
+        if (flush[c]) TANB_CUDA(flush_channel(v, c));
+  }
+  const size_t off = q.first * (size_t)B, row = (size_t)nb * B;
+  tanb::ParamDesc* pd = q.param ? &v->pdesc[0] : nullptr;
+  tanb::StageDesc* sd = q.staged ? &v->sdesc[0] : nullptr;
+  for (int c = 0; c < C; ++c) {
+    const ChanCtl cc{1, 0, v->active[c], v->slot_new[c]};
+    const float* x = q.in[c] ? (stage_in ? hin + c * row : q.in[c] + off) : nullptr;
+    float* y = stage_out ? hout + c * row : (q.out[c] ? q.out[c] + off : nullptr);
+    if (stage_in && q.in[c]) tanb::copy_rows_for_device(hin + c * row, q.in[c] + off, row * sizeof(float));
+    if (sd) {
+      sd->c.ctl[c] = tanb::pack_ctl(cc, x != nullptr);
+    } else if (pd) {
+      pd->c.ctl[c] = tanb::pack_ctl(cc, x != nullptr);
+      pd->in[c] = x;
+      pd->out[c] = y;
+    } else {
+      v->desc_ctl(v->h_stage, 0)[c] = cc;
+      v->desc_in(v->h_stage, 0)[c] = x;
+      v->desc_out(v->h_stage, 0)[c] = y;
+    }
+  }
+  if (sd) {
+    sd->in = q.pin_in ? q.pin_in->base + off : hin;
+    sd->stride = q.pin_in ? q.pin_in->stride : (long long)row;
+    sd->out = q.pin_out ? const_cast<float*>(q.pin_out->base) + off : hout;
+    sd->ostride = q.pin_out ? q.pin_out->stride : (long long)row;
+  }
+  if (stage_in) tanb::copy_for_device_fence();
+  if (!q.param) {
+    TANB_CUDA(cudaMemcpyAsync(v->d_stage, v->h_stage, v->desc_bytes, cudaMemcpyHostToDevice, v->stream));
+    TANB_CUDA(cudaEventRecord(v->ev_stage, v->stream));
+  }
+  tanb::BlockRef ref;
+  if (sd) {
+    ref.stage = sd;
+  } else if (pd) {
+    ref.param = pd;
+  } else {
+    ref.ctl = v->desc_ctl(v->d_stage, 0);
+    ref.in = v->desc_in(v->d_stage, 0);
+    ref.out = v->desc_out(v->d_stage, 0);
+  }
+  tanb::RunShape r;
+  r.X = q.work;
+  r.Y = q.work + (size_t)C * nb * B;
+  r.nb = nb;
+  r.sy = v->tiling.sy;
+  r.cur = v->cur;
+  r.trow = (int)((v->blocks + nb) & 1);
+  tanb::HeadSignal sig;
+  const bool host_out = q.out_mem == Mem::Host;
+  if (host_out) sig = tanb::HeadSignal{v->d_head_count, v->d_head_flag, ++v->head_seq};
+  v->launches[tanb_convolution::kHead] += 1;  // the inverse transforms; the forward ones count with the launch
+  v->launches[tanb_convolution::kTail] += 1;
+  TANB_CUDA(counted(v, tanb_convolution::kHead, [&] { return tanb::launch_run(v->ds, ref, r, v->stream, sig); }));
+  v->cur = ((v->cur - nb) % P + P) % P;
+  v->last_desc = v->desc_ctl(v->d_stage, 0);
+  v->last_is_param = q.param;
+  if (q.param) v->last_ctlp = sd ? sd->c : pd->c;
+  v->last_cur = v->cur;
+  if (q.in_mem == Mem::Host || host_out) {
+    TANB_CUDA(cudaEventRecord(v->ev_out, v->stream));
+    v->staging_busy = true;
+  }
+  if (ir_stage) TANB_CUDA(cudaEventRecord(v->ev_ir, v->stream));
+  if (host_out) {
+    const auto t0 = std::chrono::steady_clock::now();
+    if (wait_heads(v, v->head_seq) != TANB_OK) return TANB_FAIL;
+    *t_wait += std::chrono::duration<double, std::micro>(std::chrono::steady_clock::now() - t0).count();
+    v->staging_busy = false;
+    if (stage_out)
+      for (int c = 0; c < C; ++c)
+        if (q.out[c]) std::memcpy(q.out[c] + off, hout + c * row, row * sizeof(float));
+  }
+  *done = nb;
+  return TANB_OK;
+}
+
 int32_t process_common(tanb_convolution* v, Mem in_mem, const float* const* in, Mem out_mem, float* const* out,
                        size_t n, const uint32_t* flags, size_t* done, const PcmIO* pcm = nullptr) {
   tanb::NvtxRange range("tanb Process");
@@ -736,9 +946,36 @@ int32_t process_common(tanb_convolution* v, Mem in_mem, const float* const* in, 
   };
   const Clock::time_point t_call = Clock::now();
   double t_stage = 0, t_launch = 0, t_wait = 0, t_copy = 0;
+  // Several blocks in one launch sequence (launch_run): no channel may change
+  // state inside the call, which only STOP_INPUT makes happen (every channel
+  // then runs, and a flush can only fall on the call's first block), and the
+  // tail must sum its partitions in the register-load kernel's chunks. A swap
+  // takes its block through the one-block path first.
+  float2* run_work = nullptr;
+  bool many = nblocks > 1 && !pcm && !v->finalize_mode && v->tiling.kind == 0 && v->tiling.sy >= 8;
+  for (int c = 0; many && flags && c < C; ++c) many = (flags[c] & kStopInput) == 0;
+  if (many) many = rows_apart(in, out, C, nblocks * (size_t)B);
   while (processed < nblocks && status == TANB_OK) {
     const Clock::time_point t0 = Clock::now();
     int nb = (int)std::min<size_t>(kMaxBlocksPerChunk, nblocks - processed);
+    if (many && nblocks - processed > 1) {
+      bool pend = false;
+      for (int c = 0; c < C; ++c) pend = pend || v->pending[c];
+      if (pend) {
+        nb = 1;
+      } else if (const int cap = ensure_run(v, nblocks - processed, &run_work)) {
+        const int32_t r = run_blocks(v, RunCall{in_mem, in, out_mem, out, flags, processed, direct_in ? &pin_in : nullptr,
+                                                direct_out ? &pin_out : nullptr, param, staged, run_work},
+                                     even_share(nblocks - processed, cap), &nb, &t_wait);
+        if (r != TANB_OK) return r;
+        processed += nb;
+        v->blocks += nb;
+        t_launch += us(t0, Clock::now());
+        continue;
+      } else {
+        many = false;
+      }
+    }
     TANB_CUDA(cudaEventSynchronize(v->ev_stage));
     if (v->staging_busy) {
       TANB_CUDA(cudaEventSynchronize(v->ev_out));
@@ -1388,7 +1625,7 @@ int32_t init_impl(tanb_convolution* v, uint32_t method, uint32_t L, uint32_t B, 
     return TANB_OK;
   }
   if (nlevels) return fail(TANB_INVALID_ARG, "a level schedule needs a non-uniform method");
-  if ((e = tanb::prepare_kernels()) != cudaSuccess) return fail(TANB_FAIL, "kernel setup: %s", cudaGetErrorString(e));
+  if ((e = tanb::prepare_kernels(log2B)) != cudaSuccess) return fail(TANB_FAIL, "kernel setup: %s", cudaGetErrorString(e));
   if ((e = cudaStreamCreateWithFlags(&v->stream, cudaStreamNonBlocking)) != cudaSuccess)
     return fail(TANB_FAIL, "stream: %s", cudaGetErrorString(e));
   const size_t Cs = C, Bs = B, Ps = v->P;

@@ -130,7 +130,10 @@ __device__ __forceinline__ float2 irfft_pre_dc(float2 a, float inv_n) {
 }
 
 // acc + a * b with the operation order of the reference's AVX2 planar MAC
-// (re: fma(ar, br, -(ai*bi)) + cr, im: fma(ar, bi, ai*br) + ci).
+// (re: fma(ar, br, -(ai*bi)) + cr, im: fma(ar, bi, ai*br) + ci). The product is
+// rounded before it meets the sum: accumulating with fused multiply-adds alone
+// is two operations shorter but rounds twice at the sum's magnitude (error
+// against 64 bits 2.4e-7 instead of 2.2e-7 over 128 partitions).
 __device__ __forceinline__ float2 c_mac(float2 acc, float2 a, float2 b) {
   const float re = __fmaf_rn(a.x, b.x, -__fmul_rn(a.y, b.y));
   const float im = __fmaf_rn(a.x, b.y, __fmul_rn(a.y, b.x));

@@ -228,6 +228,22 @@ cudaError_t launch_head(const DevState& s, const BlockRef& d, int cur, int parit
 cudaError_t launch_tail(const DevState& s, const BlockRef& d, int which, int cur, int trow, MacTiling t,
                         cudaStream_t st, bool pdl = false);
 
+// One call over nb blocks of every channel: all channels run, none swaps, the
+// descriptor's rows hold the nb blocks back to back. X and Y are workspaces of
+// [C][nb][B] float2; `cur` is the delay-line slot of the newest spectrum before
+// the call, `sy` the partition chunks of the object's tail tiling (kind 0, at
+// least 8), `trow` the tail row of the block after the call.
+struct RunShape {
+  float2* X = nullptr;
+  float2* Y = nullptr;
+  int nb = 0;
+  int sy = 8;
+  int cur = 0;
+  int trow = 0;
+};
+cudaError_t launch_run(const DevState& s, const BlockRef& d, const RunShape& r, cudaStream_t st,
+                       const HeadSignal& sig = HeadSignal{});
+
 // Per-channel descriptor of one TIME_DOMAIN call.
 struct TdChan {
   const float* in;      // device row of n input samples (null: silence)
@@ -246,8 +262,9 @@ struct TdChan {
 // history (len samples, [C][len]) and compute n direct-FIR outputs.
 cudaError_t launch_td(float* hist, int len, const TdChan* ch, int C, int n, int fade_len, cudaStream_t st);
 
-// Sets the shared-memory attributes of every kernel (once per device).
-cudaError_t prepare_kernels();
+// Sets the shared-memory attributes of the kernels of one block size (once per
+// device and size: setting one loads the kernel).
+cudaError_t prepare_kernels(int log2B);
 
 // Fills the twiddle table W_N^j = exp(-2 pi i j / N) on the host, computed in
 // double and rounded to float, exact at multiples of pi/2.

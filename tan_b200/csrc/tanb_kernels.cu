@@ -17,6 +17,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -472,6 +473,20 @@ __device__ __forceinline__ void head_body(const DevState& s, const D& desc, int 
   if (epi.active) mix_epilogue<M, T>(epi, c);
 }
 
+// Completion signal of a launch of `total` CTAs: every CTA, running or not,
+// counts itself once its output stores are visible to the host; the last one
+// raises the flag.
+__device__ __forceinline__ void signal_heads(const HeadSignal& sig, unsigned total) {
+  if (sig.seq == 0) return;
+  __threadfence_system();
+  __syncthreads();
+  if (threadIdx.x == 0 && atomicAdd(sig.count, 1u) == total - 1) {
+    *sig.count = 0u;
+    __threadfence_system();
+    *reinterpret_cast<volatile long long*>(sig.flag) = sig.seq;
+  }
+}
+
 template <int LOG2M, class D>
 __global__ void __launch_bounds__(RegFft<LOG2M>::T)
     head_kernel(DevState s, const __grid_constant__ D desc, int cur, int parity, MixEpi epi, HeadSignal sig) {
@@ -479,16 +494,7 @@ __global__ void __launch_bounds__(RegFft<LOG2M>::T)
   // shares no data with it and may start at once.
   griddep_launch_dependents();
   head_body<LOG2M>(s, desc, cur, parity, epi);
-  if (sig.seq == 0) return;
-  // Every CTA, running or not, counts itself once its output stores are
-  // visible to the host; the last one raises the flag.
-  __threadfence_system();
-  __syncthreads();
-  if (threadIdx.x == 0 && atomicAdd(sig.count, 1u) == gridDim.x - 1) {
-    *sig.count = 0u;
-    __threadfence_system();
-    *reinterpret_cast<volatile long long*>(sig.flag) = sig.seq;
-  }
+  signal_heads(sig, gridDim.x);
 }
 
 // One float4 = two packed bins. u == 0 holds the packed (DC, Nyquist) pair.
@@ -555,6 +561,539 @@ __global__ void __launch_bounds__(UX* SY)
     }
   }
   if (u < U) reinterpret_cast<float4*>(s.tail + ((size_t)c * 3 + trow) * s.B)[u] = acc;
+}
+
+// ---------------------------------------------------------------------------
+// Several blocks in one call. With nb blocks in hand the sum
+//   Y_b = sum_i X_{b - i} H_i,  b = 0 .. nb - 1
+// reads each spectrum once per group of output blocks instead of once per
+// block, so the call is bound by its transforms and its products and no longer
+// by the IR spectra and the delay line (67 MB per block at 64 channels of 65536
+// taps: 10.2 us a block in the one-block form, head and tail). Three launches:
+//   run_forward_kernel  every new spectrum X_b, b < nb, into the workspace
+//   run_mac_kernel      Y_b for every b, and the tail of block nb for the call
+//                       after this one
+//   run_inverse_kernel  the outputs, and the last P new spectra into the delay
+//                       line
+// The sums are formed in the order of tail_kernel and head_kernel (partitions
+// 2 .. P-1 in the tiling's chunks, the chunks in order, then partition 1, then
+// 0) and the transforms are the same register passes, so a call over several
+// blocks gives the bits of the one-block calls.
+
+// Threads of the transforms: as IrShape, runs of consecutive blocks per group.
+template <int LOG2M, class D>
+__global__ void __launch_bounds__(IrShape<LOG2M>::THREADS)
+    run_forward_kernel(DevState s, const __grid_constant__ D desc, float2* __restrict__ X, int nb, int run) {
+  using Sh = IrShape<LOG2M>;
+  using F = RegFft<LOG2M>;
+  constexpr int M = F::M, T = F::T, E = F::E, G = Sh::G, R0 = F::R0, RL = F::RL, NPAIR = E / 2;
+  extern __shared__ __align__(16) float2 sm[];
+  auto sync = [] { group_sync<T, G>(); };
+  const int grp = (int)threadIdx.x / T, t = (int)threadIdx.x % T;
+  float2* buf0 = sm + (Sh::PP ? 2 : 1) * grp * F::PM;
+  float2* buf1 = Sh::PP ? buf0 + F::PM : buf0;
+  const int c = blockIdx.y;
+  const float* x = desc.get_in(c);
+  const float2* tw = s.tw;
+  const int r0 = ((int)blockIdx.x * G + grp) * run, r1 = min(nb, r0 + run);
+  if (r0 >= nb) return;
+  float2 w[Sh::WREG ? F::TWT : 1];
+  if constexpr (Sh::WREG) {
+    reg_twiddles<LOG2M, 1>(w, tw, t);
+    if constexpr (F::NP > 2) reg_twiddles<LOG2M, 2>(w + F::tw_base(2), tw, t);
+  }
+  const bool x8 = (reinterpret_cast<uintptr_t>(x) & 7) == 0;
+  // samples of block r where pass 0 takes a frame's halves: the same thread
+  // reads block r as the new half of frame r and the old half of frame r + 1
+  auto load = [&](int r, float2 (&q)[NPAIR]) {
+    const float* src = r < 0 ? s.prev + (size_t)c * M : x + (size_t)r * M;
+#pragma unroll
+    for (int p = 0; p < NPAIR; ++p) {
+      const int n = reg_in_index<LOG2M>(t, p / (R0 / 2) * R0 + p % (R0 / 2));
+      if (r >= 0 && !x) q[p] = make_float2(0.f, 0.f);
+      else if (x8 || r < 0) q[p] = reinterpret_cast<const float2*>(src)[n];
+      else q[p] = make_float2(src[2 * n], src[2 * n + 1]);
+    }
+  };
+  float2 lo[NPAIR], hi[NPAIR];
+  load(r0 - 1, lo);
+  load(r0, hi);
+  for (int r = r0; r < r1; ++r) {
+    float2 v[E];
+#pragma unroll
+    for (int i = 0; i < E; ++i) {
+      const int p = i / R0 * (R0 / 2) + i % (R0 / 2);
+      v[i] = (i % R0 < R0 / 2) ? lo[p] : hi[p];
+    }
+#pragma unroll
+    for (int p = 0; p < NPAIR; ++p) lo[p] = hi[p];
+    if (r + 1 < r1) load(r + 1, hi);
+    reg_fft<LOG2M, false, Sh::WREG>(v, w, tw, buf0, buf1, t, sync);
+    float2* pb = (F::NP & 1) ? buf0 : buf1;
+#pragma unroll
+    for (int i = 0; i < E; ++i)
+      if (i % RL >= RL / 2) pb[F::pad(reg_out_index<LOG2M>(t, i))] = v[i];
+    sync();
+    float2* Xr = X + ((size_t)c * nb + r) * M;
+#pragma unroll
+    for (int p = 0; p < NPAIR; ++p) {
+      const int i = p / (RL / 2) * RL + p % (RL / 2);
+      const int k = reg_out_index<LOG2M>(t, i), km = (k == 0) ? M / 2 : M - k;
+      const float2 b = pb[F::pad(km)];
+      float2 Xk, Xm;
+      if (k == 0) {
+        Xk = x_post_dc(v[i]);
+        Xm = x_post_mid(b);
+      } else {
+        x_post(v[i], b, tw[k], Xk, Xm);
+      }
+      Xr[k] = Xk;
+      Xr[km] = Xm;
+    }
+    if constexpr (!Sh::PP) {
+      sync();
+    } else if constexpr ((F::NP & 1) != 0) {
+      float2* b = buf0;
+      buf0 = buf1;
+      buf1 = b;
+    }
+  }
+}
+
+template <int LOG2M, class D>
+__global__ void __launch_bounds__(IrShape<LOG2M>::THREADS)
+    run_inverse_kernel(DevState s, const __grid_constant__ D desc, const float2* __restrict__ X,
+                       const float2* __restrict__ Y, int nb, int run, int cur, HeadSignal sig) {
+  using Sh = IrShape<LOG2M>;
+  using F = RegFft<LOG2M>;
+  constexpr int M = F::M, T = F::T, E = F::E, G = Sh::G, RL = F::RL, NPAIR = E / 2;
+  extern __shared__ __align__(16) float2 sm[];
+  auto sync = [] { group_sync<T, G>(); };
+  const int grp = (int)threadIdx.x / T, t = (int)threadIdx.x % T;
+  float2* buf0 = sm + (Sh::PP ? 2 : 1) * grp * F::PM;
+  float2* buf1 = Sh::PP ? buf0 + F::PM : buf0;
+  const int c = blockIdx.y;
+  float* y = desc.get_out(c);
+  const bool y8 = (reinterpret_cast<uintptr_t>(y) & 7) == 0;
+  const float2* tw = s.tw;
+  const int r0 = ((int)blockIdx.x * G + grp) * run, r1 = min(nb, r0 + run);
+  const float inv_n = 1.0f / (float)(2 * M);
+  if (r0 < nb) {
+    float2 w[Sh::WREG ? F::TWT : 1];
+    if constexpr (Sh::WREG) {
+      reg_twiddles<LOG2M, 1>(w, tw, t);
+      if constexpr (F::NP > 2) reg_twiddles<LOG2M, 2>(w + F::tw_base(2), tw, t);
+    }
+    for (int r = r0; r < r1; ++r) {
+      const float2* A = Y + ((size_t)c * nb + r) * M;
+      if (r >= nb - s.P) {  // X_r into the delay line (older ones are already overwritten by newer)
+        const float4* src = reinterpret_cast<const float4*>(X + ((size_t)c * nb + r) * M);
+        int slot = (cur - 1 - r) % s.P;
+        if (slot < 0) slot += s.P;
+        float4* dst = reinterpret_cast<float4*>(s.fdl + ((size_t)c * s.P + slot) * M);
+#pragma unroll
+        for (int e = 0; e < NPAIR; ++e) dst[t + e * T] = src[t + e * T];
+      }
+      if (!y) continue;  // the same for every thread of the group: a channel's output is read or not
+      float2 v[E];
+#pragma unroll
+      for (int p = 0; p < NPAIR; ++p) {
+        const int i = p / (RL / 2) * RL + p % (RL / 2);
+        const int k = reg_out_index<LOG2M>(t, i), km = (k == 0) ? M / 2 : M - k;
+        const float2 a = A[k], b = A[km];
+        float2 zk, zm;
+        if (k == 0) {
+          zk = x_pre_dc(a, inv_n);
+          zm = x_pre_mid(b, inv_n);
+        } else {
+          x_pre(a, b, tw[k], inv_n, zk, zm);
+        }
+        if constexpr (F::SYM) v[i] = zk;
+        else buf0[F::pad(k)] = zk;
+        buf0[F::pad(km)] = zm;
+      }
+      sync();
+      if constexpr (F::SYM) {
+#pragma unroll
+        for (int i = 0; i < E; ++i)
+          if (i % F::R0 >= F::R0 / 2) v[i] = buf0[F::pad(reg_in_index<LOG2M>(t, i))];
+      } else {
+        reg_load<LOG2M, 0>(v, buf0, t);
+      }
+      if constexpr (!Sh::PP) sync();
+      reg_fft<LOG2M, true, Sh::WREG>(v, w, tw, buf1, buf0, t, sync);
+      float* yr = y + (size_t)r * M;
+#pragma unroll
+      for (int p = 0; p < NPAIR; ++p) {
+        const int i = p / (RL / 2) * RL + p % (RL / 2) + RL / 2, n = reg_out_index<LOG2M>(t, i) - M / 2;
+        if (y8) {
+          reinterpret_cast<float2*>(yr)[n] = v[i];
+        } else {
+          yr[2 * n] = v[i].x;
+          yr[2 * n + 1] = v[i].y;
+        }
+      }
+      if constexpr (Sh::PP && (F::NP & 1) != 0) {
+        float2* b = buf0;
+        buf0 = buf1;
+        buf1 = b;
+      }
+    }
+  }
+  signal_heads(sig, gridDim.x * gridDim.y);
+}
+
+// Output blocks of one run_mac_kernel CTA at most, bins per CTA, partition
+// chunks in flight and spectra each thread has in flight. A thread keeps NB sums
+// of one bin and the NB input spectra that a partition meets, so one partition
+// and one spectrum are loaded for NB products. The products (six
+// FP32 operations each; packed FP32 pairs issue at half the rate of two scalar
+// operations and made every form slower) are what bounds the kernel.
+constexpr int kRunBlocks = 8, kRunBins = 32, kRunRows = 8, kRunAhead = 4;
+
+template <bool DC>
+__device__ __forceinline__ float2 run_mac(float2 acc, float2 x, float2 h, bool dc) {
+  const float2 a = c_mac(acc, x, h);
+  if constexpr (!DC) return a;
+  const float2 b = c_mac_dc(acc, x, h);
+  return dc ? b : a;
+}
+
+// The spectra X_r of descending r of one bin: new blocks r >= 0 in the
+// workspace, older ones in the delay line (slot (cur + i) mod P holds X_{-1-i}).
+struct SpecWalk {
+  const float2* p;
+  const float2* fdl;
+  ptrdiff_t step;
+  int left, slot, B, P;
+  __device__ __forceinline__ SpecWalk(const float2* X, const float2* fdl_, int r, int cur, int B_, int P_)
+      : fdl(fdl_), B(B_), P(P_) {
+    slot = cur;
+    if (r >= 0) {
+      p = X + (size_t)r * B;
+      step = -(ptrdiff_t)B;
+      left = r + 1;
+    } else {
+      slot = cur - 1 - r;
+      if (slot >= P) slot -= P;
+      line();
+    }
+  }
+  __device__ __forceinline__ void line() {
+    p = fdl + (size_t)slot * B;
+    step = B;
+    left = P - slot;
+    slot = 0;  // where the line goes on after its end
+  }
+  __device__ __forceinline__ float2 next() {
+    const float2 v = *p;
+    p += step;
+    if (--left == 0) line();
+    return v;
+  }
+};
+
+// The products of one bin for output blocks b0 .. b0 + NB - 1, partition by
+// partition: the inputs a partition meets are a window over the spectra, one
+// more of which enters with each partition. Rounds of NB partitions turn the
+// window through the registers with compile-time positions; what is left of a
+// span moves it by hand. kRunAhead partitions' loads are in flight (past the
+// last partition they repeat its row, or go round the delay line, unused).
+template <int NB, bool DC>
+struct MacSpan {
+  static constexpr int A = kRunAhead;
+  static_assert(NB % A == 0, "the load queue turns with the window");
+  SpecWalk walk;
+  const float2* h;
+  int hleft;  // partitions after the one h points to
+  float2 win[NB];  // win[m] = X_{b0 + NB - 1 - i - m}, i the next partition (m = NB - 1 enters with it)
+  float2 hq[A], xq[A];
+  float2 acc[NB];
+
+  // starts at partition i0 of a row of P: X_r for r >= nb do not exist; the
+  // outputs that would read them are not stored
+  __device__ __forceinline__ MacSpan(const float2* H, const float2* fdl, const float2* X, int B, int P, int cur, int nb,
+                                     int b0, int i0)
+      : walk(X, fdl, min(nb - 1, b0 + NB - 1 - i0), cur, B, P), h(H + (size_t)i0 * B), hleft(P - 1 - i0) {
+    const int skip = max(0, b0 + NB - 1 - i0 - (nb - 1));
+#pragma unroll
+    for (int m = 0; m < NB - 1; ++m) {
+      win[m] = make_float2(0.f, 0.f);
+      if (m >= skip) win[m] = walk.next();
+    }
+#pragma unroll
+    for (int a = 0; a < A; ++a) fetch(a);
+    clear();
+  }
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int b = 0; b < NB; ++b) acc[b] = make_float2(0.f, 0.f);
+  }
+  __device__ __forceinline__ void fetch(int a) {
+    hq[a] = __ldg(h);
+    xq[a] = walk.next();
+    h += hleft > 0 ? walk.B : 0;
+    --hleft;
+  }
+  // n more partitions into the sums
+  __device__ __forceinline__ void run(int n, bool dc) {
+    for (; n >= NB; n -= NB) {
+#pragma unroll
+      for (int u = 0; u < NB; ++u) {
+        const float2 hv = hq[u % A];
+        win[(NB - 1 + u) % NB] = xq[u % A];
+        fetch(u % A);
+#pragma unroll
+        for (int b = 0; b < NB; ++b) acc[b] = run_mac<DC>(acc[b], win[(NB - 1 - b + u) % NB], hv, dc);
+      }
+    }
+#pragma unroll 1
+    for (; n > 0; --n) {
+      const float2 hv = hq[0];
+      win[NB - 1] = xq[0];
+#pragma unroll
+      for (int a = 0; a + 1 < A; ++a) {
+        hq[a] = hq[a + 1];
+        xq[a] = xq[a + 1];
+      }
+      fetch(A - 1);
+#pragma unroll
+      for (int b = 0; b < NB; ++b) acc[b] = run_mac<DC>(acc[b], win[NB - 1 - b], hv, dc);
+      const float2 first = win[0];
+#pragma unroll
+      for (int m = 0; m + 1 < NB; ++m) win[m] = win[m + 1];
+      win[NB - 1] = first;
+    }
+  }
+};
+
+template <int NB, bool DC, class D>
+__device__ __forceinline__ void run_mac_body(const DevState& s, const D& desc, const float2* __restrict__ X,
+                                             float2* __restrict__ Y, int nb, int per, int sy, int cur, int trow,
+                                             float2 (*red)[NB][kRunBins]) {
+  constexpr int NO = (NB + kRunRows - 1) / kRunRows;  // outputs a row finishes
+  const int c = blockIdx.y, tx = threadIdx.x, ty = threadIdx.y;
+  const int u = blockIdx.x * kRunBins + tx;
+  const int B = s.B, P = s.P;
+  const int b0 = blockIdx.z * per, b1 = min(nb + 1, b0 + per);  // output nb: the next call's first tail
+  const bool dc = (u == 0);
+  const ChanCtl cc = desc.get_ctl(c);
+  const float2* H = s.H + h_index(s, c, cc.slot_cur, 0) + u;
+  const float2* fdl = s.fdl + (size_t)c * P * B + u;
+  const float2* Xc = X + (size_t)c * nb * B + u;
+  if (blockIdx.z == 0 && ty == 0) {
+    // the last block's samples are the next call's history
+    const float* x = desc.get_in(c);
+    s.prev[(size_t)c * B + u] = x ? x[(size_t)(nb - 1) * B + u] : 0.f;
+  }
+  float2 tot[NO];
+#pragma unroll
+  for (int o = 0; o < NO; ++o) tot[o] = make_float2(0.f, 0.f);
+  const int nparts = max(0, P - 2), chunk = (nparts + sy - 1) / sy;
+  if (nparts > 0) {
+    for (int q0 = 0; q0 < sy; q0 += kRunRows) {
+      const int i0 = 2 + (q0 + ty) * chunk, i1 = min(P, i0 + chunk);
+      if (q0) __syncthreads();
+      if (i0 < i1) {
+        MacSpan<NB, DC> span(H, fdl, Xc, B, P, cur, nb, b0, i0);
+        span.run(i1 - i0, dc);
+#pragma unroll
+        for (int b = 0; b < NB; ++b) red[ty][b][tx] = span.acc[b];
+      } else {
+#pragma unroll
+        for (int b = 0; b < NB; ++b) red[ty][b][tx] = make_float2(0.f, 0.f);
+      }
+      __syncthreads();
+#pragma unroll
+      for (int o = 0; o < NO; ++o) {
+        const int b = ty + o * kRunRows;
+        if (b < NB) {
+          float2 a = red[0][b][tx];
+          if (q0) a = make_float2(__fadd_rn(tot[o].x, a.x), __fadd_rn(tot[o].y, a.y));
+#pragma unroll
+          for (int q = 1; q < kRunRows; ++q) {
+            const float2 r = red[q][b][tx];
+            a = make_float2(__fadd_rn(a.x, r.x), __fadd_rn(a.y, r.y));
+          }
+          tot[o] = a;
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int o = 0; o < NO; ++o) {
+    const int b = b0 + ty + o * kRunRows;
+    if (ty + o * kRunRows >= NB || b >= b1) continue;
+    if (b == nb) {
+      if (nparts > 0) s.tail[((size_t)c * 3 + trow) * B + u] = tot[o];
+      continue;
+    }
+    float2 a = tot[o];
+    if (P > 1) {
+      const float2 x = b > 0 ? Xc[(size_t)(b - 1) * B] : fdl[(size_t)cur * B];
+      a = dc ? c_mac_dc(a, x, H[B]) : c_mac(a, x, H[B]);
+    }
+    const float2 x = Xc[(size_t)b * B];
+    Y[((size_t)c * nb + b) * B + u] = dc ? c_mac_dc(a, x, H[0]) : c_mac(a, x, H[0]);
+  }
+}
+
+// The same sums for calls with enough work to fill the GPU: one warp takes all
+// partitions of NB output blocks of 64 bins (two a thread), and the warps of a
+// CTA are the output groups of the same bins, which share the rows they read.
+// Rows reach shared memory by asynchronous copies of 16 bytes a thread, stages
+// of kLineStage partitions, kLineDepth of them ahead: IR rows in a ring by
+// partition, input rows in a ring by q = top - r, X_top the newest spectrum the
+// CTA meets, so that group g's row for partition i is q = (G - 1 - g) NB + NB - 3
+// + i. The inner loop is one copy of code for every bin, stage and chunk: the
+// kernel runs for some twenty stages, and with the loop doubled for the packed
+// bin 0 and for chunk ends it waited for instructions (64 us at 64 channels of
+// 128 partitions of 512 and 32 blocks; with each warp loading its own rows into
+// registers 86 us).
+constexpr int kLineStage = 8, kLineDepth = 2, kLineGroups = 6, kLineBins = 64, kLineXRows = 64, kLineHRows = 32;
+
+// acc + x h for two bins; (h0, nh0, g0, k0): of the first bin, h.x, -h.y and
+// h.y, h.x, or for the packed bin 0 h.x, 0 and 0, h.y
+__device__ __forceinline__ float4 line_mac(float4 acc, float4 x, float4 h, float nh0, float g0, float k0) {
+  return make_float4(__fadd_rn(__fmaf_rn(x.x, h.x, __fmul_rn(x.y, nh0)), acc.x),
+                     __fadd_rn(__fmaf_rn(x.x, g0, __fmul_rn(x.y, k0)), acc.y),
+                     __fadd_rn(__fmaf_rn(x.z, h.z, -__fmul_rn(x.w, h.w)), acc.z),
+                     __fadd_rn(__fmaf_rn(x.z, h.w, __fmul_rn(x.w, h.z)), acc.w));
+}
+__device__ __forceinline__ float4 add4(float4 a, float4 b) {
+  return make_float4(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y), __fadd_rn(a.z, b.z), __fadd_rn(a.w, b.w));
+}
+
+template <int NB, class D>
+__global__ void __launch_bounds__(kLineGroups * 32, 4)
+    run_mac_line_kernel(DevState s, const __grid_constant__ D desc, const float2* __restrict__ Xw,
+                        float2* __restrict__ Y, int nb, int span, int sy, int cur, int trow) {
+  // rows in use (the groups' offsets, a window behind, a stage) and in flight
+  static_assert(kLineGroups * NB + (kLineDepth + 1) * kLineStage <= kLineXRows + 1, "input row ring");
+  static_assert((kLineDepth + 1) * kLineStage <= kLineHRows, "IR row ring");
+  __shared__ __align__(16) float4 xring[kLineXRows][32];
+  __shared__ __align__(16) float4 hring[kLineHRows][32];
+  const int c = blockIdx.y, lane = threadIdx.x & 31, grp = threadIdx.x >> 5, G = blockDim.x >> 5;
+  const int B = s.B, P = s.P, ub = blockIdx.x * kLineBins, u0 = ub + 2 * lane;
+  const int bs = blockIdx.z * span, be = min(nb + 1, bs + span);  // this CTA's outputs
+  const int b0 = bs + grp * NB;
+  const bool dc = u0 == 0;
+  const ChanCtl cc = desc.get_ctl(c);
+  const float2* H = s.H + h_index(s, c, cc.slot_cur, 0) + ub;
+  const float2* fdl = s.fdl + (size_t)c * P * B + ub;
+  const float2* X = Xw + (size_t)c * nb * B + ub;
+  if (bs == 0 && grp == 0) {
+    // the last block's samples are the next call's history
+    const float* x = desc.get_in(c);
+    float* prev = s.prev + (size_t)c * B + u0;
+    prev[0] = x ? x[(size_t)(nb - 1) * B + u0] : 0.f;
+    prev[1] = x ? x[(size_t)(nb - 1) * B + u0 + 1] : 0.f;
+  }
+  const int nparts = max(0, P - 2), chunk = (nparts + sy - 1) / sy;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 tot[NB];
+#pragma unroll
+  for (int b = 0; b < NB; ++b) tot[b] = zero;
+  auto mac = [&](float4& acc, float4 x, float4 h) {
+    acc = line_mac(acc, x, h, dc ? 0.f : -h.y, dc ? 0.f : h.y, dc ? h.y : h.x);
+  };
+  if (nparts > 0) {
+    const int top = bs + G * NB - 3;
+    auto copy16 = [](float4* dst, const float2* src) {
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                       static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(src) : "memory");
+    };
+    auto x_row = [&](int r) -> const float2* {
+      r = min(r, nb - 1);  // newer ones are read by outputs that are not stored
+      if (r >= 0) return X + (size_t)r * B;
+      int slot = cur - 1 - max(r, -P);
+      if (slot >= P) slot -= P;
+      return fdl + (size_t)slot * B;
+    };
+    // partitions i0 .. i0 + kLineStage - 1 and the input rows that enter group
+    // 0's window with them (past the last partition: its row again)
+    auto issue = [&](int i0) {
+      for (int v = threadIdx.x; v < kLineStage * 32; v += blockDim.x) {
+        const int i = i0 + (v >> 5), at = v & 31;
+        copy16(&hring[i & (kLineHRows - 1)][at], H + (size_t)min(i, P - 1) * B + 2 * at);
+        copy16(&xring[(top - bs + i) & (kLineXRows - 1)][at], x_row(bs - i) + 2 * at);
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    for (int v = threadIdx.x; v < (G * NB - 1) * 32; v += blockDim.x) {  // the first windows
+      const int q = v >> 5, at = v & 31;
+      copy16(&xring[q & (kLineXRows - 1)][at], x_row(top - q) + 2 * at);
+    }
+#pragma unroll 1
+    for (int d = 0; d < kLineDepth; ++d) issue(2 + d * kLineStage);
+    float4 acc[NB];
+#pragma unroll
+    for (int b = 0; b < NB; ++b) acc[b] = zero;
+    const int q0 = (G - 1 - grp) * NB + NB - 3;
+    int flush = 2 + chunk;  // partition before which the running chunk ends
+    int i = 2;
+#pragma unroll 1
+    for (int i0 = 2; i0 < P; i0 += kLineStage) {
+      // a copy group per stage, in order: all but the newest one have landed
+      asm volatile("cp.async.wait_group %0;" ::"n"(kLineDepth - 1) : "memory");
+      __syncthreads();  // and everyone is done with the stage before this one
+      issue(i0 + kLineDepth * kLineStage);
+      const int i1 = min(P, i0 + kLineStage);
+#pragma unroll 1
+      while (i < i1) {
+        const int n = min(i1, flush) - i;
+        const int q = q0 + i, hs = i & (kLineHRows - 1);
+        float4 win[NB];
+#pragma unroll
+        for (int m = 0; m < NB - 1; ++m) win[m] = xring[(q - (NB - 1) + m) & (kLineXRows - 1)][lane];
+#pragma unroll
+        for (int u = 0; u < kLineStage; ++u) {
+          if (u >= n) break;
+          const float4 h = hring[(hs + u) & (kLineHRows - 1)][lane];
+          win[(NB - 1 + u) % NB] = xring[(q + u) & (kLineXRows - 1)][lane];
+          const float nh0 = dc ? 0.f : -h.y, g0 = dc ? 0.f : h.y, k0 = dc ? h.y : h.x;
+#pragma unroll
+          for (int b = 0; b < NB; ++b) acc[b] = line_mac(acc[b], win[(NB - 1 - b + u) % NB], h, nh0, g0, k0);
+        }
+        i += n;
+        if (i == flush || i == P) {
+          flush += chunk;
+#pragma unroll
+          for (int b = 0; b < NB; ++b) {
+            tot[b] = add4(tot[b], acc[b]);
+            acc[b] = zero;
+          }
+        }
+      }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+  }
+#pragma unroll
+  for (int j = 0; j < NB; ++j) {
+    const int b = b0 + j;
+    if (b >= be) continue;
+    float4 a = tot[j];
+    if (b == nb) {  // the next call's first tail
+      if (nparts > 0) *reinterpret_cast<float4*>(s.tail + ((size_t)c * 3 + trow) * B + u0) = a;
+      continue;
+    }
+    const float4* Hl = reinterpret_cast<const float4*>(H) + lane;
+    if (P > 1) {
+      const float2* xp = b > 0 ? X + (size_t)(b - 1) * B : fdl + (size_t)cur * B;
+      mac(a, reinterpret_cast<const float4*>(xp)[lane], Hl[B / 2]);
+    }
+    mac(a, reinterpret_cast<const float4*>(X + (size_t)b * B)[lane], Hl[0]);
+    *reinterpret_cast<float4*>(Y + ((size_t)c * nb + b) * B + u0) = a;
+  }
+}
+
+template <int NB, class D>
+__global__ void __launch_bounds__(kRunBins* kRunRows)
+    run_mac_kernel(DevState s, const __grid_constant__ D desc, const float2* __restrict__ X, float2* __restrict__ Y,
+                   int nb, int per, int sy, int cur, int trow) {
+  __shared__ float2 red[kRunRows][NB][kRunBins];  // the chunks' sums
+  if (blockIdx.x == 0) run_mac_body<NB, true>(s, desc, X, Y, nb, per, sy, cur, trow, red);
+  else run_mac_body<NB, false>(s, desc, X, Y, nb, per, sy, cur, trow, red);
 }
 
 // ---------------------------------------------------------------------------
@@ -682,6 +1221,15 @@ constexpr int bulk_smem_bytes() {
   return 2 * NS * RS * BR * (int)sizeof(float2) + NS * 8;
 }
 
+template <int LOG2M, class D>
+cudaError_t set_run_attrs() {
+  cudaError_t e = cudaFuncSetAttribute(run_forward_kernel<LOG2M, D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       IrShape<LOG2M>::SMEM);
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(run_inverse_kernel<LOG2M, D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              IrShape<LOG2M>::SMEM);
+}
+
 template <int LOG2M>
 cudaError_t set_attrs() {
   constexpr int smem = HeadShape<LOG2M>::SMEM;
@@ -694,6 +1242,12 @@ cudaError_t set_attrs() {
   if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute(ir_spectrum_kernel<LOG2M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               IrShape<LOG2M>::SMEM);
+}
+
+template <int LOG2M>
+cudaError_t set_attrs_once() {
+  static OncePerDevice once;
+  return once.run([] { return set_attrs<LOG2M>(); });
 }
 
 // Partitions of an IR update that one group of threads takes in turn: enough to
@@ -725,6 +1279,58 @@ cudaError_t launch_head_t(const DevState& s, const BlockRef& d, int cur, int par
                     cur, parity, epi, sig);
   return launch_k(head_kernel<LOG2M, DevDesc>, dim3(s.C), dim3(T), smem, st, false, cv, s,
                   DevDesc{d.ctl, d.in, d.out}, cur, parity, epi, sig);
+}
+
+// Consecutive blocks one group of threads transforms in turn: enough that
+// twiddles and (for caller rows on the host bus) samples are read once, few
+// enough that every SM has work.
+constexpr int kRunMax = 8;
+
+// Warps from which run_mac_line_kernel takes the sums.
+constexpr int kRunLineWarps = 148 * 4;
+
+template <int LOG2M>
+cudaError_t launch_run_t(const DevState& s, const BlockRef& d, const RunShape& r, cudaStream_t st,
+                         const HeadSignal& sig) {
+  using Sh = IrShape<LOG2M>;
+  const int run = (int)std::max<long long>(1, std::min<long long>(kRunMax, (long long)s.C * r.nb / (Sh::G * 148LL * 2)));
+  const dim3 gf((r.nb + Sh::G * run - 1) / (Sh::G * run), s.C);
+  const int groups = (r.nb + 1 + kRunBlocks - 1) / kRunBlocks, per = (r.nb + 1 + groups - 1) / groups;
+  const dim3 gm(s.B / kRunBins, s.C, groups), bm(kRunBins, kRunRows);
+  auto go = [&](const auto& desc) {
+    using D = std::decay_t<decltype(desc)>;
+    static OncePerDevice once;
+    cudaError_t e = once.run([] { return set_run_attrs<LOG2M, D>(); });
+    if (e != cudaSuccess) return e;
+    e = launch_k(run_forward_kernel<LOG2M, D>, gf, dim3(Sh::THREADS), Sh::SMEM, st, false, -1, s, desc, r.X,
+                             r.nb, run);
+    if (e != cudaSuccess) return e;
+    if (s.B >= kLineBins && (long long)s.B / kLineBins * s.C * groups >= kRunLineWarps) {
+      // outputs (and the next call's first tail) over CTAs of at most
+      // kLineGroups groups of NB
+      const int n = r.nb + 1, NB = n <= 4 ? 4 : 6;
+      const int supers = (n + kLineGroups * NB - 1) / (kLineGroups * NB), span = ((n + supers - 1) / supers + NB - 1) / NB * NB;
+      const dim3 gl(s.B / kLineBins, s.C, (n + span - 1) / span);
+      auto line = [&](auto kernel) {
+        return launch_k(kernel, gl, dim3(32 * span / NB), 0, st, false, -1, s, desc, r.X, r.Y, r.nb, span, r.sy, r.cur,
+                        r.trow);
+      };
+      e = NB == 4 ? line(run_mac_line_kernel<4, D>) : line(run_mac_line_kernel<6, D>);
+      if (e != cudaSuccess) return e;
+      return launch_k(run_inverse_kernel<LOG2M, D>, gf, dim3(Sh::THREADS), Sh::SMEM, st, false, -1, s, desc, r.X, r.Y,
+                      r.nb, run, r.cur, sig);
+    }
+    auto mac = [&](auto kernel) {
+      return launch_k(kernel, gm, bm, 0, st, false, -1, s, desc, r.X, r.Y, r.nb, per, r.sy, r.cur, r.trow);
+    };
+    e = per <= 4 ? mac(run_mac_kernel<4, D>) : mac(run_mac_kernel<kRunBlocks, D>);
+    if (e != cudaSuccess) return e;
+    return launch_k(run_inverse_kernel<LOG2M, D>, gf, dim3(Sh::THREADS), Sh::SMEM, st, false, -1, s, desc, r.X, r.Y,
+                    r.nb, run, r.cur, sig);
+  };
+  if (d.stage) return go(StgDesc{*d.stage});
+  if (d.param) return go(ParDesc{*d.param});
+  return go(DevDesc{d.ctl, d.in, d.out});
 }
 
 #define TANB_DISPATCH_LOG2(L2, FN, ...)                          \
@@ -799,21 +1405,7 @@ constexpr int kTailCount = sizeof(kTail) / sizeof(kTail[0]);
 
 }  // namespace
 
-cudaError_t prepare_kernels() {
-  static OncePerDevice once;
-  return once.run([] {
-    cudaError_t e;
-    if ((e = set_attrs<5>()) != cudaSuccess) return e;
-    if ((e = set_attrs<6>()) != cudaSuccess) return e;
-    if ((e = set_attrs<7>()) != cudaSuccess) return e;
-    if ((e = set_attrs<8>()) != cudaSuccess) return e;
-    if ((e = set_attrs<9>()) != cudaSuccess) return e;
-    if ((e = set_attrs<10>()) != cudaSuccess) return e;
-    if ((e = set_attrs<11>()) != cudaSuccess) return e;
-    if ((e = set_attrs<12>()) != cudaSuccess) return e;
-    return set_attrs<13>();
-  });
-}
+cudaError_t prepare_kernels(int log2B) { TANB_DISPATCH_LOG2(log2B, set_attrs_once); }
 
 cudaError_t launch_ir_spectrum(const DevState& s, const IrRows& ir, const int* chans, int nch,
                                const ChanCtl* ctl, cudaStream_t st) {
@@ -834,6 +1426,11 @@ cudaError_t launch_tail(const DevState& s, const BlockRef& d, int which, int cur
         kTail[i].t.kind == t.kind)
       return kTail[i].fn(s, d, which, cur, trow, st, pdl);
   return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_run(const DevState& s, const BlockRef& d, const RunShape& r, cudaStream_t st,
+                       const HeadSignal& sig) {
+  TANB_DISPATCH_LOG2(s.log2B, launch_run_t, s, d, r, st, sig);
 }
 
 int mac_tiling_count() { return kTailCount; }

@@ -143,7 +143,9 @@ extern "C" int32_t tanb_convolve_no_alloc(const float* in, const float* ir, floa
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   unsigned char* base = nullptr;
   cudaError_t e = scratch_base(&base);
-  if (e == cudaSuccess) e = tanb::prepare_kernels();
+  int log2B = 0;
+  while ((1 << log2B) < (int)B) ++log2B;
+  if (e == cudaSuccess) e = tanb::prepare_kernels(log2B);
   if (e != cudaSuccess) {
     tanb::set_last_error(cudaGetErrorString(e));
     return TANB_FAIL;
@@ -151,7 +153,7 @@ extern "C" int32_t tanb_convolve_no_alloc(const float* in, const float* ir, floa
   float2* tw = reinterpret_cast<float2*>(base + o_tw);
   tanb::DevState s{};
   s.B = (int)B;
-  while ((1 << s.log2B) < (int)B) ++s.log2B;
+  s.log2B = log2B;
   s.P = (int)P;
   s.C = (int)C;
   s.H = reinterpret_cast<float2*>(base + o_H);
