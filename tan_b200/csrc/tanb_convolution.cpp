@@ -176,11 +176,13 @@ struct tanb_convolution {
   bool td = false;
   float* td_hist = nullptr;    // [C][length]
   float* td_ir = nullptr;      // [2 slots][C][length]  (Process IRs)
-  float* td_dir = nullptr;     // [C][length]           (ProcessDirect per-call IRs)
-  float* td_io = nullptr;      // [2][C][length]        (device in / out staging)
-  float* h_td = nullptr;       // pinned [3][C][length] (IR, in, out staging)
-  tanb::TdChan* d_tdchan = nullptr;
-  tanb::TdChan* h_tdchan = nullptr;
+  // A call's descriptors, ProcessDirect's IR rows and host input rows lie in
+  // one block, pinned (h_td) and on the device (d_td), so that one transfer
+  // takes what the call uses of it; host output rows are written in place in
+  // pinned memory.
+  char* h_td = nullptr;        // pinned: TdChan[C], then [2][C][length] floats
+  char* d_td = nullptr;
+  float* h_td_out = nullptr;   // pinned [C][length]
   std::vector<int> td_pos;
   int td_fade = -1;            // crossfade sample index, -1 when none
   std::vector<int> td_swapping;
@@ -294,13 +296,11 @@ void free_all(tanb_convolution* v) {
   v->staging_busy = false;
   cudaFree(v->td_hist);
   cudaFree(v->td_ir);
-  cudaFree(v->td_dir);
-  cudaFree(v->td_io);
-  cudaFree(v->d_tdchan);
+  cudaFree(v->d_td);
   cudaFreeHost(v->h_td);
-  cudaFreeHost(v->h_tdchan);
-  v->td_hist = v->td_ir = v->td_dir = v->td_io = v->h_td = nullptr;
-  v->d_tdchan = v->h_tdchan = nullptr;
+  cudaFreeHost(v->h_td_out);
+  v->td_hist = v->td_ir = v->h_td_out = nullptr;
+  v->d_td = v->h_td = nullptr;
   if (v->ev_stage) cudaEventDestroy(v->ev_stage);
   if (v->ev_ir) cudaEventDestroy(v->ev_ir);
   if (v->ev_out) cudaEventDestroy(v->ev_out);
@@ -361,6 +361,24 @@ int32_t run_pending_finalize(tanb_convolution* v) {
                                                v->stream);
                     }));
   return TANB_OK;
+}
+
+// True when no input row of n samples touches a byte between the first and the
+// last output row (null rows aside).
+bool spans_apart(const float* const* in, float* const* out, int C, size_t n) {
+  uintptr_t il = UINTPTR_MAX, ih = 0, ol = UINTPTR_MAX, oh = 0;
+  for (int c = 0; c < C; ++c) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(in[c]), b = reinterpret_cast<uintptr_t>(out[c]);
+    if (a) {
+      il = std::min(il, a);
+      ih = std::max(ih, a + n * sizeof(float));
+    }
+    if (b) {
+      ol = std::min(ol, b);
+      oh = std::max(oh, b + n * sizeof(float));
+    }
+  }
+  return il >= oh || ol >= ih;
 }
 
 int32_t td_update(tanb_convolution* v, Mem mem, const float* const* ir, size_t n, const uint32_t* flags,
@@ -738,21 +756,9 @@ int ensure_run(tanb_convolution* v, size_t nb, float2** work) {
 // apart, or every channel's output is its own input row: reading all inputs
 // before writing any output then gives what block-by-block processing gives.
 bool rows_apart(const float* const* in, float* const* out, int C, size_t n) {
-  uintptr_t il = UINTPTR_MAX, ih = 0, ol = UINTPTR_MAX, oh = 0;
+  if (spans_apart(in, out, C, n)) return true;
   bool same = true;
-  for (int c = 0; c < C; ++c) {
-    const uintptr_t a = reinterpret_cast<uintptr_t>(in[c]), b = reinterpret_cast<uintptr_t>(out[c]);
-    same = same && a == b;
-    if (a) {
-      il = std::min(il, a);
-      ih = std::max(ih, a + n * sizeof(float));
-    }
-    if (b) {
-      ol = std::min(ol, b);
-      oh = std::max(oh, b + n * sizeof(float));
-    }
-  }
-  if (il >= oh || ol >= ih) return true;
+  for (int c = 0; c < C; ++c) same = same && in[c] == out[c];
   if (!same) return false;
   // in place: the rows must not overlap one another
   std::vector<uintptr_t> r;
@@ -1336,16 +1342,20 @@ int32_t nu_process(tanb_convolution* v, Mem in_mem, const float* const* in, Mem 
 // TIME_DOMAIN method (ConvolutionImpl.cpp:407-468, 721-762, 2645-2782)
 // ---------------------------------------------------------------------------
 
+// Rows of a direct call of at least this many bytes are staged on the host pool.
+constexpr size_t kTdParallelBytes = 256u << 10;
+
+// Bytes of the call descriptors in front of the rows.
+size_t td_desc_bytes(size_t C) { return (C * sizeof(tanb::TdChan) + 255) & ~size_t(255); }
+
 cudaError_t td_alloc(tanb_convolution* v) {
-  const size_t C = v->C, len = v->length;
+  const size_t C = v->C, len = v->length, block = td_desc_bytes(C) + 2 * C * len * sizeof(float);
   cudaError_t e;
   if ((e = dev_alloc(v, &v->td_hist, C * len)) != cudaSuccess) return e;
   if ((e = dev_alloc(v, &v->td_ir, 2 * C * len)) != cudaSuccess) return e;
-  if ((e = dev_alloc(v, &v->td_dir, C * len)) != cudaSuccess) return e;
-  if ((e = dev_alloc(v, &v->td_io, 2 * C * len)) != cudaSuccess) return e;
-  if ((e = dev_alloc(v, &v->d_tdchan, C)) != cudaSuccess) return e;
-  if ((e = cudaMallocHost(&v->h_td, 3 * C * len * sizeof(float))) != cudaSuccess) return e;
-  if ((e = cudaMallocHost(&v->h_tdchan, C * sizeof(tanb::TdChan))) != cudaSuccess) return e;
+  if ((e = dev_alloc(v, &v->d_td, block)) != cudaSuccess) return e;
+  if ((e = cudaMallocHost(&v->h_td, block)) != cudaSuccess) return e;
+  if ((e = cudaMallocHost(&v->h_td_out, C * len * sizeof(float))) != cudaSuccess) return e;
   v->td_pos.assign(C, 0);
   v->td_fade = -1;
   v->td_swapping.assign(C, 0);
@@ -1373,7 +1383,7 @@ int32_t td_update(tanb_convolution* v, Mem mem, const float* const* ir, size_t n
     }
     float* dst = td_ir_row(v, v->slot_new[c], c);
     if (mem == Mem::Host) {
-      float* row = v->h_td + (size_t)c * len;
+      float* row = reinterpret_cast<float*>(v->h_td + td_desc_bytes(v->C)) + (size_t)c * len;
       if (n) tanb::copy_for_device(row, ir[c], n * sizeof(float));
       std::memset(row + n, 0, (len - n) * sizeof(float));
       TANB_CUDA(cudaMemcpyAsync(dst, row, len * sizeof(float), cudaMemcpyHostToDevice, v->stream));
@@ -1386,26 +1396,30 @@ int32_t td_update(tanb_convolution* v, Mem mem, const float* const* ir, size_t n
   return TANB_OK;
 }
 
-// Runs one TIME_DOMAIN call: the descriptors in h_tdchan are filled; inputs
-// are staged (host) or referenced (device); outputs go to staging (host).
-int32_t td_launch(tanb_convolution* v, int n, bool host_in, bool host_out, float* const* out) {
+// Runs one TIME_DOMAIN call of n samples: the descriptors are in h_td and, behind
+// them, `rows` floats of IR and input rows that the descriptors point to on the
+// device. Host outputs are written to h_td_out, rows of n samples. `overlap`:
+// output rows may overlap input rows.
+int32_t td_launch(tanb_convolution* v, int n, size_t rows, bool overlap, float* const* host_out) {
   const size_t C = v->C, len = v->length;
-  float* h_in = v->h_td + C * len;
-  float* h_out = v->h_td + 2 * C * len;
-  if (host_in)
-    TANB_CUDA(cudaMemcpyAsync(v->td_io, h_in, C * len * sizeof(float), cudaMemcpyHostToDevice, v->stream));
-  TANB_CUDA(cudaMemcpyAsync(v->d_tdchan, v->h_tdchan, C * sizeof(tanb::TdChan), cudaMemcpyHostToDevice,
-                            v->stream));
-  TANB_CUDA(counted(v, tanb_convolution::kTail,
-                    [&] { return tanb::launch_td(v->td_hist, (int)len, v->d_tdchan, (int)C, n, v->B, v->stream); }));
-  if (host_out) {
-    TANB_CUDA(cudaMemcpyAsync(h_out, v->td_io + C * len, C * len * sizeof(float), cudaMemcpyDeviceToHost,
-                              v->stream));
+  const tanb::TdChan* h_ch = reinterpret_cast<const tanb::TdChan*>(v->h_td);
+  const tanb::TdChan* d_ch = reinterpret_cast<const tanb::TdChan*>(v->d_td);
+  if (overlap) {
+    // the inputs enter the history first, from descriptors that still hold them
+    TANB_CUDA(cudaMemcpyAsync(v->d_td, v->h_td, C * sizeof(tanb::TdChan), cudaMemcpyHostToDevice, v->stream));
+    TANB_CUDA(tanb::launch_td_insert(v->td_hist, (int)len, d_ch, (int)C, n, v->stream));
+    TANB_CUDA(cudaStreamSynchronize(v->stream));
+    for (size_t c = 0; c < C; ++c) reinterpret_cast<tanb::TdChan*>(v->h_td)[c].in = nullptr;
   }
+  const size_t bytes = rows ? td_desc_bytes(C) + rows * sizeof(float) : C * sizeof(tanb::TdChan);
+  TANB_CUDA(cudaMemcpyAsync(v->d_td, v->h_td, bytes, cudaMemcpyHostToDevice, v->stream));
+  TANB_CUDA(counted(v, tanb_convolution::kTail, [&] {
+    return tanb::launch_td(v->td_hist, (int)len, d_ch, (int)C, n, v->B, v->stream);
+  }));
   TANB_CUDA(cudaStreamSynchronize(v->stream));
   if (host_out)
     for (size_t c = 0; c < C; ++c)
-      if (v->h_tdchan[c].run && out[c]) std::memcpy(out[c], h_out + c * len, n * sizeof(float));
+      if (h_ch[c].run && host_out[c]) std::memcpy(host_out[c], v->h_td_out + c * n, n * sizeof(float));
   return TANB_OK;
 }
 
@@ -1430,9 +1444,11 @@ int32_t td_process(tanb_convolution* v, Mem in_mem, const float* const* in, Mem 
     }
     if (any) v->td_fade = 0;
   }
-  float* h_in = v->h_td + C * len;
+  tanb::TdChan* h_ch = reinterpret_cast<tanb::TdChan*>(v->h_td);
+  float* h_rows = reinterpret_cast<float*>(v->h_td + td_desc_bytes(C));
+  const float* d_rows = reinterpret_cast<const float*>(v->d_td + td_desc_bytes(C));
   for (size_t c = 0; c < C; ++c) {
-    tanb::TdChan& t = v->h_tdchan[c];
+    tanb::TdChan& t = h_ch[c];
     t = tanb::TdChan{};
     t.run = run[c];
     t.pos = v->td_pos[c];
@@ -1443,14 +1459,16 @@ int32_t td_process(tanb_convolution* v, Mem in_mem, const float* const* in, Mem 
     t.swap = (v->td_fade >= 0 && v->td_swapping[c]) ? 1 : 0;
     t.fade0 = v->td_fade < 0 ? 0 : v->td_fade;
     if (in_mem == Mem::Host) {
-      t.in = in[c] ? v->td_io + c * len : nullptr;
-      if (in[c] && run[c]) tanb::copy_for_device(h_in + c * len, in[c], ns * sizeof(float));
+      t.in = in[c] ? d_rows + c * ns : nullptr;
+      if (in[c] && run[c]) tanb::copy_for_device(h_rows + c * ns, in[c], ns * sizeof(float));
     } else {
       t.in = in[c];
     }
-    t.out = out_mem == Mem::Host ? v->td_io + (C + c) * len : out[c];
+    t.out = out_mem == Mem::Host ? v->h_td_out + c * ns : out[c];
   }
-  int32_t r = td_launch(v, ns, in_mem == Mem::Host, out_mem == Mem::Host, out);
+  const bool overlap = in_mem == Mem::Device && out_mem == Mem::Device && !spans_apart(in, out, (int)C, ns);
+  int32_t r = td_launch(v, ns, in_mem == Mem::Host ? C * ns : 0, overlap,
+                        out_mem == Mem::Host ? out : nullptr);
   if (r != TANB_OK) return r;
   for (size_t c = 0; c < C; ++c)
     if (run[c]) v->td_pos[c] = (int)((v->td_pos[c] + ns) % len);
@@ -1482,27 +1500,38 @@ int32_t td_process_direct(tanb_convolution* v, const float* const* ir, const flo
   }
   if (n == 0) return TANB_OK;
   TANB_CUDA(cudaStreamSynchronize(v->stream));
-  float* h_in = v->h_td + C * len;
+  // compact rows behind the descriptors: the inputs, then each channel's taps
+  // in use
+  tanb::TdChan* h_ch = reinterpret_cast<tanb::TdChan*>(v->h_td);
+  float* h_rows = reinterpret_cast<float*>(v->h_td + td_desc_bytes(C));
+  const float* d_rows = reinterpret_cast<const float*>(v->d_td + td_desc_bytes(C));
+  size_t at = C * n;
   for (size_t c = 0; c < C; ++c) {
     const int first = nz ? nz[2 * c] : 0, last = nz ? nz[2 * c + 1] : (int)len;
-    float* row = v->h_td + c * len;
-    if (last > first) {
-      tanb::copy_for_device(row + first, ir[c] + first, (last - first) * sizeof(float));
-      TANB_CUDA(cudaMemcpyAsync(v->td_dir + c * len + first, row + first, (last - first) * sizeof(float),
-                                cudaMemcpyHostToDevice, v->stream));
-    }
-    tanb::copy_for_device(h_in + c * len, in[c], n * sizeof(float));
-    tanb::TdChan& t = v->h_tdchan[c];
+    const int taps = last - first;
+    tanb::TdChan& t = h_ch[c];
     t = tanb::TdChan{};
     t.run = 1;
     t.pos = v->td_pos[c];
     t.first = first;
     t.last = last;
-    t.ir = v->td_dir + c * len;
-    t.in = v->td_io + c * len;
-    t.out = v->td_io + (C + c) * len;
+    // addressed by tap number: the row holds taps [first, last) alone
+    t.ir = reinterpret_cast<const float*>(reinterpret_cast<uintptr_t>(d_rows + at) - (uintptr_t)first * sizeof(float));
+    t.in = d_rows + c * n;
+    t.out = v->h_td_out + c * n;
+    at += taps;
   }
-  int32_t r = td_launch(v, (int)n, true, true, out);
+  auto stage = [&](int c) {
+    const tanb::TdChan& t = h_ch[c];
+    const size_t row = (size_t)(t.ir + t.first - d_rows);  // where the taps go
+    tanb::copy_for_device(h_rows + row, ir[c] + t.first, (size_t)(t.last - t.first) * sizeof(float));
+    tanb::copy_for_device(h_rows + c * n, in[c], n * sizeof(float));
+  };
+  if (at * sizeof(float) >= kTdParallelBytes)
+    tanb::host_parallel_for((int)C, stage);
+  else
+    for (size_t c = 0; c < C; ++c) stage((int)c);
+  int32_t r = td_launch(v, (int)n, at, false, out);
   if (r != TANB_OK) return r;
   for (size_t c = 0; c < C; ++c) v->td_pos[c] = (int)((v->td_pos[c] + n) % len);
   if (done) *done = n;
