@@ -1263,8 +1263,18 @@ int32_t nu_process(tanb_convolution* v, Mem in_mem, const float* const* in, Mem 
   const bool tables = in_mem == Mem::Device || out_mem == Mem::Device;
   size_t processed = 0;
   int32_t status = TANB_OK;
+  // Device rows of several blocks, no channel changing state inside the call: as
+  // one launch sequence over the engine's levels where it allows (an update's
+  // block goes one by one first).
+  bool many = !host_io && nblocks > 1;
+  for (int c = 0; many && flags && c < C; ++c) many = (flags[c] & kStopInput) == 0;
+  many = many && rows_apart(in, out, C, nblocks * (size_t)B);
+  const int overlap = !host_io && !spans_apart(in, out, C, nblocks * (size_t)B);
   while (processed < nblocks && status == TANB_OK) {
-    const int nb = host_io ? 1 : (int)std::min<size_t>(kNuBlocksPerChunk, nblocks - processed);
+    const int next = many ? tanb::engine_run_fit(v->nu_eng, v->nu_sess, nblocks - processed) : -1;
+    const int fit = std::max(next, 0);
+    // one row table for a sequence or a block by itself, else one per block
+    const int nb = host_io || next >= 0 ? 1 : (int)std::min<size_t>(kNuBlocksPerChunk, nblocks - processed);
     TANB_CUDA(cudaEventSynchronize(v->ev_stage));  // the previous chunk's tables have been uploaded
     // pass 1: channel flags of every block of the chunk and its row tables
     int filled = 0;
@@ -1300,6 +1310,7 @@ int32_t nu_process(tanb_convolution* v, Mem in_mem, const float* const* in, Mem 
       }
       tanb::EngRows rows;
       rows.ld = B;
+      rows.overlap = overlap;
       if (in_mem == Mem::Host) {
         // free channels and missing rows read silence
         for (int c = 0; c < C; ++c) {
@@ -1319,7 +1330,16 @@ int32_t nu_process(tanb_convolution* v, Mem in_mem, const float* const* in, Mem 
       else
         rows.out_tab = reinterpret_cast<float* const*>(const_cast<float**>(v->d_nu_tab + (size_t)(2 * b + 1) * C));
       int32_t r;
-      if (in_mem == Mem::Host && out_mem == Mem::Host) {
+      if (fit) {
+        int ran = 0;
+        r = tanb::engine_run_blocks(v->nu_eng, v->nu_sess, rows, (size_t)fit, &ran);
+        if (r == TANB_OK && ran != fit) r = fail(TANB_FAIL, "non-uniform blocks: %d of %d ran", ran, fit);
+        // the flags of the blocks after the first: every channel runs, none flushes
+        for (int q = 1; r == TANB_OK && q < fit; ++q) channel_flags(v, flags, v->scr_run, v->scr_flush);
+        filled = fit;
+        if (r != TANB_OK) return r;
+        break;
+      } else if (in_mem == Mem::Host && out_mem == Mem::Host) {
         r = tanb_engine_process(v->nu_eng);  // the engine's graph over its pinned rows; waits for the output
       } else {
         r = tanb::engine_process_rows(v->nu_eng, rows);

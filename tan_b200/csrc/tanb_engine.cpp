@@ -178,7 +178,7 @@ struct tanb_engine {
   EngLevel* h_levels = nullptr;
   std::vector<RangeAlloc> lvl_alloc;
   std::vector<size_t> lvl_hwm;
-  std::vector<float2*> d_tw_lv;       // twiddles of each size class (2N entries)
+  std::vector<float2*> d_tw_lv;       // each size class's table of the register passes (2N entries)
   float* h_in = nullptr;   // pinned; read in place by the heads
   float* h_out = nullptr;  // pinned; written in place by the heads
   long long* d_block = nullptr;     // blocks processed (device)
@@ -191,7 +191,8 @@ struct tanb_engine {
   EngUpd* d_upd = nullptr;
   EngLvlUpd* h_lupd = nullptr;
   EngLvlUpd* d_lupd = nullptr;
-  float2* d_tw = nullptr;
+  float2* d_tw = nullptr;     // the block kernel's twiddles (2B entries)
+  float2* d_tw_ir = nullptr;  // the IR transforms' (the register passes' table, 2B entries)
   int tail_grid = 0;
   int sms = 148;  // SMs of the device
   size_t nslots_hwm = 0, nitems_hwm = 0;
@@ -265,6 +266,10 @@ int level_class(const tanb_engine* e, int log2N) { return log2N - e->log2B - 1; 
 
 constexpr size_t kMaxRetiredGraphs = 64;
 
+// Blocks from which a launch sequence over several blocks (a launch or two per
+// level, whatever their number) replaces one launch or more per block.
+constexpr size_t kRunMinBlocks = 4;
+
 void destroy_retired(tanb_engine* e) {
   for (cudaGraphExec_t g : e->retired) cudaGraphExecDestroy(g);
   e->retired.clear();
@@ -294,6 +299,7 @@ void free_engine(tanb_engine* e) {
   cudaFree(e->d_upd);
   cudaFree(e->d_lupd);
   cudaFree(e->d_tw);
+  cudaFree(e->d_tw_ir);
   for (float2* t : e->d_tw_lv) cudaFree(t);
   cudaFreeHost(e->h_chans);
   cudaFreeHost(e->h_items);
@@ -459,9 +465,13 @@ cudaError_t enqueue_block(tanb_engine* e, const tanb::EngRows& rows, unsigned du
   // memory (the latency of the heads bounds such a launch); more heads share
   // them in L1 (the item CTAs' streaming bounds it)
   const bool tw_stage = e->nslots_hwm <= 2 * (size_t)e->sms;
-  r = tanb::eng_launch_block(e->log2B, e->spec, e->d_chans, (int)e->nslots_hwm, e->d_items, (int)e->nitems_hwm, tc,
-                             e->d_levels, rows, e->d_tw, tw_stage, sync, total, e->stream);
-  if (r != cudaSuccess || !due) return r;
+  auto block = [&] {
+    return tanb::eng_launch_block(e->log2B, e->spec, e->d_chans, (int)e->nslots_hwm, e->d_items, (int)e->nitems_hwm,
+                                  tc, e->d_levels, rows, e->d_tw, tw_stage, sync, total, e->stream);
+  };
+  // the block launch first, so that the level heads take the SMs it leaves; after
+  // them where its outputs may overwrite inputs that they read
+  if (!(due && rows.overlap) && (r = block()) != cudaSuccess) return r;
   for (int c = 0; c < e->nclass; ++c) {
     if (!(due >> c & 1u)) continue;
     r = tanb::eng_launch_level_heads(e->log2B, e->log2B + 1 + c, e->spec, e->d_chans, (int)e->nslots_hwm,
@@ -471,7 +481,7 @@ cudaError_t enqueue_block(tanb_engine* e, const tanb::EngRows& rows, unsigned du
     if ((r = cudaEventRecord(e->ev_joins[c], e->lstreams[c])) != cudaSuccess) return r;
     if ((r = cudaStreamWaitEvent(e->stream, e->ev_joins[c], 0)) != cudaSuccess) return r;
   }
-  return cudaSuccess;
+  return due && rows.overlap ? block() : cudaSuccess;
 }
 
 std::vector<size_t> graph_key(const tanb_engine* e) {
@@ -856,7 +866,7 @@ int32_t engine_update(tanb_engine* e, int32_t session, const float* const* ir, s
     for (int q = 0; q < nch; ++q) e->h_upd[q].src = e->d_ir + (size_t)q * n;
   }
   ENG_CUDA(cudaMemcpyAsync(e->d_upd, e->h_upd, nch * sizeof(EngUpd), cudaMemcpyHostToDevice, e->upd_stream));
-  ENG_CUDA(tanb::eng_launch_ir(e->log2B, e->spec, e->d_chans, e->d_upd, nch, s.P, e->d_tw, e->upd_stream));
+  ENG_CUDA(tanb::eng_launch_ir(e->log2B, e->spec, e->d_chans, e->d_upd, nch, s.P, e->d_tw_ir, e->upd_stream));
   // the levels of a non-uniform session, one transform launch per level
   for (size_t l = 0; l < s.lv.size(); ++l) {
     const int c = level_class(e, s.lv[l].log2N);
@@ -915,6 +925,75 @@ int32_t run_block(tanb_engine* e, const tanb::EngRows* rows) {
   return TANB_OK;
 }
 
+// Blocks of the next launch sequence over several blocks of the engine's only
+// session (tanb_engine_kernels.cu, eng_run_*), of at most `nb`: 0 when the next
+// block has to go by itself (an update takes effect on it), -1 when all do.
+// Non-uniform, FP32 spectra, at most two partitions in the base level; a sequence
+// stays within one
+// period of the largest level and of every level with work items, so that each
+// of those has at most one head in it and its partial rows are those of two
+// level blocks (two parities).
+int run_blocks_fit(tanb_engine* e, const Session& s, size_t nb) {
+  if (e->spec != tanb::kSpecFP32 || s.lv.empty() || s.nitem || nb < kRunMinBlocks) return -1;
+  for (const LevelSpec& l : s.lv)
+    if (l.ngroup && (1u << (l.log2N - e->log2B)) < kRunMinBlocks) return -1;
+  if (s.staged) return 0;
+  for (int j = 0; j < s.C; ++j)
+    if (e->h_chans[s.slot0 + j].pending) return 0;
+  const long long t0 = e->k_host << e->log2B;
+  size_t fit = nb;
+  long long off = 0, reach = 0;
+  for (const LevelSpec& l : s.lv) {
+    const long long N = 1LL << l.log2N;
+    if (l.ngroup || &l == &s.lv.back()) fit = std::min(fit, (size_t)(N >> e->log2B));
+    // a sample's sum takes the levels in order, those with a head for it in this
+    // sequence before those whose rings hold it: where the latter begin has to
+    // grow with the level
+    off = l.off + t0 / N * N;
+    if (off < reach) return 0;
+    reach = off;
+  }
+  return fit >= kRunMinBlocks ? (int)fit : -1;
+}
+
+// One launch sequence over nb blocks (as run_blocks_fit allows) of the engine's
+// only session: rows hold the blocks back to back. Caller holds mu.
+cudaError_t run_blocks(tanb_engine* e, Session& s, const tanb::EngRows& rows, int nb) {
+  const long long k0 = e->k_host;
+  const int ns = (int)e->nslots_hwm;
+  cudaError_t r = tanb::eng_launch_run_input(e->log2B, e->d_chans, ns, rows, k0, nb, e->stream);
+  if (r == cudaSuccess) r = tanb::eng_launch_run_base(e->log2B, e->d_chans, ns, rows, e->d_tw, k0, nb, e->stream);
+  for (size_t l = 0; l < s.lv.size() && r == cudaSuccess; ++l) {
+    const LevelSpec& ls = s.lv[l];
+    const int c = level_class(e, ls.log2N), pshift = ls.log2N - e->log2B, nlev = (int)e->lvl_hwm[c];
+    const EngLevel* lv = e->d_levels + (size_t)c * e->max_channels;
+    const long long j0 = k0 >> pshift;                       // first head at or after block k0
+    const int m = (int)(((k0 + nb) >> pshift) - j0);         // heads in the sequence
+    // work items of blocks up to the head, the head, those of the blocks after it
+    // (whose rows are the ones the head has read)
+    const long long kh = m && ls.ngroup ? std::min(k0 + nb, (j0 + 1) << pshift) : k0 + nb;
+    const int nit = s.C * s.items_per_chan, grid = std::min<long long>(e->tail_grid, (long long)nit * nb);
+    if (ls.ngroup)
+      r = tanb::eng_launch_run_items(e->log2B, e->d_chans, e->d_levels, e->d_items, (int)s.item0, nit, ls.log2N, k0,
+                                     (int)(kh - k0), grid, e->stream);
+    const bool with_ring = (long long)nb * e->B + ls.off <= ls.R;
+    if (r == cudaSuccess && !with_ring)
+      r = tanb::eng_launch_run_ring(e->log2B, e->d_chans, lv, nlev, rows, k0, nb, j0, e->stream);
+    if (r == cudaSuccess && (m || with_ring))
+      r = tanb::eng_launch_run_level(e->log2B, ls.log2N, e->d_chans, lv, nlev, rows, e->d_tw_lv[c], k0, nb, j0, m,
+                                     with_ring, e->stream);
+    if (r == cudaSuccess && ls.ngroup)
+      r = tanb::eng_launch_run_items(e->log2B, e->d_chans, e->d_levels, e->d_items, (int)s.item0, nit, ls.log2N, kh,
+                                     (int)(k0 + nb - kh), grid, e->stream);
+  }
+  if (r == cudaSuccess)
+    r = tanb::eng_launch_run_end(e->d_chans, ns, tanb::EngSync{e->d_block, e->d_done}, nb, e->stream);
+  if (r != cudaSuccess) return r;
+  e->n_block += nb;
+  for (int b = 0; b < nb; ++b) advance_mirror(e);
+  return cudaSuccess;
+}
+
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -951,6 +1030,25 @@ int32_t engine_process_rows(tanb_engine* e, const EngRows& rows) {
   ENG_CUDA(cudaSetDevice(e->ctx->device));
   if (e->sessions.empty()) return efail(TANB_WRONG_STATE, "no open sessions");
   return run_block(e, &rows);
+}
+
+int32_t engine_run_blocks(tanb_engine* e, int32_t session, const EngRows& rows, size_t nb, int* done) {
+  *done = 0;
+  std::lock_guard<std::mutex> lock(e->mu);
+  ENG_CUDA(cudaSetDevice(e->ctx->device));
+  auto it = e->sessions.find(session);
+  if (it == e->sessions.end() || e->sessions.size() != 1) return TANB_OK;
+  const int fit = run_blocks_fit(e, it->second, nb);
+  if (fit <= 0) return TANB_OK;
+  ENG_CUDA(run_blocks(e, it->second, rows, fit));
+  *done = fit;
+  return TANB_OK;
+}
+
+int engine_run_fit(tanb_engine* e, int32_t session, size_t nb) {
+  std::lock_guard<std::mutex> lock(e->mu);
+  auto it = e->sessions.find(session);
+  return it == e->sessions.end() || e->sessions.size() != 1 ? -1 : run_blocks_fit(e, it->second, nb);
 }
 
 }  // namespace tanb
@@ -1004,6 +1102,7 @@ int32_t tanb_engine_create(tanb_context* ctx, uint32_t block, uint32_t spectrum,
   if (r == cudaSuccess) r = cudaMalloc(&e->d_upd, e->max_channels * sizeof(EngUpd));
   if (r == cudaSuccess) r = cudaMalloc(&e->d_lupd, tanb::kMaxLevels * e->max_channels * sizeof(EngLvlUpd));
   if (r == cudaSuccess) r = cudaMalloc(&e->d_tw, 2 * e->B * sizeof(float2));
+  if (r == cudaSuccess) r = cudaMalloc(&e->d_tw_ir, 2 * e->B * sizeof(float2));
   if (r == cudaSuccess) r = cudaMallocHost(&e->h_chans, e->max_channels * sizeof(EngChan));
   if (r == cudaSuccess) r = cudaMallocHost(&e->h_items, e->max_items * sizeof(EngItem));
   if (r == cudaSuccess) r = cudaMallocHost(&e->h_levels, std::max<size_t>(1, nlev) * sizeof(EngLevel));
@@ -1045,9 +1144,13 @@ int32_t tanb_engine_create(tanb_context* ctx, uint32_t block, uint32_t spectrum,
   std::vector<float2> tw(2 * e->B);
   tanb::make_twiddles(2 * e->B, tw.data());
   r = cudaMemcpy(e->d_tw, tw.data(), tw.size() * sizeof(float2), cudaMemcpyHostToDevice);
+  if (r == cudaSuccess) {
+    tanb::make_plan_twiddles(e->log2B, tw.data());
+    r = cudaMemcpy(e->d_tw_ir, tw.data(), tw.size() * sizeof(float2), cudaMemcpyHostToDevice);
+  }
   for (int c = 0; c < e->nclass && r == cudaSuccess; ++c) {
     std::vector<float2> twl((size_t)4 << (e->log2B + c));
-    tanb::make_twiddles((int)twl.size(), twl.data());
+    tanb::make_plan_twiddles(e->log2B + 1 + c, twl.data());
     r = cudaMemcpy(e->d_tw_lv[c], twl.data(), twl.size() * sizeof(float2), cudaMemcpyHostToDevice);
   }
   if (r == cudaSuccess) r = cudaMemsetAsync(e->d_chans, 0, e->max_channels * sizeof(EngChan), e->stream);
@@ -1400,6 +1503,9 @@ int32_t tanb_engine_process_device(tanb_engine* e, const float* in, float* out, 
   rows.in_base = in;
   rows.out_base = out;
   rows.ld = ld ? (int)ld : e->B;
+  const uintptr_t span = ((uintptr_t)rows.ld * (e->nslots_hwm ? e->nslots_hwm - 1 : 0) + e->B) * sizeof(float);
+  const uintptr_t a = reinterpret_cast<uintptr_t>(in), b = reinterpret_cast<uintptr_t>(out);
+  rows.overlap = in && a < b + span && b < a + span;
   return run_block(e, &rows);
 }
 

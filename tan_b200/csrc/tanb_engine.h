@@ -120,6 +120,9 @@ struct EngRows {
   int ld = 0;
   const float* const* in_tab = nullptr;
   float* const* out_tab = nullptr;
+  // output rows may overlap input rows: the level heads, which read the input
+  // rows, run before the block launch, which writes the output rows
+  int overlap = 0;
 };
 
 cudaError_t eng_prepare();
@@ -164,5 +167,24 @@ cudaError_t eng_launch_level_commit_items(int log2B, int spec, const EngChan* ch
 cudaError_t eng_launch_level_commit_out(int log2B, int log2N, int spec, const EngChan* chans,
                                         const EngLevel* levels, int first, int n, int nfl, const float2* tw,
                                         const long long* block, cudaStream_t st);
+
+// Several blocks k0 .. k0 + nb - 1 of a non-uniform FP32 session, level by level
+// (device rows that hold the blocks back to back): the input history, the base
+// level's output (at most two partitions), what one level size's rings hold for
+// the call, its heads (level blocks j0 .. j0 + m - 1, those due in the call; with
+// what the rings hold, when `with_ring`), its work items for blocks [ka, ka + nk), and the state after
+// the call.
+cudaError_t eng_launch_run_input(int log2B, const EngChan* chans, int nslots, const EngRows& rows, long long k0, int nb,
+                                 cudaStream_t st);
+cudaError_t eng_launch_run_base(int log2B, const EngChan* chans, int nslots, const EngRows& rows, const float2* tw,
+                                long long k0, int nb, cudaStream_t st);
+cudaError_t eng_launch_run_level(int log2B, int log2N, const EngChan* chans, const EngLevel* levels, int nlev,
+                                 const EngRows& rows, const float2* tw, long long k0, int nb, long long j0, int m,
+                                 bool with_ring, cudaStream_t st);
+cudaError_t eng_launch_run_ring(int log2B, const EngChan* chans, const EngLevel* levels, int nlev, const EngRows& rows,
+                                long long k0, int nb, long long j0, cudaStream_t st);
+cudaError_t eng_launch_run_items(int log2B, const EngChan* chans, const EngLevel* levels, const EngItem* items,
+                                 int item0, int nitems, int log2N, long long ka, int nk, int grid, cudaStream_t st);
+cudaError_t eng_launch_run_end(EngChan* chans, int nslots, EngSync sync, int nb, cudaStream_t st);
 
 }  // namespace tanb

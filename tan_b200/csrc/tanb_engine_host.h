@@ -23,5 +23,12 @@ size_t engine_nu_session_bytes(int block, int spectrum, int channels, uint32_t i
                                const uint32_t* level_block, const uint32_t* level_parts);
 // One block with the given rows (direct launches on the audio stream).
 int32_t engine_process_rows(tanb_engine* e, const EngRows& rows);
+// Up to nb blocks of the engine's only session as one launch sequence, rows
+// holding the blocks back to back: *done of them (0: they have to go one by one).
+// Same samples as engine_process_rows bit for bit.
+int32_t engine_run_blocks(tanb_engine* e, int32_t session, const EngRows& rows, size_t nb, int* done);
+// Blocks that engine_run_blocks would run now; 0: the next block goes by itself,
+// -1: all of the nb do.
+int engine_run_fit(tanb_engine* e, int32_t session, size_t nb);
 
 }  // namespace tanb

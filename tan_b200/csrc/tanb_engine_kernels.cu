@@ -53,7 +53,7 @@
 #include <cstdint>
 
 #include "tanb_engine.h"
-#include "tanb_fft.cuh"
+#include "tanb_fft_reg.cuh"
 #include "tanb_internal.h"
 
 namespace tanb {
@@ -172,101 +172,142 @@ __device__ __forceinline__ float4 x_unit(const float2* fdl, int slot, int u) {
 }
 
 // ---------------------------------------------------------------------------
-// R2C of one IR partition into IR slot `slot` of a spectrum table [2][P][M]
-// (with scales [2][P] for FP16 / BF16): samples [t0, t0 + M) of `src`, zero at
-// and after n, zero-padded to 2M. Every thread of the CTA calls it.
+// R2C of IR partitions into IR slot `slot` of a spectrum table [2][P][M] (with
+// scales [2][P] for FP16 / BF16): partition `part` holds samples [t0 + part M,
+// t0 + (part + 1) M) of `src`, zero at and after n, zero-padded to 2M. The groups
+// of a CTA (tanb_fft_reg.cuh) take the partitions part0, part0 + step, ... of one
+// channel in turn. (One partition per CTA of M / 4 threads, radix-4 stages in
+// shared memory: 36 us for 13384 partitions of 256, now 13.)
 template <int LOG2M, int SPEC>
-__device__ __forceinline__ void ir_partition(void* H, float* scale_tab, int P, int slot, int part, const float* src,
-                                             long long t0, long long n, const float2* __restrict__ tw, float2* sm) {
-  using S = FftShape<LOG2M>;
-  constexpr int M = S::M, T = S::T;
-  __shared__ float red[32];
-  for (int q = threadIdx.x; q < M; q += T) {
-    const long long t = t0 + 2 * q;
-    float2 v = make_float2(0.f, 0.f);
-    if (q < M / 2) {
-      if (t < n) v.x = src[t];
-      if (t + 1 < n) v.y = src[t + 1];
-    }
-    sm[q] = v;
+__device__ __forceinline__ void ir_partitions(void* H, float* scale_tab, int P, int slot, int part0, int step,
+                                              const float* src, long long t0, long long n,
+                                              const float2* __restrict__ tw, float2* sm) {
+  using Sh = RegGroups<LOG2M>;
+  using F = RegFft<LOG2M>;
+  constexpr int M = F::M, T = F::T, E = F::E, G = Sh::G, RL = F::RL, NPAIR = E / 2;
+  __shared__ float red[Sh::THREADS / 32 + 1];
+  auto sync = [] { group_sync<T, G>(); };
+  const int grp = (int)threadIdx.x / T, t = (int)threadIdx.x % T;
+  float2* buf0 = sm + (Sh::PP ? 2 : 1) * grp * F::PM;
+  float2* buf1 = Sh::PP ? buf0 + F::PM : buf0;
+  float2 w[Sh::WREG ? F::TWT : 1];
+  if constexpr (Sh::WREG) {
+    reg_twiddles<LOG2M, 1>(w, tw, t);
+    if constexpr (F::NP > 2) reg_twiddles<LOG2M, 2>(w + F::tw_base(2), tw, t);
   }
-  __syncthreads();
-  fft_inplace<LOG2M, false>(sm, tw);
-  // split step in place: thread owning pair (k, M-k) writes both
-  for (int k = threadIdx.x; k <= M / 2; k += T) {
-    if (k == 0) {
-      sm[0] = rfft_post_dc(sm[0]);
-    } else {
-      const int km = M - k;
-      const float2 a = sm[k], b = sm[km];
-      const float2 Xk = rfft_post(a, b, __ldg(tw + k));
-      const float2 Xm = rfft_post(b, a, __ldg(tw + km));
-      sm[k] = Xk;
-      if (km != k) sm[km] = Xm;
+  const bool h8 = ((reinterpret_cast<uintptr_t>(src) + 4 * (uintptr_t)t0) & 7) == 0;  // pairs load as one float2
+  for (int part = part0; part < P; part += step) {
+    float2 v[E];
+#pragma unroll
+    for (int i = 0; i < E; ++i) {
+      v[i] = make_float2(0.f, 0.f);
+      if (i % F::R0 < F::R0 / 2) {
+        const long long at = t0 + (long long)part * M + 2 * reg_in_index<LOG2M>(t, i);
+        if (h8 && at + 1 < n) {
+          v[i] = __ldg(reinterpret_cast<const float2*>(src + at));
+        } else {
+          if (at < n) v[i].x = src[at];
+          if (at + 1 < n) v[i].y = src[at + 1];
+        }
+      }
     }
-  }
-  __syncthreads();
-  float scale = 1.0f;
-  if constexpr (kScaled<SPEC>) {
+    reg_fft<LOG2M, false, Sh::WREG>(v, w, tw, buf0, buf1, t, sync);
+    float2* pb = (F::NP & 1) ? buf0 : buf1;
+#pragma unroll
+    for (int i = 0; i < E; ++i)
+      if (i % RL >= RL / 2) pb[F::pad(reg_out_index<LOG2M>(t, i))] = v[i];
+    sync();
+    // X_k in place of the lower half, X_{M-k} in place of the upper one (bin M/2
+    // beside bin 0)
     float mx = 0.f;
-    for (int k = threadIdx.x; k < M; k += T) mx = fmaxf(mx, fmaxf(fabsf(sm[k].x), fabsf(sm[k].y)));
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-      mx = (threadIdx.x < (T + 31) / 32) ? red[threadIdx.x] : 0.f;
-      for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      if (threadIdx.x == 0) red[0] = mx;
+#pragma unroll
+    for (int p = 0; p < NPAIR; ++p) {
+      const int i = reg_pair<LOG2M>(p), k = reg_out_index<LOG2M>(t, i);
+      const float2 a = v[i], b = pb[F::pad(k == 0 ? M / 2 : M - k)];
+      if (k == 0) {
+        v[i] = x_post_dc(a);
+        v[i + RL / 2] = x_post_mid(b);
+      } else {
+        x_post(a, b, __ldg(tw + k), v[i], v[i + RL / 2]);
+      }
+      if constexpr (kScaled<SPEC>)
+        mx = fmaxf(fmaxf(mx, fmaxf(fabsf(v[i].x), fabsf(v[i].y))), fmaxf(fabsf(v[i + RL / 2].x), fabsf(v[i + RL / 2].y)));
     }
-    __syncthreads();
-    mx = red[0];
-    // power of two with the largest magnitude mapped to [2^14, 2^15)
-    int e = 0;
-    if (mx > 0.f) {
-      frexpf(mx, &e);  // mx = f * 2^e, f in [0.5, 1)
-      e -= 15;
+    float scale = 1.0f;
+    if constexpr (kScaled<SPEC>) {
+      constexpr int W = T < 32 ? T : 32;
+      const unsigned mask = T < 32 ? (((1u << W) - 1u) << ((threadIdx.x & 31u) / W * W)) : 0xffffffffu;
+#pragma unroll
+      for (int o = W / 2; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(mask, mx, o));
+      if constexpr (T > 32) {
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
+        sync();
+        mx = 0.f;
+        for (int q = 0; q < T / 32; ++q) mx = fmaxf(mx, red[grp * (T / 32) + q]);
+      }
+      // power of two with the largest magnitude mapped to [2^14, 2^15)
+      int e = 0;
+      if (mx > 0.f) {
+        frexpf(mx, &e);  // mx = f * 2^e, f in [0.5, 1)
+        e -= 15;
+      }
+      // a partition of denormal samples: keep the scale a normal number (2^-149
+      // would round to zero and its inverse overflow)
+      e = e < -126 ? -126 : e;
+      scale = ldexpf(1.0f, e);
+      if (t == 0) scale_tab[(size_t)slot * P + part] = scale;
     }
-    // a partition of denormal samples: keep the scale a normal number (2^-149
-    // would round to zero and its inverse overflow)
-    e = e < -126 ? -126 : e;
-    scale = ldexpf(1.0f, e);
-    if (threadIdx.x == 0) scale_tab[(size_t)slot * P + part] = scale;
-  }
-  const float inv = 1.0f / scale;  // exact: power of two
-  const size_t row = (size_t)slot * P + part;
-  if constexpr (SPEC == kSpecFP24) {
-    void* r = f24_row<M>(H, row);
-    for (int k = threadIdx.x; k < M; k += T) f24_put<M>(r, k, sm[k]);
-  } else {
-    for (int k = threadIdx.x; k < M; k += T)
-      SpecT<SPEC>::put(H, row * M + k, make_float2(sm[k].x * inv, sm[k].y * inv));
+    const float inv = 1.0f / scale;  // exact: power of two
+    const size_t row = (size_t)slot * P + part;
+#pragma unroll
+    for (int p = 0; p < NPAIR; ++p) {
+      const int i = reg_pair<LOG2M>(p), k = reg_out_index<LOG2M>(t, i), km = k == 0 ? M / 2 : M - k;
+      const float2 Xk = v[i], Xm = v[i + RL / 2];
+      if constexpr (SPEC == kSpecFP24) {
+        void* r = f24_row<M>(H, row);
+        f24_put<M>(r, k, Xk);
+        f24_put<M>(r, km, Xm);
+      } else {
+        SpecT<SPEC>::put(H, row * M + k, make_float2(Xk.x * inv, Xk.y * inv));
+        SpecT<SPEC>::put(H, row * M + km, make_float2(Xm.x * inv, Xm.y * inv));
+      }
+    }
+    if constexpr (!Sh::PP) {
+      sync();
+    } else {
+      if constexpr (kScaled<SPEC> && T > 32) sync();  // red is written again by the next partition
+      if constexpr ((F::NP & 1) != 0) {
+        float2* b = buf0;
+        buf0 = buf1;
+        buf1 = b;
+      }
+    }
   }
 }
 
 template <int LOG2M, int SPEC>
-__global__ void __launch_bounds__(FftShape<LOG2M>::T)
+__global__ void __launch_bounds__(RegGroups<LOG2M>::THREADS)
     eng_ir_kernel(EngChan* __restrict__ chans, const EngUpd* __restrict__ upd, const float2* __restrict__ tw) {
-  extern __shared__ float2 sm[];
-  const int part = blockIdx.x;
+  using Sh = RegGroups<LOG2M>;
+  extern __shared__ __align__(16) float2 sm[];
   const EngUpd u = upd[blockIdx.y];
   const EngChan ch = chans[u.chan];
-  if (part >= ch.P) return;
-  ir_partition<LOG2M, SPEC>(ch.H, ch.scale, ch.P, u.slot, part, u.src, (long long)part * (1 << LOG2M), u.n, tw, sm);
+  ir_partitions<LOG2M, SPEC>(ch.H, ch.scale, ch.P, u.slot, blockIdx.x * Sh::G + threadIdx.x / Sh::F::T,
+                             gridDim.x * Sh::G, u.src, 0, u.n, tw, sm);
 }
 
 // Partitions of non-uniform levels of one size (2^LOG2M): partition `part` of
 // level record u.lvl covers taps [off + part M, off + (part + 1) M).
 template <int LOG2M, int SPEC>
-__global__ void __launch_bounds__(FftShape<LOG2M>::T)
+__global__ void __launch_bounds__(RegGroups<LOG2M>::THREADS)
     eng_level_ir_kernel(EngLevel* __restrict__ levels, const EngLvlUpd* __restrict__ upd,
                         const float2* __restrict__ tw) {
-  extern __shared__ float2 sm[];
-  const int part = blockIdx.x;
+  using Sh = RegGroups<LOG2M>;
+  extern __shared__ __align__(16) float2 sm[];
   const EngLvlUpd u = upd[blockIdx.y];
   const EngLevel lv = levels[u.lvl];
-  if (part >= lv.K) return;
-  ir_partition<LOG2M, SPEC>(lv.H, lv.scale, lv.K, u.slot, part, u.src, lv.off + (long long)part * (1 << LOG2M), u.n,
-                            tw, sm);
+  ir_partitions<LOG2M, SPEC>(lv.H, lv.scale, lv.K, u.slot, blockIdx.x * Sh::G + threadIdx.x / Sh::F::T,
+                             gridDim.x * Sh::G, u.src, lv.off, u.n, tw, sm);
 }
 
 // ---------------------------------------------------------------------------
@@ -823,20 +864,143 @@ __global__ void __launch_bounds__(FftShape<LOG2M>::T, 1024 / FftShape<LOG2M>::T)
   finish_block(chans, nslots, sync, total, k);
 }
 
+// ---------------------------------------------------------------------------
+// Level transforms: register passes (tanb_fft_reg.cuh) with one exchange buffer.
+// A 16384-sample level block took 122 us per CTA as radix-4 stages in shared
+// memory (fourteen barriers a transform and a strided twiddle load per stage).
+
+// Frame of 2M samples from s0 on, as pass 0 takes it: sample t < kB from the input
+// history, later ones from x (this block's row, or null: silence).
+template <int LOG2M>
+__device__ __forceinline__ void lv_frame(float2 (&v)[RegFft<LOG2M>::E], const float* hist, int hmask, const float* x,
+                                         long long kB, long long s0, int t) {
+#pragma unroll
+  for (int i = 0; i < RegFft<LOG2M>::E; ++i) {
+    const long long a = s0 + 2 * reg_in_index<LOG2M>(t, i);  // even, and kB is even: a and a + 1 on one side
+    v[i] = make_float2(0.f, 0.f);
+    if (a >= 0 && a < kB) v[i] = *reinterpret_cast<const float2*>(hist + (a & hmask));
+    else if (a >= kB && x) v[i] = make_float2(x[a - kB], x[a + 1 - kB]);
+  }
+}
+
+// After the forward passes: X_k in the register of pair (k, M - k)'s lower bin,
+// X_{M-k} in the upper one's (register + RL / 2); bin M / 2 beside bin 0.
+template <int LOG2M, class Sync>
+__device__ __forceinline__ void lv_split(float2 (&v)[RegFft<LOG2M>::E], float2* buf, const float2* __restrict__ tw, int t,
+                                         Sync&& sync) {
+  using F = RegFft<LOG2M>;
+  constexpr int M = F::M, E = F::E, RL = F::RL;
+#pragma unroll
+  for (int i = 0; i < E; ++i)
+    if (i % RL >= RL / 2) buf[F::pad(reg_out_index<LOG2M>(t, i))] = v[i];
+  sync();
+#pragma unroll
+  for (int p = 0; p < E / 2; ++p) {
+    const int i = reg_pair<LOG2M>(p), k = reg_out_index<LOG2M>(t, i);
+    const float2 a = v[i], b = buf[F::pad(k == 0 ? M / 2 : M - k)];
+    if (k == 0) {
+      v[i] = x_post_dc(a);
+      v[i + RL / 2] = x_post_mid(b);
+    } else {
+      x_post(a, b, __ldg(tw + k), v[i], v[i + RL / 2]);
+    }
+  }
+  sync();
+}
+
+// Products A of the pairs (laid out as lv_split leaves X) to the inverse
+// transform's output registers.
+template <int LOG2M, bool WREG, class Sync>
+__device__ __forceinline__ void lv_inverse(float2 (&v)[RegFft<LOG2M>::E], const float2* w, float2* buf,
+                                           const float2* __restrict__ tw, int t, Sync&& sync) {
+  using F = RegFft<LOG2M>;
+  constexpr int M = F::M, E = F::E, RL = F::RL;
+  const float inv_n = 1.0f / (float)(2 * M);
+#pragma unroll
+  for (int p = 0; p < E / 2; ++p) {
+    const int i = reg_pair<LOG2M>(p), k = reg_out_index<LOG2M>(t, i), km = k == 0 ? M / 2 : M - k;
+    float2 zk, zm;
+    if (k == 0) {
+      zk = x_pre_dc(v[i], inv_n);
+      zm = x_pre_mid(v[i + RL / 2], inv_n);
+    } else {
+      x_pre(v[i], v[i + RL / 2], __ldg(tw + k), inv_n, zk, zm);
+    }
+    if constexpr (F::SYM) v[i] = zk;
+    else buf[F::pad(k)] = zk;
+    buf[F::pad(km)] = zm;
+  }
+  sync();
+  if constexpr (F::SYM) {
+#pragma unroll
+    for (int i = 0; i < E; ++i)
+      if (i % F::R0 >= F::R0 / 2) v[i] = buf[F::pad(reg_in_index<LOG2M>(t, i))];
+  } else {
+    reg_load<LOG2M, 0>(v, buf, t);
+  }
+  sync();
+  reg_fft<LOG2M, true, WREG>(v, w, tw, buf, buf, t, sync);
+}
+
+// X_j in `v` -> the products of level block j: partial rows (parity j & 1, in row
+// order), X_{j-1} H_1 (X_{j-1} from `xp` in v's layout, or from the delay line)
+// and X_j H_0.
+template <int LOG2M, int SPEC, bool XP>
+__device__ __forceinline__ void lv_products(float2 (&v)[RegFft<LOG2M>::E], const float2* xp, const EngLevel& lv,
+                                            int slot, long long j, int t) {
+  using F = RegFft<LOG2M>;
+  constexpr int M = F::M, E = F::E, RL = F::RL;
+  const int prv = lv_slot(j - 1, lv.Kr);
+  const float2* prow = lv.part + (size_t)((j & 1) * lv.ngroup) * M;
+#pragma unroll
+  for (int p = 0; p < E / 2; ++p) {
+    const int i = reg_pair<LOG2M>(p), k = reg_out_index<LOG2M>(t, i), km = k == 0 ? M / 2 : M - k;
+    float2 tk = make_float2(0.f, 0.f), tm = tk;
+    for (int r = 0; r < lv.ngroup; ++r) {
+      tk = c_add(tk, prow[(size_t)r * M + k]);
+      tm = c_add(tm, prow[(size_t)r * M + km]);
+    }
+    if (lv.K > 1) {
+      const float2 xk = XP ? xp[i] : x_bin<SPEC, M>(lv.fdl, prv, k);
+      const float2 xm = XP ? xp[i + RL / 2] : x_bin<SPEC, M>(lv.fdl, prv, km);
+      const float2 hk = lv_spec_bin<SPEC, M>(lv, slot, 1, k);
+      tk = k == 0 ? c_mac_dc(tk, xk, hk) : c_mac(tk, xk, hk);
+      tm = c_mac(tm, xm, lv_spec_bin<SPEC, M>(lv, slot, 1, km));
+    }
+    const float2 hk = lv_spec_bin<SPEC, M>(lv, slot, 0, k);
+    v[i] = k == 0 ? c_mac_dc(tk, v[i], hk) : c_mac(tk, v[i], hk);
+    v[i + RL / 2] = c_mac(tm, v[i + RL / 2], lv_spec_bin<SPEC, M>(lv, slot, 0, km));
+  }
+}
+
+template <int LOG2M, int SPEC>
+__device__ __forceinline__ void lv_insert(const float2 (&v)[RegFft<LOG2M>::E], const EngLevel& lv, int cur, int t) {
+  constexpr int M = RegFft<LOG2M>::M, RL = RegFft<LOG2M>::RL;
+#pragma unroll
+  for (int p = 0; p < RegFft<LOG2M>::E / 2; ++p) {
+    const int i = reg_pair<LOG2M>(p), k = reg_out_index<LOG2M>(t, i);
+    x_put<SPEC, M>(lv.fdl, cur, k, v[i]);
+    x_put<SPEC, M>(lv.fdl, cur, k == 0 ? M / 2 : M - k, v[i + RL / 2]);
+  }
+}
+
 // Head of level block j = (k + 1) / p - 1 of every level record of one size
 // class (2^LOG2M) at a block k where that size is due: frame = input samples
 // [(j-1) N, (j+1) N) (the last B of them, this block's, from the input row),
-// X_j into the level's delay line, Y = sum of the partial rows (parity j & 1,
-// in row order) + X_{j-1} H_1 + X_j H_0, C2R, samples [N, 2N) of the result
-// into the output ring of the IR in effect after this block at positions
-// off + jN + i. It reads no data the block kernel of this block writes.
+// X_j into the level's delay line, Y = sum of the partial rows + X_{j-1} H_1 +
+// X_j H_0, C2R, samples [N, 2N) of the result into the output ring of the IR in
+// effect after this block at positions off + jN + i. It reads no data the block
+// kernel of this block writes.
 template <int LOG2M, int SPEC>
-__global__ void __launch_bounds__(FftShape<LOG2M>::T)
+__global__ void __launch_bounds__(RegFft<LOG2M>::T)
     eng_level_head_kernel(EngChan* __restrict__ chans, int nslots, const EngLevel* __restrict__ levels, int log2B,
                           EngRows rows, const float2* __restrict__ tw, EngSync sync, unsigned total) {
-  using S = FftShape<LOG2M>;
-  constexpr int M = S::M, T = S::T;
-  extern __shared__ float2 sm[];
+  using F = RegFft<LOG2M>;
+  constexpr int M = F::M, T = F::T, E = F::E, RL = F::RL;
+  constexpr bool WREG = E == 8;
+  extern __shared__ __align__(16) float2 sm[];
+  auto bar = [] { group_sync<T, 1>(); };
+  const int t = threadIdx.x;
   const long long k = *sync.block;
   const EngLevel lv = levels[blockIdx.x];
   const int pshift = LOG2M - log2B;
@@ -849,74 +1013,285 @@ __global__ void __launch_bounds__(FftShape<LOG2M>::T)
   if (work) {
     const long long j = ((k + 1) >> pshift) - 1;
     const int slot = ch.pending ? 1 - ch.active : ch.active;
-    const EngNu* nu = ch.nu;
-    const float* hist = nu->in_ring;
-    const int hmask = nu->rin - 1;
-    const float* x = row_in(rows, lv.chan);
-    const long long s0 = (j - 1) * M, kB = k << log2B;
-    float2* z = sm;
-    for (int n = threadIdx.x; n < M; n += T) {
-      const long long a = s0 + 2 * n;  // even, and kB is even: a and a + 1 on one side
-      float2 v = make_float2(0.f, 0.f);
-      if (a >= 0 && a < kB) {
-        v = make_float2(hist[a & hmask], hist[(a + 1) & hmask]);
-      } else if (a >= kB && x) {
-        v = make_float2(x[a - kB], x[a + 1 - kB]);
-      }
-      z[n] = v;
+    float2 w[WREG ? F::TWT : 1];
+    if constexpr (WREG) {
+      reg_twiddles<LOG2M, 1>(w, tw, t);
+      if constexpr (F::NP > 2) reg_twiddles<LOG2M, 2>(w + F::tw_base(2), tw, t);
     }
-    __syncthreads();
-    fft_inplace<LOG2M, false>(z, tw);
-    const int K = lv.K, Kr = lv.Kr;
-    const int cur = lv_slot(j, Kr), prv = lv_slot(j - 1, Kr);
-    const float2* prow = lv.part + (size_t)((j & 1) * lv.ngroup) * M;
-    const float inv_n = 1.0f / (float)(2 * M);
-    for (int kk = threadIdx.x; kk <= M / 2; kk += T) {
-      const int km = (kk == 0) ? 0 : M - kk;
-      float2 tk = make_float2(0.f, 0.f), tm = tk;
-      for (int r = 0; r < lv.ngroup; ++r) {
-        const float2 a = prow[(size_t)r * M + kk], b = prow[(size_t)r * M + km];
-        tk.x += a.x; tk.y += a.y;
-        tm.x += b.x; tm.y += b.y;
-      }
-      if (K > 1) {
-        const float2 xk = x_bin<SPEC, M>(lv.fdl, prv, kk), xm = x_bin<SPEC, M>(lv.fdl, prv, km);
-        if (kk == 0) {
-          tk = c_mac_dc(tk, xk, lv_spec_bin<SPEC, M>(lv, slot, 1, 0));
-        } else {
-          tk = c_mac(tk, xk, lv_spec_bin<SPEC, M>(lv, slot, 1, kk));
-          tm = c_mac(tm, xm, lv_spec_bin<SPEC, M>(lv, slot, 1, km));
-        }
-      }
-      if (kk == 0) {
-        const float2 X = rfft_post_dc(z[0]);
-        x_put<SPEC, M>(lv.fdl, cur, 0, X);
-        z[0] = irfft_pre_dc(c_mac_dc(tk, X, lv_spec_bin<SPEC, M>(lv, slot, 0, 0)), inv_n);
-      } else {
-        const float2 wk = __ldg(tw + kk), wm = __ldg(tw + km);
-        const float2 a = z[kk], b = z[km];
-        const float2 Xk = rfft_post(a, b, wk);
-        const float2 Xm = rfft_post(b, a, wm);
-        x_put<SPEC, M>(lv.fdl, cur, kk, Xk);
-        if (km != kk) x_put<SPEC, M>(lv.fdl, cur, km, Xm);
-        const float2 Ak = c_mac(tk, Xk, lv_spec_bin<SPEC, M>(lv, slot, 0, kk));
-        const float2 Am = c_mac(tm, Xm, lv_spec_bin<SPEC, M>(lv, slot, 0, km));
-        z[kk] = irfft_pre(Ak, Am, wk, inv_n);
-        if (km != kk) z[km] = irfft_pre(Am, Ak, wm, inv_n);
-      }
-    }
-    __syncthreads();
-    fft_inplace<LOG2M, true>(z, tw);
+    float2 v[E];
+    lv_frame<LOG2M>(v, ch.nu->in_ring, ch.nu->rin - 1, row_in(rows, lv.chan), k << log2B, (j - 1) * M, t);
+    reg_fft<LOG2M, false, WREG>(v, w, tw, sm, sm, t, bar);
+    lv_split<LOG2M>(v, sm, tw, t, bar);
+    lv_insert<LOG2M, SPEC>(v, lv, lv_slot(j, lv.Kr), t);
+    lv_products<LOG2M, SPEC, false>(v, nullptr, lv, slot, j, t);
+    lv_inverse<LOG2M, WREG>(v, w, sm, tw, t, bar);
     float* ring = lv.ring + (size_t)slot * lv.R;
     const int rmask = lv.R - 1;
     const long long base = lv.off + j * M;
-    for (int m = M / 2 + threadIdx.x; m < M; m += T) {
-      const int i = 2 * (m - M / 2);
-      ring[(base + i) & rmask] = z[m].x;
-      ring[(base + i + 1) & rmask] = z[m].y;
+#pragma unroll
+    for (int p = 0; p < E / 2; ++p) {
+      const int i = reg_pair<LOG2M>(p) + RL / 2;
+      *reinterpret_cast<float2*>(ring + ((base + 2 * (reg_out_index<LOG2M>(t, i) - M / 2)) & rmask)) = v[i];
     }
   }
   finish_block(chans, nslots, sync, total, k);
+}
+
+// ---------------------------------------------------------------------------
+// Several blocks of a non-uniform session in one call (device rows, no IR change
+// inside): the session's blocks k0 .. k0 + nb - 1, level by level instead of
+// block by block. Each base block's heads and each level's heads then run over
+// all the blocks they have in the call side by side, and a level's work items
+// over all their bin slices, in about ten launches; block by block the same
+// work is one launch per block and, beside it, up to seven launches of level
+// heads that wait for memory and for one another (40 us a block at 256 channels
+// of 2^20 taps). The transforms, products and sums are those of the block
+// kernels in the same order, so that the samples are the same bit for bit:
+//   eng_run_input_kernel  the call's samples into the input history
+//   eng_run_base_kernel   the base level's output into the output rows
+//   eng_run_ring_kernel, eng_run_level_kernel  per level, in order: what its ring
+//                         holds for the call's blocks, and its heads, whose
+//                         samples go into the output rows as far as the call
+//                         reaches, then into the ring
+//   eng_run_items_kernel  partial rows of levels with work items
+//   eng_run_end_kernel    channel state and block counter
+__global__ void eng_run_input_kernel(const EngChan* __restrict__ chans, EngRows rows, int log2B, long long k0, int nb) {
+  const EngChan ch = chans[blockIdx.y];
+  if (!ch.run) return;
+  const float* x = row_in(rows, blockIdx.y);
+  float* ring = ch.nu->in_ring;
+  const int mask = ch.nu->rin - 1, n = nb << log2B, last = (nb - 1) << log2B;
+  const long long t0 = k0 << log2B;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const float v = x ? x[i] : 0.f;
+    ring[(t0 + i) & mask] = v;
+    if (i >= last) ch.prev[i - last] = v;
+  }
+}
+
+// Blocks [k0 + r0, k0 + r0 + run) of one channel per CTA, base level of at most
+// two partitions. X of the block before the run is transformed again rather than
+// read from the delay line, whose slots the other runs overwrite.
+template <int LOG2M>
+__global__ void __launch_bounds__(FftShape<LOG2M>::T)
+    eng_run_base_kernel(const EngChan* __restrict__ chans, EngRows rows, const float2* __restrict__ tw, long long k0,
+                        int nb, int run) {
+  constexpr int M = 1 << LOG2M, T = FftShape<LOG2M>::T;
+  extern __shared__ __align__(16) float2 sm[];
+  float2* z = sm;
+  float2* xp = sm + M;  // X of the block before
+  const int c = blockIdx.y;
+  const EngChan ch = chans[c];
+  if (!ch.run) return;
+  float* y = row_out(rows, c);
+  const float* hist = ch.nu->in_ring;
+  const int hmask = ch.nu->rin - 1, P = ch.P;
+  const int r0 = blockIdx.x * run, r1 = min(nb, r0 + run);
+  const float2* H0 = reinterpret_cast<const float2*>(ch.H) + (size_t)ch.active * P * M;
+  const float inv_n = 1.0f / (float)(2 * M);
+  const bool y_vec = (reinterpret_cast<uintptr_t>(y) & 7) == 0;
+  for (int r = P > 1 ? r0 - 1 : r0; r < r1; ++r) {
+    const long long s0 = (k0 + r - 1) * M;
+    for (int q = threadIdx.x; q < M; q += T) {
+      const long long a = s0 + 2 * q;
+      z[q] = a >= 0 ? *reinterpret_cast<const float2*>(hist + (a & hmask)) : make_float2(0.f, 0.f);
+    }
+    __syncthreads();
+    fft_inplace<LOG2M, false>(z, tw);
+    int slot = (ch.cur - 1 - r) % P;
+    if (slot < 0) slot += P;
+    float2* F = ch.fdl + (size_t)slot * M;
+    const bool keep = r >= r0 && r >= nb - P;  // the delay line after the call
+    for (int k = threadIdx.x; k <= M / 2; k += T) {
+      const int km = k == 0 ? 0 : M - k;
+      const float2 wk = tw[k], wm = tw[km];
+      const float2 a = z[k], b = z[km];
+      const float2 Xk = k == 0 ? rfft_post_dc(a) : rfft_post(a, b, wk);
+      const float2 Xm = k == 0 ? Xk : rfft_post(b, a, wm);
+      if (keep) {
+        F[k] = Xk;
+        if (km != k) F[km] = Xm;
+      }
+      if (r >= r0) {
+        float2 tk = make_float2(0.f, 0.f), tm = tk;
+        if (P > 1) {
+          tk = k == 0 ? c_mac_dc(tk, xp[0], H0[M]) : c_mac(tk, xp[k], H0[M + k]);
+          if (k != 0) tm = c_mac(tm, xp[km], H0[M + km]);
+        }
+        if (k == 0) {
+          z[0] = irfft_pre_dc(c_mac_dc(tk, Xk, H0[0]), inv_n);
+        } else {
+          const float2 Ak = c_mac(tk, Xk, H0[k]), Am = c_mac(tm, Xm, H0[km]);
+          z[k] = irfft_pre(Ak, Am, wk, inv_n);
+          if (km != k) z[km] = irfft_pre(Am, Ak, wm, inv_n);
+        }
+      }
+      xp[k] = Xk;
+      xp[km] = Xm;
+    }
+    __syncthreads();
+    if (r < r0) continue;
+    fft_inplace<LOG2M, true>(z, tw);
+    if (y) {
+      float* yr = y + (size_t)r * M;
+      for (int m = M / 2 + threadIdx.x; m < M; m += T) {
+        const int i = 2 * (m - M / 2);
+        if (y_vec) {
+          reinterpret_cast<float2*>(yr)[i / 2] = z[m];
+        } else {
+          yr[i] = z[m].x;
+          yr[i + 1] = z[m].y;
+        }
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// What the rings of one size class hold for the call's samples (of heads before
+// the call, up to off + j0 N), added to the output rows: a launch of its own
+// before the level's heads where the samples that those put into the ring can
+// take the places of these.
+__global__ void eng_run_ring_kernel(const EngChan* __restrict__ chans, const EngLevel* __restrict__ levels, int log2B,
+                                    EngRows rows, long long k0, int nb, long long j0) {
+  const EngLevel lv = levels[blockIdx.y];
+  if (lv.chan < 0) return;
+  const EngChan ch = chans[lv.chan];
+  float* y = row_out(rows, lv.chan);
+  if (!ch.run || !y) return;
+  const float* ring = lv.ring + (size_t)ch.active * lv.R;
+  const long long tb = k0 << log2B, te = (k0 + nb) << log2B, e = min(te, lv.off + (j0 << lv.log2N));
+  for (long long a = tb + blockIdx.x * (long long)blockDim.x + threadIdx.x; a < e; a += (long long)gridDim.x * blockDim.x)
+    y[a - tb] = __fadd_rn(y[a - tb], ring[a & (lv.R - 1)]);
+}
+
+// Level blocks j0 .. j0 + m - 1 of every record of one size class (those whose
+// heads fall into the call); run of them per group in turn. X_{j-1} comes from the
+// delay line when m == 1, else from a transform of its own (the other groups
+// overwrite the delay line).
+template <int LOG2M, int SPEC>
+__global__ void __launch_bounds__(RegGroups<LOG2M>::THREADS)
+    eng_run_level_kernel(const EngChan* __restrict__ chans, const EngLevel* __restrict__ levels, int log2B, EngRows rows,
+                         const float2* __restrict__ tw, long long k0, int nb, long long j0, int m, int run,
+                         int with_ring) {
+  using F = RegFft<LOG2M>;
+  using Sh = RegGroups<LOG2M>;
+  constexpr int M = F::M, T = F::T, E = F::E, G = Sh::G, RL = F::RL;
+  constexpr bool WREG = E == 8, XP = E <= 16;
+  extern __shared__ __align__(16) float2 sm[];
+  auto bar = [] { group_sync<T, G>(); };
+  const int grp = (int)threadIdx.x / T, t = (int)threadIdx.x % T;
+  float2* buf = sm + grp * F::PM;
+  const EngLevel lv = levels[blockIdx.y];
+  if (lv.chan < 0) return;
+  const EngChan ch = chans[lv.chan];
+  if (!ch.run) return;
+  float* y = row_out(rows, lv.chan);
+  const bool y_vec = (reinterpret_cast<uintptr_t>(y) & 7) == 0;
+  float* ring = lv.ring + (size_t)ch.active * lv.R;
+  const int rmask = lv.R - 1;
+  const long long tb = k0 << log2B, te = (k0 + nb) << log2B;
+  auto add = [&](long long at, float2 o) {  // samples at, at + 1 of the stream, both inside the call or both after it
+    if (at < te) {
+      if (!y) return;
+      float* q = y + (at - tb);
+      if (y_vec) {
+        float2* q2 = reinterpret_cast<float2*>(q);
+        *q2 = c_add(*q2, o);
+      } else {
+        q[0] = __fadd_rn(q[0], o.x);
+        q[1] = __fadd_rn(q[1], o.y);
+      }
+    } else {
+      *reinterpret_cast<float2*>(ring + (at & rmask)) = o;
+    }
+  };
+  if (with_ring) {
+    // samples of earlier heads that fall into the call
+    const long long e = min(te, max(tb, lv.off + j0 * M));
+    for (long long a = tb + 2 * (blockIdx.x * (long long)blockDim.x + threadIdx.x); a < e;
+         a += 2LL * gridDim.x * blockDim.x)
+      add(a, *reinterpret_cast<const float2*>(ring + (a & rmask)));
+  }
+  const int r0 = ((int)blockIdx.x * G + grp) * run, r1 = min(m, r0 + run);
+  if (r0 >= m) return;
+  float2 w[WREG ? F::TWT : 1];
+  if constexpr (WREG) {
+    reg_twiddles<LOG2M, 1>(w, tw, t);
+    if constexpr (F::NP > 2) reg_twiddles<LOG2M, 2>(w + F::tw_base(2), tw, t);
+  }
+  float2 v[E], xp[XP ? E : 1];
+  auto spectrum = [&](long long j) {
+    lv_frame<LOG2M>(v, ch.nu->in_ring, ch.nu->rin - 1, nullptr, te, (j - 1) * M, t);
+    reg_fft<LOG2M, false, WREG>(v, w, tw, buf, buf, t, bar);
+    lv_split<LOG2M>(v, buf, tw, t, bar);
+  };
+  if constexpr (XP) {
+    if (m > 1 && lv.K > 1) {
+      spectrum(j0 + r0 - 1);
+#pragma unroll
+      for (int i = 0; i < E; ++i) xp[i] = v[i];
+    }
+  }
+  for (int r = r0; r < r1; ++r) {
+    const long long j = j0 + r;
+    spectrum(j);
+    if (r >= m - lv.Kr) lv_insert<LOG2M, SPEC>(v, lv, lv_slot(j, lv.Kr), t);
+    float2 xn[XP && E == 8 ? E : 1];
+    if constexpr (XP && E == 8) {
+#pragma unroll
+      for (int i = 0; i < E; ++i) xn[i] = v[i];
+    }
+    if constexpr (XP) {
+      if (m > 1) lv_products<LOG2M, SPEC, true>(v, xp, lv, ch.active, j, t);
+      else lv_products<LOG2M, SPEC, false>(v, nullptr, lv, ch.active, j, t);
+    } else {
+      lv_products<LOG2M, SPEC, false>(v, nullptr, lv, ch.active, j, t);
+    }
+    lv_inverse<LOG2M, WREG>(v, w, buf, tw, t, bar);
+    const long long base = lv.off + j * M;
+#pragma unroll
+    for (int p = 0; p < E / 2; ++p) {
+      const int i = reg_pair<LOG2M>(p) + RL / 2;
+      add(base + 2 * (reg_out_index<LOG2M>(t, i) - M / 2), v[i]);
+    }
+    bar();
+    if constexpr (XP && E == 8) {
+#pragma unroll
+      for (int i = 0; i < E; ++i) xp[i] = xn[i];
+    }
+  }
+}
+
+// Work items of the level records of size 2^log2N for blocks [ka, ka + nk): one
+// (item, block) pair per step, the blocks of an item side by side (they are
+// consecutive bin slices of its rows).
+template <int LOG2B, int SPEC>
+__global__ void __launch_bounds__((1 << LOG2B) / 4)
+    eng_run_items_kernel(const EngChan* __restrict__ chans, const EngLevel* __restrict__ levels,
+                         const EngItem* __restrict__ items, int item0, int nitems, int log2N, long long ka, int nk) {
+  const long long total = (long long)nitems * nk;
+  for (long long v = blockIdx.x; v < total; v += gridDim.x) {
+    const EngItem w = items[item0 + (int)(v / nk)];
+    if (w.chan < 0 || w.lvl < 0) continue;
+    const EngLevel lv = levels[w.lvl];
+    if (lv.log2N != log2N) continue;
+    const EngChan ch = chans[w.chan];
+    if (!ch.run) continue;
+    const long long k = ka + v % nk;
+    const int pshift = log2N - LOG2B;
+    eng_level_item<LOG2B, SPEC>(lv, w, ch.active, (k >> pshift) + 1, (int)(k & ((1LL << pshift) - 1)));
+  }
+}
+
+__global__ void eng_run_end_kernel(EngChan* __restrict__ chans, int nslots, EngSync sync, int nb) {
+  for (int c = threadIdx.x; c < nslots; c += blockDim.x) {
+    EngChan* ch = chans + c;
+    if (!ch->run) continue;
+    const int cur = (ch->cur - nb) % ch->P;
+    ch->cur = cur < 0 ? cur + ch->P : cur;
+  }
+  if (threadIdx.x == 0) *sync.block += nb;
 }
 
 template <int LOG2M, int SPEC>
@@ -964,12 +1339,15 @@ __global__ void __launch_bounds__((1 << LOG2B) / 4)
 // j = j_c - 1 - blockIdx.y over every partition, C2R, written into the new IR's
 // ring at positions >= k B. Blocks before the stream start write zeros.
 template <int LOG2M, int SPEC>
-__global__ void __launch_bounds__(FftShape<LOG2M>::T)
+__global__ void __launch_bounds__(RegFft<LOG2M>::T)
     eng_level_commit_out_kernel(const EngChan* __restrict__ chans, const EngLevel* __restrict__ levels, int log2B,
                                 const float2* __restrict__ tw, const long long* __restrict__ block) {
-  using S = FftShape<LOG2M>;
-  constexpr int M = S::M, T = S::T;
-  extern __shared__ float2 sm[];
+  using F = RegFft<LOG2M>;
+  constexpr int M = F::M, T = F::T, E = F::E, RL = F::RL;
+  constexpr bool WREG = E == 8;
+  extern __shared__ __align__(16) float2 sm[];
+  auto bar = [] { group_sync<T, 1>(); };
+  const int t = threadIdx.x;
   const EngLevel lv = levels[blockIdx.x];
   if (lv.chan < 0) return;
   const EngChan ch = chans[lv.chan];
@@ -985,40 +1363,36 @@ __global__ void __launch_bounds__(FftShape<LOG2M>::T)
   const int rmask = lv.R - 1;
   const long long base = lv.off + j * M;
   if (j < 0) {
-    for (int i = threadIdx.x; i < M; i += T)
+    for (int i = t; i < M; i += T)
       if (base + i >= tmin) ring[(base + i) & rmask] = 0.f;
     return;
   }
-  float2* z = sm;
-  const int K = lv.K, Kr = lv.Kr;
-  const float inv_n = 1.0f / (float)(2 * M);
-  for (int kk = threadIdx.x; kk <= M / 2; kk += T) {
-    const int km = (kk == 0) ? 0 : M - kk;
-    float2 tk = make_float2(0.f, 0.f), tm = tk;
-    for (int i = 0; i < K; ++i) {
-      const int fs = lv_slot(j - i, Kr);
-      const float2 xk = x_bin<SPEC, M>(lv.fdl, fs, kk);
-      if (kk == 0) {
-        tk = c_mac_dc(tk, xk, lv_spec_bin<SPEC, M>(lv, slot, i, 0));
-      } else {
-        tk = c_mac(tk, xk, lv_spec_bin<SPEC, M>(lv, slot, i, kk));
-        tm = c_mac(tm, x_bin<SPEC, M>(lv.fdl, fs, km), lv_spec_bin<SPEC, M>(lv, slot, i, km));
-      }
-    }
-    if (kk == 0) {
-      z[0] = irfft_pre_dc(tk, inv_n);
-    } else {
-      const float2 wk = __ldg(tw + kk), wm = __ldg(tw + km);
-      z[kk] = irfft_pre(tk, tm, wk, inv_n);
-      if (km != kk) z[km] = irfft_pre(tm, tk, wm, inv_n);
-    }
+  float2 w[WREG ? F::TWT : 1];
+  if constexpr (WREG) {
+    reg_twiddles<LOG2M, 1>(w, tw, t);
+    if constexpr (F::NP > 2) reg_twiddles<LOG2M, 2>(w + F::tw_base(2), tw, t);
   }
-  __syncthreads();
-  fft_inplace<LOG2M, true>(z, tw);
-  for (int m = M / 2 + threadIdx.x; m < M; m += T) {
-    const int i = 2 * (m - M / 2);
-    if (base + i >= tmin) ring[(base + i) & rmask] = z[m].x;
-    if (base + i + 1 >= tmin) ring[(base + i + 1) & rmask] = z[m].y;
+  float2 v[E];
+#pragma unroll
+  for (int p = 0; p < E / 2; ++p) {
+    const int i = reg_pair<LOG2M>(p), kk = reg_out_index<LOG2M>(t, i), km = kk == 0 ? M / 2 : M - kk;
+    float2 tk = make_float2(0.f, 0.f), tm = tk;
+    for (int q = 0; q < lv.K; ++q) {
+      const int fs = lv_slot(j - q, lv.Kr);
+      const float2 xk = x_bin<SPEC, M>(lv.fdl, fs, kk), hk = lv_spec_bin<SPEC, M>(lv, slot, q, kk);
+      tk = kk == 0 ? c_mac_dc(tk, xk, hk) : c_mac(tk, xk, hk);
+      tm = c_mac(tm, x_bin<SPEC, M>(lv.fdl, fs, km), lv_spec_bin<SPEC, M>(lv, slot, q, km));
+    }
+    v[i] = tk;
+    v[i + RL / 2] = tm;
+  }
+  lv_inverse<LOG2M, WREG>(v, w, sm, tw, t, bar);
+#pragma unroll
+  for (int p = 0; p < E / 2; ++p) {
+    const int i = reg_pair<LOG2M>(p) + RL / 2;
+    const long long at = base + 2 * (reg_out_index<LOG2M>(t, i) - M / 2);
+    if (at >= tmin) ring[at & rmask] = v[i].x;
+    if (at + 1 >= tmin) ring[(at + 1) & rmask] = v[i].y;
   }
 }
 
@@ -1042,7 +1416,7 @@ cudaError_t attrs_t() {
                                        eng_block_smem<LOG2M>(true));
   if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute(eng_ir_kernel<LOG2M, SPEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (1 << LOG2M) * (int)sizeof(float2));
+                              RegGroups<LOG2M>::SMEM);
 }
 
 template <int LOG2M>
@@ -1054,17 +1428,23 @@ cudaError_t attrs_all() {
   return attrs_t<LOG2M, kSpecFP24>();
 }
 
-// Level kernels of one size: one buffer of M complex values.
+// Level kernels of one size: one exchange buffer per transform.
+template <int LOG2M>
+constexpr int level_smem() {
+  return RegFft<LOG2M>::PM * (int)sizeof(float2);
+}
+
 template <int LOG2M, int SPEC>
 cudaError_t lattrs_t() {
-  const int smem = (1 << LOG2M) * (int)sizeof(float2);
+  const int smem = level_smem<LOG2M>();
   cudaError_t e =
       cudaFuncSetAttribute(eng_level_head_kernel<LOG2M, SPEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(eng_level_commit_out_kernel<LOG2M, SPEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            smem);
   if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(eng_level_ir_kernel<LOG2M, SPEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  return cudaFuncSetAttribute(eng_level_ir_kernel<LOG2M, SPEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              RegGroups<LOG2M>::SMEM);
 }
 
 template <int LOG2M>
@@ -1076,20 +1456,27 @@ cudaError_t lattrs_all() {
   return lattrs_t<LOG2M, kSpecFP24>();
 }
 
+// Partitions one group of threads takes in turn: enough to pay for loading the
+// twiddles, few enough that every SM has several CTAs.
+int ir_grid(int parts, int nupd, int groups) {
+  const long long ctas = ((long long)parts * nupd + groups - 1) / groups;  // at one partition per group
+  const int turns = (int)(ctas / (148 * 2) < 1 ? 1 : ctas / (148 * 2) > 4 ? 4 : ctas / (148 * 2));
+  return (parts + groups * turns - 1) / (groups * turns);
+}
+
 template <int LOG2M, int SPEC>
 cudaError_t ir_t(EngChan* chans, const EngUpd* upd, int nupd, int maxP, const float2* tw, cudaStream_t st) {
-  using S = FftShape<LOG2M>;
-  dim3 grid(maxP, nupd);
-  eng_ir_kernel<LOG2M, SPEC><<<grid, S::T, S::M * sizeof(float2), st>>>(chans, upd, tw);
+  using Sh = RegGroups<LOG2M>;
+  eng_ir_kernel<LOG2M, SPEC><<<dim3(ir_grid(maxP, nupd, Sh::G), nupd), Sh::THREADS, Sh::SMEM, st>>>(chans, upd, tw);
   return cudaGetLastError();
 }
 
 template <int LOG2M, int SPEC>
 cudaError_t level_ir_t(EngLevel* levels, const EngLvlUpd* upd, int nupd, int maxK, const float2* tw,
                        cudaStream_t st) {
-  using S = FftShape<LOG2M>;
-  dim3 grid(maxK, nupd);
-  eng_level_ir_kernel<LOG2M, SPEC><<<grid, S::T, S::M * sizeof(float2), st>>>(levels, upd, tw);
+  using Sh = RegGroups<LOG2M>;
+  eng_level_ir_kernel<LOG2M, SPEC><<<dim3(ir_grid(maxK, nupd, Sh::G), nupd), Sh::THREADS, Sh::SMEM, st>>>(levels, upd,
+                                                                                                        tw);
   return cudaGetLastError();
 }
 
@@ -1106,9 +1493,48 @@ cudaError_t block_t(EngChan* chans, int nslots, const EngItem* items, int nitems
 template <int LOG2M, int SPEC>
 cudaError_t level_head_t(int log2B, EngChan* chans, int nslots, const EngLevel* levels, int nlev,
                          const EngRows& rows, const float2* tw, EngSync sync, unsigned total, cudaStream_t st) {
-  using S = FftShape<LOG2M>;
-  eng_level_head_kernel<LOG2M, SPEC><<<nlev, S::T, S::M * sizeof(float2), st>>>(chans, nslots, levels, log2B, rows,
-                                                                                 tw, sync, total);
+  eng_level_head_kernel<LOG2M, SPEC><<<nlev, RegFft<LOG2M>::T, level_smem<LOG2M>(), st>>>(chans, nslots, levels, log2B,
+                                                                                        rows, tw, sync, total);
+  return cudaGetLastError();
+}
+
+template <int LOG2M>
+cudaError_t run_base_t(const EngChan* chans, int nslots, const EngRows& rows, const float2* tw, long long k0, int nb,
+                       cudaStream_t st) {
+  // runs of blocks per CTA: two thousand CTAs or more, at most 16 blocks (one
+  // transform more than its blocks per run)
+  const long long all = (long long)nslots * nb;
+  const int run = (int)(all / 2048 < 1 ? 1 : all / 2048 > 16 ? 16 : all / 2048);
+  eng_run_base_kernel<LOG2M><<<dim3((nb + run - 1) / run, nslots), FftShape<LOG2M>::T, 2 * (1 << LOG2M) * sizeof(float2),
+                               st>>>(chans, rows, tw, k0, nb, run);
+  return cudaGetLastError();
+}
+
+template <int LOG2M, int SPEC>
+cudaError_t run_level_t(int log2B, const EngChan* chans, const EngLevel* levels, int nlev, const EngRows& rows,
+                        const float2* tw, long long k0, int nb, long long j0, int m, bool with_ring, cudaStream_t st) {
+  using Sh = RegGroups<LOG2M>;
+  constexpr int smem = Sh::G * level_smem<LOG2M>();
+  static OncePerDevice once;
+  const cudaError_t attr = once.run([] {
+    return cudaFuncSetAttribute(eng_run_level_kernel<LOG2M, SPEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  });
+  if (attr != cudaSuccess) return attr;
+  // runs of level blocks per group (sizes whose X_{j-1} stays in registers):
+  // about two thousand groups or more
+  const long long all = (long long)nlev * m;
+  const int run = Sh::F::E > 8 ? 1 : (int)(all / 2048 < 1 ? 1 : all / 2048 > 8 ? 8 : all / 2048);
+  const int gx = m > 0 ? (m + Sh::G * run - 1) / (Sh::G * run) : 1;
+  eng_run_level_kernel<LOG2M, SPEC><<<dim3(gx, nlev), Sh::THREADS, smem, st>>>(chans, levels, log2B, rows, tw, k0, nb,
+                                                                             j0, m, run, with_ring ? 1 : 0);
+  return cudaGetLastError();
+}
+
+template <int LOG2M, int SPEC>
+cudaError_t run_items_t(const EngChan* chans, const EngLevel* levels, const EngItem* items, int item0, int nitems,
+                        int log2N, long long ka, int nk, int grid, cudaStream_t st) {
+  eng_run_items_kernel<LOG2M, SPEC><<<grid, (1 << LOG2M) / 4, 0, st>>>(chans, levels, items, item0, nitems, log2N, ka,
+                                                                      nk);
   return cudaGetLastError();
 }
 
@@ -1131,9 +1557,8 @@ cudaError_t level_commit_items_t(const EngChan* chans, const EngLevel* levels, c
 template <int LOG2M, int SPEC>
 cudaError_t level_commit_out_t(int log2B, const EngChan* chans, const EngLevel* levels, int n, int nfl,
                                const float2* tw, const long long* block, cudaStream_t st) {
-  using S = FftShape<LOG2M>;
-  eng_level_commit_out_kernel<LOG2M, SPEC><<<dim3(n, nfl), S::T, S::M * sizeof(float2), st>>>(chans, levels, log2B,
-                                                                                             tw, block);
+  eng_level_commit_out_kernel<LOG2M, SPEC><<<dim3(n, nfl), RegFft<LOG2M>::T, level_smem<LOG2M>(), st>>>(chans, levels,
+                                                                                                    log2B, tw, block);
   return cudaGetLastError();
 }
 
@@ -1271,6 +1696,64 @@ cudaError_t eng_launch_level_commit_out(int log2B, int log2N, int spec, const En
                                         const long long* block, cudaStream_t st) {
   if (n <= 0 || nfl <= 0) return cudaSuccess;
   ENG_LEVEL_DISPATCH(log2N, spec, level_commit_out_t, log2B, chans, levels + first, n, nfl, tw, block, st);
+}
+
+cudaError_t eng_launch_run_input(int log2B, const EngChan* chans, int nslots, const EngRows& rows, long long k0, int nb,
+                                 cudaStream_t st) {
+  const int n = nb << log2B;
+  eng_run_input_kernel<<<dim3((n + 1023) / 1024, nslots), 256, 0, st>>>(chans, rows, log2B, k0, nb);
+  return cudaGetLastError();
+}
+
+cudaError_t eng_launch_run_base(int log2B, const EngChan* chans, int nslots, const EngRows& rows, const float2* tw,
+                                long long k0, int nb, cudaStream_t st) {
+  switch (log2B) {
+    case 7: return run_base_t<7>(chans, nslots, rows, tw, k0, nb, st);
+    case 8: return run_base_t<8>(chans, nslots, rows, tw, k0, nb, st);
+    case 9: return run_base_t<9>(chans, nslots, rows, tw, k0, nb, st);
+    case 10: return run_base_t<10>(chans, nslots, rows, tw, k0, nb, st);
+    case 11: return run_base_t<11>(chans, nslots, rows, tw, k0, nb, st);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+cudaError_t eng_launch_run_level(int log2B, int log2N, const EngChan* chans, const EngLevel* levels, int nlev,
+                                 const EngRows& rows, const float2* tw, long long k0, int nb, long long j0, int m,
+                                 bool with_ring, cudaStream_t st) {
+  switch (log2N) {
+    case 8: return run_level_t<8, kSpecFP32>(log2B, chans, levels, nlev, rows, tw, k0, nb, j0, m, with_ring, st);
+    case 9: return run_level_t<9, kSpecFP32>(log2B, chans, levels, nlev, rows, tw, k0, nb, j0, m, with_ring, st);
+    case 10: return run_level_t<10, kSpecFP32>(log2B, chans, levels, nlev, rows, tw, k0, nb, j0, m, with_ring, st);
+    case 11: return run_level_t<11, kSpecFP32>(log2B, chans, levels, nlev, rows, tw, k0, nb, j0, m, with_ring, st);
+    case 12: return run_level_t<12, kSpecFP32>(log2B, chans, levels, nlev, rows, tw, k0, nb, j0, m, with_ring, st);
+    case 13: return run_level_t<13, kSpecFP32>(log2B, chans, levels, nlev, rows, tw, k0, nb, j0, m, with_ring, st);
+    case 14: return run_level_t<14, kSpecFP32>(log2B, chans, levels, nlev, rows, tw, k0, nb, j0, m, with_ring, st);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+cudaError_t eng_launch_run_ring(int log2B, const EngChan* chans, const EngLevel* levels, int nlev, const EngRows& rows,
+                                long long k0, int nb, long long j0, cudaStream_t st) {
+  eng_run_ring_kernel<<<dim3(((nb << log2B) + 1023) / 1024, nlev), 256, 0, st>>>(chans, levels, log2B, rows, k0, nb, j0);
+  return cudaGetLastError();
+}
+
+cudaError_t eng_launch_run_items(int log2B, const EngChan* chans, const EngLevel* levels, const EngItem* items,
+                                 int item0, int nitems, int log2N, long long ka, int nk, int grid, cudaStream_t st) {
+  if (nitems <= 0 || nk <= 0) return cudaSuccess;
+  switch (log2B) {
+    case 7: return run_items_t<7, kSpecFP32>(chans, levels, items, item0, nitems, log2N, ka, nk, grid, st);
+    case 8: return run_items_t<8, kSpecFP32>(chans, levels, items, item0, nitems, log2N, ka, nk, grid, st);
+    case 9: return run_items_t<9, kSpecFP32>(chans, levels, items, item0, nitems, log2N, ka, nk, grid, st);
+    case 10: return run_items_t<10, kSpecFP32>(chans, levels, items, item0, nitems, log2N, ka, nk, grid, st);
+    case 11: return run_items_t<11, kSpecFP32>(chans, levels, items, item0, nitems, log2N, ka, nk, grid, st);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+cudaError_t eng_launch_run_end(EngChan* chans, int nslots, EngSync sync, int nb, cudaStream_t st) {
+  eng_run_end_kernel<<<1, 256, 0, st>>>(chans, nslots, sync, nb);
+  return cudaGetLastError();
 }
 
 }  // namespace tanb

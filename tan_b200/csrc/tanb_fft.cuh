@@ -17,10 +17,16 @@
 
 namespace tanb {
 
-__device__ __forceinline__ float2 c_add(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 c_sub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+// Explicit round-to-nearest operations throughout, so that kernels that run the
+// same transform give the same bits whatever else they contain.
+__device__ __forceinline__ float2 c_add(float2 a, float2 b) {
+  return make_float2(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y));
+}
+__device__ __forceinline__ float2 c_sub(float2 a, float2 b) {
+  return make_float2(__fsub_rn(a.x, b.x), __fsub_rn(a.y, b.y));
+}
 __device__ __forceinline__ float2 c_mul(float2 a, float2 b) {
-  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+  return make_float2(__fmaf_rn(a.x, b.x, -__fmul_rn(a.y, b.y)), __fmaf_rn(a.x, b.y, __fmul_rn(a.y, b.x)));
 }
 __device__ __forceinline__ float2 c_conj(float2 a) { return make_float2(a.x, -a.y); }
 
@@ -107,10 +113,10 @@ __device__ __forceinline__ void fft_inplace(float2* s, const float2* __restrict_
 // w = W^k): returns X[k].
 __device__ __forceinline__ float2 rfft_post(float2 a, float2 b, float2 w) {
   const float2 bc = c_conj(b);
-  const float2 e = make_float2(0.5f * (a.x + bc.x), 0.5f * (a.y + bc.y));
-  const float2 d = make_float2(0.5f * (a.x - bc.x), 0.5f * (a.y - bc.y));
+  const float2 e = make_float2(__fmul_rn(0.5f, __fadd_rn(a.x, bc.x)), __fmul_rn(0.5f, __fadd_rn(a.y, bc.y)));
+  const float2 d = make_float2(__fmul_rn(0.5f, __fsub_rn(a.x, bc.x)), __fmul_rn(0.5f, __fsub_rn(a.y, bc.y)));
   const float2 t = c_mul(w, d);
-  return make_float2(e.x + t.y, e.y - t.x);
+  return make_float2(__fadd_rn(e.x, t.y), __fsub_rn(e.y, t.x));
 }
 
 // Mirror step of the inverse real transform for bin k (a = A[k],
@@ -120,13 +126,15 @@ __device__ __forceinline__ float2 irfft_pre(float2 a, float2 b, float2 w, float 
   const float2 e = c_add(a, bc);
   const float2 d = c_sub(a, bc);
   const float2 o = c_mul(d, c_conj(w));
-  return make_float2((e.x - o.y) * inv_n, (e.y + o.x) * inv_n);
+  return make_float2(__fmul_rn(__fsub_rn(e.x, o.y), inv_n), __fmul_rn(__fadd_rn(e.y, o.x), inv_n));
 }
 
 // Packed bin 0: forward (Z[0] -> (X[0], X[M])) and inverse.
-__device__ __forceinline__ float2 rfft_post_dc(float2 z0) { return make_float2(z0.x + z0.y, z0.x - z0.y); }
+__device__ __forceinline__ float2 rfft_post_dc(float2 z0) {
+  return make_float2(__fadd_rn(z0.x, z0.y), __fsub_rn(z0.x, z0.y));
+}
 __device__ __forceinline__ float2 irfft_pre_dc(float2 a, float inv_n) {
-  return make_float2((a.x + a.y) * inv_n, (a.x - a.y) * inv_n);
+  return make_float2(__fmul_rn(__fadd_rn(a.x, a.y), inv_n), __fmul_rn(__fsub_rn(a.x, a.y), inv_n));
 }
 
 // acc + a * b with the operation order of the reference's AVX2 planar MAC

@@ -64,7 +64,8 @@ __host__ __device__ inline int plan_twiddle_index(int l, int i) {
 template <int LOG2M>
 struct RegFft {
   static constexpr int M = 1 << LOG2M;
-  static constexpr int E = LOG2M <= 9 ? 8 : 16;  // complex values per thread
+  // complex values per thread (16384 points: 512 threads, 128 registers each)
+  static constexpr int E = LOG2M <= 9 ? 8 : (LOG2M <= 13 ? 16 : 32);
   static constexpr int T = M / E;
   static constexpr int NP = reg_fft_passes(LOG2M);
   static constexpr int R0 = 1 << reg_fft_lr(LOG2M, 0);
@@ -208,6 +209,24 @@ __device__ __forceinline__ void reg_pass(float2* v, const float2* w) {
   }
 }
 
+// The same with each butterfly's twiddles read from the table as it needs them.
+template <int LOG2M, int P, bool INV>
+__device__ __forceinline__ void reg_pass_table(float2* v, const float2* __restrict__ tw, int t) {
+  using F = RegFft<LOG2M>;
+  constexpr int R = F::radix(P), Ns = F::span(P);
+  const float2* s = tw + F::M + reg_fft_twoff(LOG2M, P);
+#pragma unroll
+  for (int e = 0; e < F::E / R; ++e) {
+    const int k = (t + e * F::T) & (Ns - 1);
+#pragma unroll
+    for (int r = 1; r < R; ++r) {
+      const float2 w = s[(r - 1) * Ns + k];
+      v[e * R + r] = INV ? x_mulc(v[e * R + r], w) : x_mul(v[e * R + r], w);
+    }
+    x_dft<R, INV>(v + e * R);
+  }
+}
+
 // This thread's twiddles of pass P from the table (global or shared memory).
 template <int LOG2M, int P>
 __device__ __forceinline__ void reg_twiddles(float2* w, const float2* __restrict__ tw, int t) {
@@ -268,9 +287,7 @@ __device__ __forceinline__ void reg_fft(float2* v, const float2* w, const float2
                                         float2* buf1, int t, Sync&& sync) {
   using F = RegFft<LOG2M>;
   if constexpr (P > 0 && !WREG) {
-    float2 wl[F::twn(P)];
-    reg_twiddles<LOG2M, P>(wl, tw, t);
-    reg_pass<LOG2M, P, INV>(v, wl);
+    reg_pass_table<LOG2M, P, INV>(v, tw, t);
   } else {
     reg_pass<LOG2M, P, INV>(v, w + F::tw_base(P));
   }
@@ -310,6 +327,40 @@ __device__ __forceinline__ float2 x_post_mid(float2 z) { return make_float2(z.x,
 __device__ __forceinline__ float2 x_pre_mid(float2 a, float inv_n) {
   const float s = __fmul_rn(2.0f, inv_n);
   return make_float2(__fmul_rn(a.x, s), -__fmul_rn(a.y, s));
+}
+
+// Transforms side by side in a CTA: G groups of T threads.
+template <int LOG2M>
+struct RegGroups {
+  using F = RegFft<LOG2M>;
+  static constexpr int G = F::T >= 256 ? 1 : 256 / F::T;
+  static constexpr int THREADS = G * F::T;
+  static constexpr bool PP = LOG2M <= 12;    // two exchange buffers (larger: one)
+  static constexpr bool WREG = F::E == 8;    // all twiddles in registers
+  static constexpr int SMEM = G * (PP ? 2 : 1) * F::PM * (int)sizeof(float2);
+};
+
+// Barrier of the T threads of one group: a warp or part of one, a named barrier
+// of whole warps, or the whole CTA.
+template <int T, int G>
+__device__ __forceinline__ void group_sync() {
+  if constexpr (T < 32) {
+    const unsigned lane = threadIdx.x & 31u;
+    __syncwarp(((1u << T) - 1u) << (lane / T * T));
+  } else if constexpr (T == 32) {
+    __syncwarp();
+  } else if constexpr (G > 1) {
+    asm volatile("bar.sync %0, %1;" ::"r"((int)threadIdx.x / T + 1), "n"(T) : "memory");
+  } else {
+    __syncthreads();
+  }
+}
+
+// Register that holds the lower bin of pair p after the last pass.
+template <int LOG2M>
+__device__ __forceinline__ constexpr int reg_pair(int p) {
+  constexpr int RL = RegFft<LOG2M>::RL;
+  return p / (RL / 2) * RL + p % (RL / 2);
 }
 
 }  // namespace tanb

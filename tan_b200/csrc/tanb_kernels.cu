@@ -119,35 +119,9 @@ struct CtlDesc {
 // shared memory and CTA-wide barriers it took 22 us for 8192 partitions of 512
 // (50 MB).
 template <int LOG2M>
-struct IrShape {
-  using F = RegFft<LOG2M>;
-  static constexpr int G = F::T >= 256 ? 1 : 256 / F::T;  // groups (partitions side by side) per CTA
-  static constexpr int THREADS = G * F::T;
-  static constexpr bool PP = LOG2M <= 12;                 // two exchange buffers (8192 points: one)
-  static constexpr bool WREG = F::E == 8;                 // all twiddles in registers
-  static constexpr int SMEM = G * (PP ? 2 : 1) * F::PM * (int)sizeof(float2);
-};
-
-// Barrier of the T threads of one group: a warp or part of one, a named barrier
-// of whole warps, or the whole CTA.
-template <int T, int G>
-__device__ __forceinline__ void group_sync() {
-  if constexpr (T < 32) {
-    const unsigned lane = threadIdx.x & 31u;
-    __syncwarp(((1u << T) - 1u) << (lane / T * T));
-  } else if constexpr (T == 32) {
-    __syncwarp();
-  } else if constexpr (G > 1) {
-    asm volatile("bar.sync %0, %1;" ::"r"((int)threadIdx.x / T + 1), "n"(T) : "memory");
-  } else {
-    __syncthreads();
-  }
-}
-
-template <int LOG2M>
-__global__ void __launch_bounds__(IrShape<LOG2M>::THREADS)
+__global__ void __launch_bounds__(RegGroups<LOG2M>::THREADS)
     ir_spectrum_kernel(DevState s, IrRows ir, const int* __restrict__ chans, const ChanCtl* __restrict__ ctl) {
-  using Sh = IrShape<LOG2M>;
+  using Sh = RegGroups<LOG2M>;
   using F = RegFft<LOG2M>;
   constexpr int M = F::M, T = F::T, E = F::E, G = Sh::G, RL = F::RL, NPAIR = E / 2;
   extern __shared__ __align__(16) float2 sm[];
@@ -580,11 +554,11 @@ __global__ void __launch_bounds__(UX* SY)
 // 0) and the transforms are the same register passes, so a call over several
 // blocks gives the bits of the one-block calls.
 
-// Threads of the transforms: as IrShape, runs of consecutive blocks per group.
+// Threads of the transforms: as for the IR transforms, runs of consecutive blocks per group.
 template <int LOG2M, class D>
-__global__ void __launch_bounds__(IrShape<LOG2M>::THREADS)
+__global__ void __launch_bounds__(RegGroups<LOG2M>::THREADS)
     run_forward_kernel(DevState s, const __grid_constant__ D desc, float2* __restrict__ X, int nb, int run) {
-  using Sh = IrShape<LOG2M>;
+  using Sh = RegGroups<LOG2M>;
   using F = RegFft<LOG2M>;
   constexpr int M = F::M, T = F::T, E = F::E, G = Sh::G, R0 = F::R0, RL = F::RL, NPAIR = E / 2;
   extern __shared__ __align__(16) float2 sm[];
@@ -661,10 +635,10 @@ __global__ void __launch_bounds__(IrShape<LOG2M>::THREADS)
 }
 
 template <int LOG2M, class D>
-__global__ void __launch_bounds__(IrShape<LOG2M>::THREADS)
+__global__ void __launch_bounds__(RegGroups<LOG2M>::THREADS)
     run_inverse_kernel(DevState s, const __grid_constant__ D desc, const float2* __restrict__ X,
                        const float2* __restrict__ Y, int nb, int run, int cur, HeadSignal sig) {
-  using Sh = IrShape<LOG2M>;
+  using Sh = RegGroups<LOG2M>;
   using F = RegFft<LOG2M>;
   constexpr int M = F::M, T = F::T, E = F::E, G = Sh::G, RL = F::RL, NPAIR = E / 2;
   extern __shared__ __align__(16) float2 sm[];
@@ -1224,10 +1198,10 @@ constexpr int bulk_smem_bytes() {
 template <int LOG2M, class D>
 cudaError_t set_run_attrs() {
   cudaError_t e = cudaFuncSetAttribute(run_forward_kernel<LOG2M, D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       IrShape<LOG2M>::SMEM);
+                                       RegGroups<LOG2M>::SMEM);
   if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute(run_inverse_kernel<LOG2M, D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              IrShape<LOG2M>::SMEM);
+                              RegGroups<LOG2M>::SMEM);
 }
 
 template <int LOG2M>
@@ -1241,7 +1215,7 @@ cudaError_t set_attrs() {
   e = cudaFuncSetAttribute(head_kernel<LOG2M, StgDesc>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute(ir_spectrum_kernel<LOG2M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              IrShape<LOG2M>::SMEM);
+                              RegGroups<LOG2M>::SMEM);
 }
 
 template <int LOG2M>
@@ -1257,7 +1231,7 @@ constexpr int kIrPartsPerGroup = 4;
 template <int LOG2M>
 cudaError_t launch_ir_t(const DevState& s, const IrRows& ir, const int* chans, int nch, const ChanCtl* ctl,
                         cudaStream_t st) {
-  using R = IrShape<LOG2M>;
+  using R = RegGroups<LOG2M>;
   const long long groups = ((long long)s.P * nch + R::G - 1) / R::G;  // CTAs at one partition per group
   const int iters = (int)std::max<long long>(1, std::min<long long>(kIrPartsPerGroup, groups / (148 * 2)));
   const int gx = (s.P + R::G * iters - 1) / (R::G * iters);
@@ -1292,7 +1266,7 @@ constexpr int kRunLineWarps = 148 * 4;
 template <int LOG2M>
 cudaError_t launch_run_t(const DevState& s, const BlockRef& d, const RunShape& r, cudaStream_t st,
                          const HeadSignal& sig) {
-  using Sh = IrShape<LOG2M>;
+  using Sh = RegGroups<LOG2M>;
   const int run = (int)std::max<long long>(1, std::min<long long>(kRunMax, (long long)s.C * r.nb / (Sh::G * 148LL * 2)));
   const dim3 gf((r.nb + Sh::G * run - 1) / (Sh::G * run), s.C);
   const int groups = (r.nb + 1 + kRunBlocks - 1) / kRunBlocks, per = (r.nb + 1 + groups - 1) / groups;
