@@ -193,6 +193,8 @@ struct tanb_engine {
   EngLvlUpd* d_lupd = nullptr;
   float2* d_tw = nullptr;     // the block kernel's twiddles (2B entries)
   float2* d_tw_ir = nullptr;  // the IR transforms' (the register passes' table, 2B entries)
+  float2* d_run = nullptr;    // workspace of calls over several blocks (run_blocks)
+  size_t run_bytes = 0;
   int tail_grid = 0;
   int sms = 148;  // SMs of the device
   size_t nslots_hwm = 0, nitems_hwm = 0;
@@ -269,6 +271,7 @@ constexpr size_t kMaxRetiredGraphs = 64;
 // Blocks from which a launch sequence over several blocks (a launch or two per
 // level, whatever their number) replaces one launch or more per block.
 constexpr size_t kRunMinBlocks = 4;
+constexpr size_t kRunMaxBytes = 256u << 20;  // its workspace at most
 
 void destroy_retired(tanb_engine* e) {
   for (cudaGraphExec_t g : e->retired) cudaGraphExecDestroy(g);
@@ -300,6 +303,7 @@ void free_engine(tanb_engine* e) {
   cudaFree(e->d_lupd);
   cudaFree(e->d_tw);
   cudaFree(e->d_tw_ir);
+  cudaFree(e->d_run);
   for (float2* t : e->d_tw_lv) cudaFree(t);
   cudaFreeHost(e->h_chans);
   cudaFreeHost(e->h_items);
@@ -925,6 +929,30 @@ int32_t run_block(tanb_engine* e, const tanb::EngRows* rows) {
   return TANB_OK;
 }
 
+// Workspace of a launch sequence over nb blocks: every level's spectra in turn
+// (at most one level block more than the call's samples), one level after the
+// other. Allocated by the first such call and kept; false without memory for it.
+bool ensure_run(tanb_engine* e, const Session& s, int nb) {
+  size_t per = 0;  // complex values per channel
+  for (const LevelSpec& l : s.lv) {
+    const size_t N = (size_t)1 << l.log2N, m = ((size_t)nb << e->log2B) / N + 1;
+    per = std::max(per, m > 1 ? (m + 1) * N : N);
+  }
+  const size_t need = per * e->max_channels * sizeof(float2);
+  if (need <= e->run_bytes) return true;
+  if (need > kRunMaxBytes) return false;
+  if (e->d_run && cudaStreamSynchronize(e->stream) != cudaSuccess) return false;
+  cudaFree(e->d_run);
+  e->d_run = nullptr;
+  e->run_bytes = 0;
+  if (cudaMalloc(&e->d_run, need) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  e->run_bytes = need;
+  return true;
+}
+
 // Blocks of the next launch sequence over several blocks of the engine's only
 // session (tanb_engine_kernels.cu, eng_run_*), of at most `nb`: 0 when the next
 // block has to go by itself (an update takes effect on it), -1 when all do.
@@ -953,38 +981,48 @@ int run_blocks_fit(tanb_engine* e, const Session& s, size_t nb) {
     if (off < reach) return 0;
     reach = off;
   }
-  return fit >= kRunMinBlocks ? (int)fit : -1;
+  const size_t most = kRunMaxBytes / (sizeof(float2) * e->B * e->max_channels);  // blocks of workspace
+  fit = std::min(fit, most / 3);  // a level takes up to two level blocks more than the call's samples
+  return fit >= kRunMinBlocks && ensure_run(e, s, (int)fit) ? (int)fit : -1;
 }
 
 // One launch sequence over nb blocks (as run_blocks_fit allows) of the engine's
 // only session: rows hold the blocks back to back. Caller holds mu.
 cudaError_t run_blocks(tanb_engine* e, Session& s, const tanb::EngRows& rows, int nb) {
-  const long long k0 = e->k_host;
   const int ns = (int)e->nslots_hwm;
-  cudaError_t r = tanb::eng_launch_run_input(e->log2B, e->d_chans, ns, rows, k0, nb, e->stream);
-  if (r == cudaSuccess) r = tanb::eng_launch_run_base(e->log2B, e->d_chans, ns, rows, e->d_tw, k0, nb, e->stream);
+  tanb::EngRunLevel p;
+  p.k0 = e->k_host;
+  p.nb = nb;
+  const long long kend = p.k0 + nb;
+  cudaError_t r = tanb::eng_launch_run_input(e->log2B, e->d_chans, ns, rows, p.k0, nb, e->stream);
+  if (r == cudaSuccess) r = tanb::eng_launch_run_base(e->log2B, e->d_chans, ns, rows, e->d_tw, p.k0, nb, e->stream);
   for (size_t l = 0; l < s.lv.size() && r == cudaSuccess; ++l) {
     const LevelSpec& ls = s.lv[l];
     const int c = level_class(e, ls.log2N), pshift = ls.log2N - e->log2B, nlev = (int)e->lvl_hwm[c];
     const EngLevel* lv = e->d_levels + (size_t)c * e->max_channels;
-    const long long j0 = k0 >> pshift;                       // first head at or after block k0
-    const int m = (int)(((k0 + nb) >> pshift) - j0);         // heads in the sequence
+    p.j0 = p.k0 >> pshift;                      // first head at or after block k0
+    p.m = (int)((kend >> pshift) - p.j0);       // heads in the sequence
+    p.product = ls.ngroup > 0;
+    // the heads' launch may add what the rings hold where none of its own samples
+    // takes the place of one of those
+    p.with_ring = (long long)nb * e->B + ls.off <= ls.R;
     // work items of blocks up to the head, the head, those of the blocks after it
     // (whose rows are the ones the head has read)
-    const long long kh = m && ls.ngroup ? std::min(k0 + nb, (j0 + 1) << pshift) : k0 + nb;
-    const int nit = s.C * s.items_per_chan, grid = std::min<long long>(e->tail_grid, (long long)nit * nb);
+    const long long kh = p.m && ls.ngroup ? std::min(kend, (p.j0 + 1) << pshift) : kend;
+    const int nit = s.C * s.items_per_chan;
     if (ls.ngroup)
-      r = tanb::eng_launch_run_items(e->log2B, e->d_chans, e->d_levels, e->d_items, (int)s.item0, nit, ls.log2N, k0,
-                                     (int)(kh - k0), grid, e->stream);
-    const bool with_ring = (long long)nb * e->B + ls.off <= ls.R;
-    if (r == cudaSuccess && !with_ring)
-      r = tanb::eng_launch_run_ring(e->log2B, e->d_chans, lv, nlev, rows, k0, nb, j0, e->stream);
-    if (r == cudaSuccess && (m || with_ring))
-      r = tanb::eng_launch_run_level(e->log2B, ls.log2N, e->d_chans, lv, nlev, rows, e->d_tw_lv[c], k0, nb, j0, m,
-                                     with_ring, e->stream);
+      r = tanb::eng_launch_run_items(e->log2B, e->d_chans, e->d_levels, e->d_items, (int)s.item0, nit, ls.log2N, p.k0,
+                                     (int)(kh - p.k0), e->stream);
+    if (r == cudaSuccess && !p.with_ring)
+      r = tanb::eng_launch_run_ring(e->log2B, e->d_chans, lv, nlev, rows, p,
+                                    std::min((long long)nb * e->B, ls.off + (p.j0 << ls.log2N) - (p.k0 << e->log2B)),
+                                    e->stream);
+    if (r == cudaSuccess)
+      r = tanb::eng_launch_run_level(e->log2B, ls.log2N, e->d_chans, lv, nlev, rows, e->d_tw_lv[c], e->d_run, p,
+                                     e->stream);
     if (r == cudaSuccess && ls.ngroup)
       r = tanb::eng_launch_run_items(e->log2B, e->d_chans, e->d_levels, e->d_items, (int)s.item0, nit, ls.log2N, kh,
-                                     (int)(k0 + nb - kh), grid, e->stream);
+                                     (int)(kend - kh), e->stream);
   }
   if (r == cudaSuccess)
     r = tanb::eng_launch_run_end(e->d_chans, ns, tanb::EngSync{e->d_block, e->d_done}, nb, e->stream);

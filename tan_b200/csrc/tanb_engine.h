@@ -170,21 +170,30 @@ cudaError_t eng_launch_level_commit_out(int log2B, int log2N, int spec, const En
 
 // Several blocks k0 .. k0 + nb - 1 of a non-uniform FP32 session, level by level
 // (device rows that hold the blocks back to back): the input history, the base
-// level's output (at most two partitions), what one level size's rings hold for
-// the call, its heads (level blocks j0 .. j0 + m - 1, those due in the call; with
-// what the rings hold, when `with_ring`), its work items for blocks [ka, ka + nk), and the state after
+// level's output (at most two partitions), and per level size what its rings
+// hold for the call (samples [k0 B, k0 B + samples) at most), its heads and its
+// work items for blocks [ka, ka + nk) of one level block; then the state after
 // the call.
+struct EngRunLevel {
+  long long k0 = 0;
+  int nb = 0;
+  long long j0 = 0;        // heads of level blocks j0 .. j0 + m - 1 fall into the call
+  int m = 0;
+  bool product = false;    // the level has partial rows (m <= 1)
+  bool with_ring = false;  // the heads' launch also adds what the rings hold
+};
 cudaError_t eng_launch_run_input(int log2B, const EngChan* chans, int nslots, const EngRows& rows, long long k0, int nb,
                                  cudaStream_t st);
 cudaError_t eng_launch_run_base(int log2B, const EngChan* chans, int nslots, const EngRows& rows, const float2* tw,
                                 long long k0, int nb, cudaStream_t st);
-cudaError_t eng_launch_run_level(int log2B, int log2N, const EngChan* chans, const EngLevel* levels, int nlev,
-                                 const EngRows& rows, const float2* tw, long long k0, int nb, long long j0, int m,
-                                 bool with_ring, cudaStream_t st);
 cudaError_t eng_launch_run_ring(int log2B, const EngChan* chans, const EngLevel* levels, int nlev, const EngRows& rows,
-                                long long k0, int nb, long long j0, cudaStream_t st);
+                                const EngRunLevel& p, long long samples, cudaStream_t st);
+// W: workspace of (m + 1) N complex values per record (m > 1), or N (product).
+cudaError_t eng_launch_run_level(int log2B, int log2N, const EngChan* chans, const EngLevel* levels, int nlev,
+                                 const EngRows& rows, const float2* tw, float2* W, const EngRunLevel& p,
+                                 cudaStream_t st);
 cudaError_t eng_launch_run_items(int log2B, const EngChan* chans, const EngLevel* levels, const EngItem* items,
-                                 int item0, int nitems, int log2N, long long ka, int nk, int grid, cudaStream_t st);
+                                 int item0, int nitems, int log2N, long long ka, int nk, cudaStream_t st);
 cudaError_t eng_launch_run_end(EngChan* chans, int nslots, EngSync sync, int nb, cudaStream_t st);
 
 }  // namespace tanb

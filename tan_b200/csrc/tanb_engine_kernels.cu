@@ -943,11 +943,10 @@ __device__ __forceinline__ void lv_inverse(float2 (&v)[RegFft<LOG2M>::E], const 
 }
 
 // X_j in `v` -> the products of level block j: partial rows (parity j & 1, in row
-// order), X_{j-1} H_1 (X_{j-1} from `xp` in v's layout, or from the delay line)
-// and X_j H_0.
-template <int LOG2M, int SPEC, bool XP>
-__device__ __forceinline__ void lv_products(float2 (&v)[RegFft<LOG2M>::E], const float2* xp, const EngLevel& lv,
-                                            int slot, long long j, int t) {
+// order), X_{j-1} H_1 and X_j H_0.
+template <int LOG2M, int SPEC>
+__device__ __forceinline__ void lv_products(float2 (&v)[RegFft<LOG2M>::E], const EngLevel& lv, int slot, long long j,
+                                            int t) {
   using F = RegFft<LOG2M>;
   constexpr int M = F::M, E = F::E, RL = F::RL;
   const int prv = lv_slot(j - 1, lv.Kr);
@@ -961,8 +960,7 @@ __device__ __forceinline__ void lv_products(float2 (&v)[RegFft<LOG2M>::E], const
       tm = c_add(tm, prow[(size_t)r * M + km]);
     }
     if (lv.K > 1) {
-      const float2 xk = XP ? xp[i] : x_bin<SPEC, M>(lv.fdl, prv, k);
-      const float2 xm = XP ? xp[i + RL / 2] : x_bin<SPEC, M>(lv.fdl, prv, km);
+      const float2 xk = x_bin<SPEC, M>(lv.fdl, prv, k), xm = x_bin<SPEC, M>(lv.fdl, prv, km);
       const float2 hk = lv_spec_bin<SPEC, M>(lv, slot, 1, k);
       tk = k == 0 ? c_mac_dc(tk, xk, hk) : c_mac(tk, xk, hk);
       tm = c_mac(tm, xm, lv_spec_bin<SPEC, M>(lv, slot, 1, km));
@@ -1023,7 +1021,7 @@ __global__ void __launch_bounds__(RegFft<LOG2M>::T)
     reg_fft<LOG2M, false, WREG>(v, w, tw, sm, sm, t, bar);
     lv_split<LOG2M>(v, sm, tw, t, bar);
     lv_insert<LOG2M, SPEC>(v, lv, lv_slot(j, lv.Kr), t);
-    lv_products<LOG2M, SPEC, false>(v, nullptr, lv, slot, j, t);
+    lv_products<LOG2M, SPEC>(v, lv, slot, j, t);
     lv_inverse<LOG2M, WREG>(v, w, sm, tw, t, bar);
     float* ring = lv.ring + (size_t)slot * lv.R;
     const int rmask = lv.R - 1;
@@ -1049,10 +1047,11 @@ __global__ void __launch_bounds__(RegFft<LOG2M>::T)
 // kernels in the same order, so that the samples are the same bit for bit:
 //   eng_run_input_kernel  the call's samples into the input history
 //   eng_run_base_kernel   the base level's output into the output rows
-//   eng_run_ring_kernel, eng_run_level_kernel  per level, in order: what its ring
-//                         holds for the call's blocks, and its heads, whose
-//                         samples go into the output rows as far as the call
-//                         reaches, then into the ring
+//   per level, in order:
+//     eng_run_ring_kernel     what its ring holds for the call's blocks
+//     eng_run_forward_kernel, eng_run_product_kernel, eng_run_inverse_kernel
+//                             its heads, whose samples go into the output rows as
+//                             far as the call reaches, then into the ring
 //   eng_run_items_kernel  partial rows of levels with work items
 //   eng_run_end_kernel    channel state and block counter
 __global__ void eng_run_input_kernel(const EngChan* __restrict__ chans, EngRows rows, int log2B, long long k0, int nb) {
@@ -1165,19 +1164,101 @@ __global__ void eng_run_ring_kernel(const EngChan* __restrict__ chans, const Eng
     y[a - tb] = __fadd_rn(y[a - tb], ring[a & (lv.R - 1)]);
 }
 
-// Level blocks j0 .. j0 + m - 1 of every record of one size class (those whose
-// heads fall into the call); run of them per group in turn. X_{j-1} comes from the
-// delay line when m == 1, else from a transform of its own (the other groups
-// overwrite the delay line).
+// Spectra of the level blocks that a call's heads need: X_{j0 - 1} (m > 1) and
+// X_j0 .. X_{j0 + m - 1} of every record of one size class, into the workspace
+// [record][m + 1][M] (m > 1) and, as far as they stay, into the delay line. With
+// m > 1 X_{j0 - 1} is transformed again: its slot may be overwritten here. Few
+// enough registers for several CTAs per SM: the transforms wait for memory and
+// barriers, and with the products and the inverse in one kernel (250 registers)
+// a level took 125 us at 256 channels and 16384 samples.
+template <int LOG2M>
+constexpr int run_level_ctas() {  // CTAs per SM that the registers are cut to
+  return LOG2M <= 12 ? 3 : 1;
+}
+
 template <int LOG2M, int SPEC>
-__global__ void __launch_bounds__(RegGroups<LOG2M>::THREADS)
-    eng_run_level_kernel(const EngChan* __restrict__ chans, const EngLevel* __restrict__ levels, int log2B, EngRows rows,
-                         const float2* __restrict__ tw, long long k0, int nb, long long j0, int m, int run,
-                         int with_ring) {
+__global__ void __launch_bounds__(RegGroups<LOG2M>::THREADS, run_level_ctas<LOG2M>())
+    eng_run_forward_kernel(const EngChan* __restrict__ chans, const EngLevel* __restrict__ levels, int log2B,
+                           const float2* __restrict__ tw, float2* __restrict__ X, long long te, long long j0, int m) {
   using F = RegFft<LOG2M>;
   using Sh = RegGroups<LOG2M>;
   constexpr int M = F::M, T = F::T, E = F::E, G = Sh::G, RL = F::RL;
-  constexpr bool WREG = E == 8, XP = E <= 16;
+  extern __shared__ __align__(16) float2 sm[];
+  auto bar = [] { group_sync<T, G>(); };
+  const int grp = (int)threadIdx.x / T, t = (int)threadIdx.x % T;
+  float2* buf = sm + grp * F::PM;
+  const EngLevel lv = levels[blockIdx.y];
+  if (lv.chan < 0) return;
+  const EngChan ch = chans[lv.chan];
+  if (!ch.run) return;
+  const int q = blockIdx.x * G + grp;  // position in the workspace: X_{j0 - 1 + q}, or X_{j0 + q} (m == 1)
+  if (q >= (m > 1 ? m + 1 : m)) return;
+  const long long j = m > 1 ? j0 - 1 + q : j0 + q;
+  float2 v[E];
+  lv_frame<LOG2M>(v, ch.nu->in_ring, ch.nu->rin - 1, nullptr, te, (j - 1) * M, t);
+  reg_fft<LOG2M, false, false>(v, nullptr, tw, buf, buf, t, bar);
+  lv_split<LOG2M>(v, buf, tw, t, bar);
+  if (j >= j0 && j >= j0 + m - lv.Kr) lv_insert<LOG2M, SPEC>(v, lv, lv_slot(j, lv.Kr), t);
+  if (m > 1) {
+    float2* Xq = X + ((size_t)blockIdx.y * (m + 1) + q) * M;
+#pragma unroll
+    for (int p = 0; p < E / 2; ++p) {
+      const int i = reg_pair<LOG2M>(p), k = reg_out_index<LOG2M>(t, i);
+      Xq[k] = v[i];
+      Xq[k == 0 ? M / 2 : M - k] = v[i + RL / 2];
+    }
+  }
+}
+
+// Products of level block j (the only one of its size in the call: X_{j-1} and
+// X_j are in the delay line) with its partial rows, two bins a thread, into the
+// workspace [record][N]: a streaming kernel of its own, because the rows are
+// most of a level head's bytes and its transform leaves no room for loads in
+// flight.
+template <int SPEC>
+__global__ void __launch_bounds__(256) eng_run_product_kernel(const EngChan* __restrict__ chans,
+                                                              const EngLevel* __restrict__ levels,
+                                                              float4* __restrict__ A, long long j) {
+  const EngLevel lv = levels[blockIdx.y];
+  if (lv.chan < 0) return;
+  const EngChan ch = chans[lv.chan];
+  if (!ch.run) return;
+  const int n = 1 << lv.log2N, u = blockIdx.x * 256 + threadIdx.x;
+  if (u >= n / 2) return;
+  const int slot = ch.active;
+  const float4* row = reinterpret_cast<const float4*>(lv.part + (size_t)((j & 1) * lv.ngroup) * n) + u;
+  float2 a = make_float2(0.f, 0.f), b = a;
+#pragma unroll 8
+  for (int r = 0; r < lv.ngroup; ++r) {
+    const float4 q = __ldg(row + (size_t)r * (n / 2));
+    a = c_add(a, make_float2(q.x, q.y));
+    b = c_add(b, make_float2(q.z, q.w));
+  }
+  auto mac = [&](int part, int fs) {
+    const float4 x = lv_x_unit<SPEC>(lv.fdl, n, fs, u);
+    float2 p, q;
+    lv_h2<SPEC>(lv.H, n, (size_t)slot * lv.K + part, u, p, q);
+    a = u == 0 ? c_mac_dc(a, make_float2(x.x, x.y), p) : c_mac(a, make_float2(x.x, x.y), p);
+    b = c_mac(b, make_float2(x.z, x.w), q);
+  };
+  if (lv.K > 1) mac(1, lv_slot(j - 1, lv.Kr));
+  mac(0, lv_slot(j, lv.Kr));
+  A[(size_t)blockIdx.y * (n / 2) + u] = make_float4(a.x, a.y, b.x, b.y);
+}
+
+// Outputs of the call's heads of one size class: from the products of
+// eng_run_product_kernel (`product`), else from the spectra of
+// eng_run_forward_kernel (in W, m > 1; in the delay line, m == 1); added to the
+// output rows as far as the call reaches, then into the ring. With `with_ring`
+// also what the rings hold for the call.
+template <int LOG2M, int SPEC>
+__global__ void __launch_bounds__(RegGroups<LOG2M>::THREADS, run_level_ctas<LOG2M>())
+    eng_run_inverse_kernel(const EngChan* __restrict__ chans, const EngLevel* __restrict__ levels, int log2B,
+                           EngRows rows, const float2* __restrict__ tw, const float2* __restrict__ W, long long k0,
+                           int nb, long long j0, int m, int product, int with_ring) {
+  using F = RegFft<LOG2M>;
+  using Sh = RegGroups<LOG2M>;
+  constexpr int M = F::M, T = F::T, E = F::E, G = Sh::G, RL = F::RL;
   extern __shared__ __align__(16) float2 sm[];
   auto bar = [] { group_sync<T, G>(); };
   const int grp = (int)threadIdx.x / T, t = (int)threadIdx.x % T;
@@ -1189,7 +1270,7 @@ __global__ void __launch_bounds__(RegGroups<LOG2M>::THREADS)
   float* y = row_out(rows, lv.chan);
   const bool y_vec = (reinterpret_cast<uintptr_t>(y) & 7) == 0;
   float* ring = lv.ring + (size_t)ch.active * lv.R;
-  const int rmask = lv.R - 1;
+  const int rmask = lv.R - 1, slot = ch.active;
   const long long tb = k0 << log2B, te = (k0 + nb) << log2B;
   auto add = [&](long long at, float2 o) {  // samples at, at + 1 of the stream, both inside the call or both after it
     if (at < te) {
@@ -1213,75 +1294,93 @@ __global__ void __launch_bounds__(RegGroups<LOG2M>::THREADS)
          a += 2LL * gridDim.x * blockDim.x)
       add(a, *reinterpret_cast<const float2*>(ring + (a & rmask)));
   }
-  const int r0 = ((int)blockIdx.x * G + grp) * run, r1 = min(m, r0 + run);
-  if (r0 >= m) return;
-  float2 w[WREG ? F::TWT : 1];
-  if constexpr (WREG) {
-    reg_twiddles<LOG2M, 1>(w, tw, t);
-    if constexpr (F::NP > 2) reg_twiddles<LOG2M, 2>(w + F::tw_base(2), tw, t);
-  }
-  float2 v[E], xp[XP ? E : 1];
-  auto spectrum = [&](long long j) {
-    lv_frame<LOG2M>(v, ch.nu->in_ring, ch.nu->rin - 1, nullptr, te, (j - 1) * M, t);
-    reg_fft<LOG2M, false, WREG>(v, w, tw, buf, buf, t, bar);
-    lv_split<LOG2M>(v, buf, tw, t, bar);
-  };
-  if constexpr (XP) {
-    if (m > 1 && lv.K > 1) {
-      spectrum(j0 + r0 - 1);
-#pragma unroll
-      for (int i = 0; i < E; ++i) xp[i] = v[i];
-    }
-  }
-  for (int r = r0; r < r1; ++r) {
-    const long long j = j0 + r;
-    spectrum(j);
-    if (r >= m - lv.Kr) lv_insert<LOG2M, SPEC>(v, lv, lv_slot(j, lv.Kr), t);
-    float2 xn[XP && E == 8 ? E : 1];
-    if constexpr (XP && E == 8) {
-#pragma unroll
-      for (int i = 0; i < E; ++i) xn[i] = v[i];
-    }
-    if constexpr (XP) {
-      if (m > 1) lv_products<LOG2M, SPEC, true>(v, xp, lv, ch.active, j, t);
-      else lv_products<LOG2M, SPEC, false>(v, nullptr, lv, ch.active, j, t);
-    } else {
-      lv_products<LOG2M, SPEC, false>(v, nullptr, lv, ch.active, j, t);
-    }
-    lv_inverse<LOG2M, WREG>(v, w, buf, tw, t, bar);
-    const long long base = lv.off + j * M;
+  const int r = blockIdx.x * G + grp;
+  if (r >= m) return;
+  const long long j = j0 + r;
+  float2 v[E];
+  if (product) {
+    const float2* A = W + (size_t)blockIdx.y * M;
 #pragma unroll
     for (int p = 0; p < E / 2; ++p) {
-      const int i = reg_pair<LOG2M>(p) + RL / 2;
-      add(base + 2 * (reg_out_index<LOG2M>(t, i) - M / 2), v[i]);
+      const int i = reg_pair<LOG2M>(p), k = reg_out_index<LOG2M>(t, i);
+      v[i] = A[k];
+      v[i + RL / 2] = A[k == 0 ? M / 2 : M - k];
     }
-    bar();
-    if constexpr (XP && E == 8) {
+  } else {
+    // no partial rows: X_{j-1} H_1, then X_j H_0
+    const float2* Xj = m > 1 ? W + ((size_t)blockIdx.y * (m + 1) + r + 1) * M : lv.fdl + (size_t)lv_slot(j, lv.Kr) * M;
+    const float2* Xp = m > 1 ? Xj - M : lv.fdl + (size_t)lv_slot(j - 1, lv.Kr) * M;
+    const float2* H0 = reinterpret_cast<const float2*>(lv.H) + (size_t)slot * lv.K * M;
 #pragma unroll
-      for (int i = 0; i < E; ++i) xp[i] = xn[i];
+    for (int p = 0; p < E / 2; ++p) {
+      const int i = reg_pair<LOG2M>(p), k = reg_out_index<LOG2M>(t, i), km = k == 0 ? M / 2 : M - k;
+      float2 tk = make_float2(0.f, 0.f), tm = tk;
+      if (lv.K > 1) {
+        tk = k == 0 ? c_mac_dc(tk, Xp[k], H0[M + k]) : c_mac(tk, Xp[k], H0[M + k]);
+        tm = c_mac(tm, Xp[km], H0[M + km]);
+      }
+      v[i] = k == 0 ? c_mac_dc(tk, Xj[k], H0[k]) : c_mac(tk, Xj[k], H0[k]);
+      v[i + RL / 2] = c_mac(tm, Xj[km], H0[km]);
     }
+  }
+  lv_inverse<LOG2M, false>(v, nullptr, buf, tw, t, bar);
+  const long long base = lv.off + j * M;
+#pragma unroll
+  for (int p = 0; p < E / 2; ++p) {
+    const int i = reg_pair<LOG2M>(p) + RL / 2;
+    add(base + 2 * (reg_out_index<LOG2M>(t, i) - M / 2), v[i]);
   }
 }
 
-// Work items of the level records of size 2^log2N for blocks [ka, ka + nk): one
-// (item, block) pair per step, the blocks of an item side by side (they are
-// consecutive bin slices of its rows).
-template <int LOG2B, int SPEC>
-__global__ void __launch_bounds__((1 << LOG2B) / 4)
+// Work items of the level records of size 2^log2N for blocks [ka, ka + nk) of one
+// level block: bin slices ka mod p .. of the level block after it, consecutive
+// bins, two a thread, four partitions' loads in flight. (An item at a time, as
+// the block kernel takes them, 4.1 GB took 870 us.)
+template <int SPEC>
+__global__ void __launch_bounds__(256)
     eng_run_items_kernel(const EngChan* __restrict__ chans, const EngLevel* __restrict__ levels,
-                         const EngItem* __restrict__ items, int item0, int nitems, int log2N, long long ka, int nk) {
-  const long long total = (long long)nitems * nk;
-  for (long long v = blockIdx.x; v < total; v += gridDim.x) {
-    const EngItem w = items[item0 + (int)(v / nk)];
-    if (w.chan < 0 || w.lvl < 0) continue;
-    const EngLevel lv = levels[w.lvl];
-    if (lv.log2N != log2N) continue;
-    const EngChan ch = chans[w.chan];
-    if (!ch.run) continue;
-    const long long k = ka + v % nk;
-    const int pshift = log2N - LOG2B;
-    eng_level_item<LOG2B, SPEC>(lv, w, ch.active, (k >> pshift) + 1, (int)(k & ((1LL << pshift) - 1)));
+                         const EngItem* __restrict__ items, int item0, int log2N, int log2B, long long ka, int nk) {
+  const EngItem w = items[item0 + blockIdx.y];
+  if (w.chan < 0 || w.lvl < 0) return;
+  const EngLevel lv = levels[w.lvl];
+  if (lv.log2N != log2N) return;
+  const EngChan ch = chans[w.chan];
+  if (!ch.run) return;
+  const int v = blockIdx.x * 256 + threadIdx.x;
+  if (v >= nk << (log2B - 1)) return;
+  const int pshift = log2N - log2B, n = 1 << log2N, slot = ch.active, Kr = lv.Kr;
+  const long long jb = (ka >> pshift) + 1;
+  const int u = (int)((ka & ((1LL << pshift) - 1)) << (log2B - 1)) + v;  // unit (two bins) of the row
+  const bool dc = u == 0;
+  constexpr int D = 4;
+  float2 a = make_float2(0.f, 0.f), b = a;
+  int fs = lv_slot(jb - w.i0, Kr), i = w.i0;
+  for (; i + D <= w.i1; i += D) {
+    float4 f[D];
+    float2 p[D], q[D];
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      f[d] = lv_x_unit<SPEC>(lv.fdl, n, fs, u);
+      lv_h2<SPEC>(lv.H, n, (size_t)slot * lv.K + i + d, u, p[d], q[d]);
+      fs = (fs + 1 == Kr) ? 0 : fs + 1;
+    }
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      const float2 x = make_float2(f[d].x, f[d].y);
+      a = dc ? c_mac_dc(a, x, p[d]) : c_mac(a, x, p[d]);
+      b = c_mac(b, make_float2(f[d].z, f[d].w), q[d]);
+    }
   }
+  for (; i < w.i1; ++i) {
+    const float4 f = lv_x_unit<SPEC>(lv.fdl, n, fs, u);
+    float2 p, q;
+    lv_h2<SPEC>(lv.H, n, (size_t)slot * lv.K + i, u, p, q);
+    fs = (fs + 1 == Kr) ? 0 : fs + 1;
+    const float2 x = make_float2(f.x, f.y);
+    a = dc ? c_mac_dc(a, x, p) : c_mac(a, x, p);
+    b = c_mac(b, make_float2(f.z, f.w), q);
+  }
+  reinterpret_cast<float4*>(lv.part + (size_t)((jb & 1) * lv.ngroup + w.row) * n)[u] = make_float4(a.x, a.y, b.x, b.y);
 }
 
 __global__ void eng_run_end_kernel(EngChan* __restrict__ chans, int nslots, EngSync sync, int nb) {
@@ -1501,10 +1600,10 @@ cudaError_t level_head_t(int log2B, EngChan* chans, int nslots, const EngLevel* 
 template <int LOG2M>
 cudaError_t run_base_t(const EngChan* chans, int nslots, const EngRows& rows, const float2* tw, long long k0, int nb,
                        cudaStream_t st) {
-  // runs of blocks per CTA: two thousand CTAs or more, at most 16 blocks (one
-  // transform more than its blocks per run)
-  const long long all = (long long)nslots * nb;
-  const int run = (int)(all / 2048 < 1 ? 1 : all / 2048 > 16 ? 16 : all / 2048);
+  // runs of blocks per CTA (one transform more than its blocks per run): enough
+  // CTAs to fill the GPU at 1024 threads per SM, at most 16 blocks
+  const long long all = (long long)nslots * nb, ctas = 148 * (1024 / FftShape<LOG2M>::T);
+  const int run = (int)(all / ctas < 1 ? 1 : all / ctas > 16 ? 16 : (all + ctas - 1) / ctas);
   eng_run_base_kernel<LOG2M><<<dim3((nb + run - 1) / run, nslots), FftShape<LOG2M>::T, 2 * (1 << LOG2M) * sizeof(float2),
                                st>>>(chans, rows, tw, k0, nb, run);
   return cudaGetLastError();
@@ -1512,29 +1611,28 @@ cudaError_t run_base_t(const EngChan* chans, int nslots, const EngRows& rows, co
 
 template <int LOG2M, int SPEC>
 cudaError_t run_level_t(int log2B, const EngChan* chans, const EngLevel* levels, int nlev, const EngRows& rows,
-                        const float2* tw, long long k0, int nb, long long j0, int m, bool with_ring, cudaStream_t st) {
+                        const float2* tw, float2* W, const EngRunLevel& p, cudaStream_t st) {
   using Sh = RegGroups<LOG2M>;
   constexpr int smem = Sh::G * level_smem<LOG2M>();
   static OncePerDevice once;
   const cudaError_t attr = once.run([] {
-    return cudaFuncSetAttribute(eng_run_level_kernel<LOG2M, SPEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(eng_run_forward_kernel<LOG2M, SPEC>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(eng_run_inverse_kernel<LOG2M, SPEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   });
   if (attr != cudaSuccess) return attr;
-  // runs of level blocks per group (sizes whose X_{j-1} stays in registers):
-  // about two thousand groups or more
-  const long long all = (long long)nlev * m;
-  const int run = Sh::F::E > 8 ? 1 : (int)(all / 2048 < 1 ? 1 : all / 2048 > 8 ? 8 : all / 2048);
-  const int gx = m > 0 ? (m + Sh::G * run - 1) / (Sh::G * run) : 1;
-  eng_run_level_kernel<LOG2M, SPEC><<<dim3(gx, nlev), Sh::THREADS, smem, st>>>(chans, levels, log2B, rows, tw, k0, nb,
-                                                                             j0, m, run, with_ring ? 1 : 0);
-  return cudaGetLastError();
-}
-
-template <int LOG2M, int SPEC>
-cudaError_t run_items_t(const EngChan* chans, const EngLevel* levels, const EngItem* items, int item0, int nitems,
-                        int log2N, long long ka, int nk, int grid, cudaStream_t st) {
-  eng_run_items_kernel<LOG2M, SPEC><<<grid, (1 << LOG2M) / 4, 0, st>>>(chans, levels, items, item0, nitems, log2N, ka,
-                                                                      nk);
+  if (p.m) {
+    const int nx = p.m > 1 ? p.m + 1 : p.m;
+    eng_run_forward_kernel<LOG2M, SPEC><<<dim3((nx + Sh::G - 1) / Sh::G, nlev), Sh::THREADS, smem, st>>>(
+        chans, levels, log2B, tw, W, (p.k0 + p.nb) << log2B, p.j0, p.m);
+    if (p.product)
+      eng_run_product_kernel<SPEC><<<dim3(((1 << LOG2M) / 2 + 255) / 256, nlev), 256, 0, st>>>(
+          chans, levels, reinterpret_cast<float4*>(W), p.j0);
+  }
+  if (p.m || p.with_ring)
+    eng_run_inverse_kernel<LOG2M, SPEC><<<dim3(p.m ? (p.m + Sh::G - 1) / Sh::G : 1, nlev), Sh::THREADS, smem, st>>>(
+        chans, levels, log2B, rows, tw, W, p.k0, p.nb, p.j0, p.m, p.product ? 1 : 0, p.with_ring ? 1 : 0);
   return cudaGetLastError();
 }
 
@@ -1718,37 +1816,37 @@ cudaError_t eng_launch_run_base(int log2B, const EngChan* chans, int nslots, con
 }
 
 cudaError_t eng_launch_run_level(int log2B, int log2N, const EngChan* chans, const EngLevel* levels, int nlev,
-                                 const EngRows& rows, const float2* tw, long long k0, int nb, long long j0, int m,
-                                 bool with_ring, cudaStream_t st) {
+                                 const EngRows& rows, const float2* tw, float2* W, const EngRunLevel& p,
+                                 cudaStream_t st) {
   switch (log2N) {
-    case 8: return run_level_t<8, kSpecFP32>(log2B, chans, levels, nlev, rows, tw, k0, nb, j0, m, with_ring, st);
-    case 9: return run_level_t<9, kSpecFP32>(log2B, chans, levels, nlev, rows, tw, k0, nb, j0, m, with_ring, st);
-    case 10: return run_level_t<10, kSpecFP32>(log2B, chans, levels, nlev, rows, tw, k0, nb, j0, m, with_ring, st);
-    case 11: return run_level_t<11, kSpecFP32>(log2B, chans, levels, nlev, rows, tw, k0, nb, j0, m, with_ring, st);
-    case 12: return run_level_t<12, kSpecFP32>(log2B, chans, levels, nlev, rows, tw, k0, nb, j0, m, with_ring, st);
-    case 13: return run_level_t<13, kSpecFP32>(log2B, chans, levels, nlev, rows, tw, k0, nb, j0, m, with_ring, st);
-    case 14: return run_level_t<14, kSpecFP32>(log2B, chans, levels, nlev, rows, tw, k0, nb, j0, m, with_ring, st);
+    case 8: return run_level_t<8, kSpecFP32>(log2B, chans, levels, nlev, rows, tw, W, p, st);
+    case 9: return run_level_t<9, kSpecFP32>(log2B, chans, levels, nlev, rows, tw, W, p, st);
+    case 10: return run_level_t<10, kSpecFP32>(log2B, chans, levels, nlev, rows, tw, W, p, st);
+    case 11: return run_level_t<11, kSpecFP32>(log2B, chans, levels, nlev, rows, tw, W, p, st);
+    case 12: return run_level_t<12, kSpecFP32>(log2B, chans, levels, nlev, rows, tw, W, p, st);
+    case 13: return run_level_t<13, kSpecFP32>(log2B, chans, levels, nlev, rows, tw, W, p, st);
+    case 14: return run_level_t<14, kSpecFP32>(log2B, chans, levels, nlev, rows, tw, W, p, st);
     default: return cudaErrorInvalidValue;
   }
 }
 
 cudaError_t eng_launch_run_ring(int log2B, const EngChan* chans, const EngLevel* levels, int nlev, const EngRows& rows,
-                                long long k0, int nb, long long j0, cudaStream_t st) {
-  eng_run_ring_kernel<<<dim3(((nb << log2B) + 1023) / 1024, nlev), 256, 0, st>>>(chans, levels, log2B, rows, k0, nb, j0);
+                                const EngRunLevel& p, long long samples, cudaStream_t st) {
+  if (samples <= 0) return cudaSuccess;
+  eng_run_ring_kernel<<<dim3((unsigned)((samples + 1023) / 1024), nlev), 256, 0, st>>>(chans, levels, log2B, rows, p.k0,
+                                                                                     p.nb, p.j0);
   return cudaGetLastError();
 }
 
 cudaError_t eng_launch_run_items(int log2B, const EngChan* chans, const EngLevel* levels, const EngItem* items,
-                                 int item0, int nitems, int log2N, long long ka, int nk, int grid, cudaStream_t st) {
-  if (nitems <= 0 || nk <= 0) return cudaSuccess;
-  switch (log2B) {
-    case 7: return run_items_t<7, kSpecFP32>(chans, levels, items, item0, nitems, log2N, ka, nk, grid, st);
-    case 8: return run_items_t<8, kSpecFP32>(chans, levels, items, item0, nitems, log2N, ka, nk, grid, st);
-    case 9: return run_items_t<9, kSpecFP32>(chans, levels, items, item0, nitems, log2N, ka, nk, grid, st);
-    case 10: return run_items_t<10, kSpecFP32>(chans, levels, items, item0, nitems, log2N, ka, nk, grid, st);
-    case 11: return run_items_t<11, kSpecFP32>(chans, levels, items, item0, nitems, log2N, ka, nk, grid, st);
-    default: return cudaErrorInvalidValue;
-  }
+                                 int item0, int nitems, int log2N, long long ka, int nk, cudaStream_t st) {
+  if (nk <= 0) return cudaSuccess;
+  constexpr int kMaxY = 65535;
+  const unsigned gx = (unsigned)(((nk << (log2B - 1)) + 255) / 256);
+  for (int i = 0; i < nitems; i += kMaxY)
+    eng_run_items_kernel<kSpecFP32><<<dim3(gx, nitems - i < kMaxY ? nitems - i : kMaxY), 256, 0, st>>>(
+        chans, levels, items, item0 + i, log2N, log2B, ka, nk);
+  return cudaGetLastError();
 }
 
 cudaError_t eng_launch_run_end(EngChan* chans, int nslots, EngSync sync, int nb, cudaStream_t st) {
