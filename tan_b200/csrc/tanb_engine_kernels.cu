@@ -172,20 +172,20 @@ __device__ __forceinline__ float4 x_unit(const float2* fdl, int slot, int u) {
 }
 
 // ---------------------------------------------------------------------------
-// R2C of IR partitions into IR slot `slot` of a spectrum table [2][P][M] (with
-// scales [2][P] for FP16 / BF16): partition `part` holds samples [t0 + part M,
-// t0 + (part + 1) M) of `src`, zero at and after n, zero-padded to 2M. The groups
-// of a CTA (tanb_fft_reg.cuh) take the partitions part0, part0 + step, ... of one
-// channel in turn. (One partition per CTA of M / 4 threads, radix-4 stages in
-// shared memory: 36 us for 13384 partitions of 256, now 13.)
+// R2C of IR partitions into IR slot `slot` of a spectrum table [2][P][M] (FP32,
+// FP24): partition `part` holds samples [t0 + part M, t0 + (part + 1) M) of `src`,
+// zero at and after n, zero-padded to 2M. The groups of a CTA (tanb_fft_reg.cuh)
+// take the partitions part0, part0 + step, ... of one channel in turn. (One
+// partition per CTA of M / 4 threads, radix-4 stages in shared memory: 36 us for
+// 13384 partitions of 256, now 13.) A grid of resident CTAs that loops over every
+// channel's partitions measured the same (85.4 against 84.0 us for an update of 16
+// channels with its block, 36.0 against 36.6 for one of 64).
 template <int LOG2M, int SPEC>
-__device__ __forceinline__ void ir_partitions(void* H, float* scale_tab, int P, int slot, int part0, int step,
-                                              const float* src, long long t0, long long n,
-                                              const float2* __restrict__ tw, float2* sm) {
+__device__ __forceinline__ void ir_partitions(void* H, int P, int slot, int part0, int step, const float* src,
+                                              long long t0, long long n, const float2* __restrict__ tw, float2* sm) {
   using Sh = RegGroups<LOG2M>;
   using F = RegFft<LOG2M>;
   constexpr int M = F::M, T = F::T, E = F::E, G = Sh::G, RL = F::RL, NPAIR = E / 2;
-  __shared__ float red[Sh::THREADS / 32 + 1];
   auto sync = [] { group_sync<T, G>(); };
   const int grp = (int)threadIdx.x / T, t = (int)threadIdx.x % T;
   float2* buf0 = sm + (Sh::PP ? 2 : 1) * grp * F::PM;
@@ -219,7 +219,6 @@ __device__ __forceinline__ void ir_partitions(void* H, float* scale_tab, int P, 
     sync();
     // X_k in place of the lower half, X_{M-k} in place of the upper one (bin M/2
     // beside bin 0)
-    float mx = 0.f;
 #pragma unroll
     for (int p = 0; p < NPAIR; ++p) {
       const int i = reg_pair<LOG2M>(p), k = reg_out_index<LOG2M>(t, i);
@@ -230,34 +229,7 @@ __device__ __forceinline__ void ir_partitions(void* H, float* scale_tab, int P, 
       } else {
         x_post(a, b, __ldg(tw + k), v[i], v[i + RL / 2]);
       }
-      if constexpr (kScaled<SPEC>)
-        mx = fmaxf(fmaxf(mx, fmaxf(fabsf(v[i].x), fabsf(v[i].y))), fmaxf(fabsf(v[i + RL / 2].x), fabsf(v[i + RL / 2].y)));
     }
-    float scale = 1.0f;
-    if constexpr (kScaled<SPEC>) {
-      constexpr int W = T < 32 ? T : 32;
-      const unsigned mask = T < 32 ? (((1u << W) - 1u) << ((threadIdx.x & 31u) / W * W)) : 0xffffffffu;
-#pragma unroll
-      for (int o = W / 2; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(mask, mx, o));
-      if constexpr (T > 32) {
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
-        sync();
-        mx = 0.f;
-        for (int q = 0; q < T / 32; ++q) mx = fmaxf(mx, red[grp * (T / 32) + q]);
-      }
-      // power of two with the largest magnitude mapped to [2^14, 2^15)
-      int e = 0;
-      if (mx > 0.f) {
-        frexpf(mx, &e);  // mx = f * 2^e, f in [0.5, 1)
-        e -= 15;
-      }
-      // a partition of denormal samples: keep the scale a normal number (2^-149
-      // would round to zero and its inverse overflow)
-      e = e < -126 ? -126 : e;
-      scale = ldexpf(1.0f, e);
-      if (t == 0) scale_tab[(size_t)slot * P + part] = scale;
-    }
-    const float inv = 1.0f / scale;  // exact: power of two
     const size_t row = (size_t)slot * P + part;
 #pragma unroll
     for (int p = 0; p < NPAIR; ++p) {
@@ -268,46 +240,230 @@ __device__ __forceinline__ void ir_partitions(void* H, float* scale_tab, int P, 
         f24_put<M>(r, k, Xk);
         f24_put<M>(r, km, Xm);
       } else {
-        SpecT<SPEC>::put(H, row * M + k, make_float2(Xk.x * inv, Xk.y * inv));
-        SpecT<SPEC>::put(H, row * M + km, make_float2(Xm.x * inv, Xm.y * inv));
+        SpecT<SPEC>::put(H, row * M + k, Xk);
+        SpecT<SPEC>::put(H, row * M + km, Xm);
       }
     }
     if constexpr (!Sh::PP) {
       sync();
-    } else {
-      if constexpr (kScaled<SPEC> && T > 32) sync();  // red is written again by the next partition
-      if constexpr ((F::NP & 1) != 0) {
-        float2* b = buf0;
-        buf0 = buf1;
-        buf1 = b;
-      }
+    } else if constexpr ((F::NP & 1) != 0) {
+      float2* b = buf0;
+      buf0 = buf1;
+      buf1 = b;
     }
   }
 }
 
+// ---------------------------------------------------------------------------
+// IR partitions of FP16 and BF16 spectra: one per CTA, radix-4 stages in shared
+// memory. Rounding a bin to 11 or 8 bits turns the last-bit differences of two
+// transforms into differences of half a unit of those bits now and then (2e-5 of
+// output RMS and more for BF16, 1e-5 for FP16), so these forms keep the transform
+// their spectra have always had. FP32 and FP24 take the register passes.
+namespace staged {
+
+__device__ __forceinline__ float2 c_add(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ float2 c_sub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+__device__ __forceinline__ float2 c_mul(float2 a, float2 b) {
+  return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+}
+__device__ __forceinline__ float2 c_conj(float2 a) { return make_float2(a.x, -a.y); }
+
+// W_2M^j, j < 2M, from the table's first M entries.
+template <int M>
+__device__ __forceinline__ float2 twiddle(const float2* __restrict__ tw, int j) {
+  const float2 w = tw[j & (M - 1)];
+  return j < M ? w : make_float2(-w.x, -w.y);
+}
+
+template <int LOG2M>
+__device__ __forceinline__ void fft_inplace(float2* s, const float2* __restrict__ tw) {
+  using S = FftShape<LOG2M>;
+  constexpr int M = S::M, T = S::T, E = S::E, N = 2 * M;
+  const int tid = threadIdx.x;
+  int Ns = 1;
+  if constexpr ((LOG2M & 1) != 0) {
+    constexpr int nb = M / 2;
+    float2 v[E];
+#pragma unroll
+    for (int e = 0; e < E / 2; ++e) {
+      const int j = tid + e * T;
+      v[2 * e] = s[j];
+      v[2 * e + 1] = s[j + nb];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < E / 2; ++e) {
+      const int j = tid + e * T;
+      s[2 * j] = c_add(v[2 * e], v[2 * e + 1]);
+      s[2 * j + 1] = c_sub(v[2 * e], v[2 * e + 1]);
+    }
+    __syncthreads();
+    Ns = 2;
+  }
+#pragma unroll 1
+  for (; Ns < M; Ns <<= 2) {
+    constexpr int nb = M / 4;
+    const int tstep = N / (4 * Ns);
+    float2 v[E];
+#pragma unroll
+    for (int e = 0; e < E / 4; ++e) {
+      const int j = tid + e * T;
+      const int k = j & (Ns - 1);
+      v[4 * e] = s[j];
+#pragma unroll
+      for (int r = 1; r < 4; ++r) {
+        const float2 w = twiddle<M>(tw, r * k * tstep);
+        v[4 * e + r] = c_mul(s[j + r * nb], w);
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < E / 4; ++e) {
+      const int j = tid + e * T;
+      const int k = j & (Ns - 1);
+      const float2 t0 = c_add(v[4 * e], v[4 * e + 2]);
+      const float2 t1 = c_sub(v[4 * e], v[4 * e + 2]);
+      const float2 t2 = c_add(v[4 * e + 1], v[4 * e + 3]);
+      const float2 t3 = c_sub(v[4 * e + 1], v[4 * e + 3]);
+      const float2 it3 = make_float2(-t3.y, t3.x);
+      const int d = ((j - k) << 2) + k;
+      s[d] = c_add(t0, t2);
+      s[d + Ns] = c_sub(t1, it3);
+      s[d + 2 * Ns] = c_sub(t0, t2);
+      s[d + 3 * Ns] = c_add(t1, it3);
+    }
+    __syncthreads();
+  }
+}
+
+__device__ __forceinline__ float2 rfft_post(float2 a, float2 b, float2 w) {
+  const float2 bc = c_conj(b);
+  const float2 e = make_float2(0.5f * (a.x + bc.x), 0.5f * (a.y + bc.y));
+  const float2 d = make_float2(0.5f * (a.x - bc.x), 0.5f * (a.y - bc.y));
+  const float2 t = c_mul(w, d);
+  return make_float2(e.x + t.y, e.y - t.x);
+}
+
+__device__ __forceinline__ float2 rfft_post_dc(float2 z0) { return make_float2(z0.x + z0.y, z0.x - z0.y); }
+
+// Samples [t0, t0 + M) of `src`, zero at and after n. Every thread of the CTA
+// calls it.
+template <int LOG2M, int SPEC>
+__device__ __forceinline__ void ir_partition(void* H, float* scale_tab, int P, int slot, int part, const float* src,
+                                             long long t0, long long n, const float2* __restrict__ tw, float2* sm) {
+  using S = FftShape<LOG2M>;
+  constexpr int M = S::M, T = S::T;
+  __shared__ float red[32];
+  for (int q = threadIdx.x; q < M; q += T) {
+    const long long t = t0 + 2 * q;
+    float2 v = make_float2(0.f, 0.f);
+    if (q < M / 2) {
+      if (t < n) v.x = src[t];
+      if (t + 1 < n) v.y = src[t + 1];
+    }
+    sm[q] = v;
+  }
+  __syncthreads();
+  fft_inplace<LOG2M>(sm, tw);
+  // split step in place: thread owning pair (k, M-k) writes both
+  for (int k = threadIdx.x; k <= M / 2; k += T) {
+    if (k == 0) {
+      sm[0] = rfft_post_dc(sm[0]);
+    } else {
+      const int km = M - k;
+      const float2 a = sm[k], b = sm[km];
+      const float2 Xk = rfft_post(a, b, __ldg(tw + k));
+      const float2 Xm = rfft_post(b, a, __ldg(tw + km));
+      sm[k] = Xk;
+      if (km != k) sm[km] = Xm;
+    }
+  }
+  __syncthreads();
+  float scale = 1.0f;
+  {
+    float mx = 0.f;
+    for (int k = threadIdx.x; k < M; k += T) mx = fmaxf(mx, fmaxf(fabsf(sm[k].x), fabsf(sm[k].y)));
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      mx = (threadIdx.x < (T + 31) / 32) ? red[threadIdx.x] : 0.f;
+      for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      if (threadIdx.x == 0) red[0] = mx;
+    }
+    __syncthreads();
+    mx = red[0];
+    // power of two with the largest magnitude mapped to [2^14, 2^15)
+    int e = 0;
+    if (mx > 0.f) {
+      frexpf(mx, &e);  // mx = f * 2^e, f in [0.5, 1)
+      e -= 15;
+    }
+    // a partition of denormal samples: keep the scale a normal number (2^-149
+    // would round to zero and its inverse overflow)
+    e = e < -126 ? -126 : e;
+    scale = ldexpf(1.0f, e);
+    if (threadIdx.x == 0) scale_tab[(size_t)slot * P + part] = scale;
+  }
+  const float inv = 1.0f / scale;  // exact: power of two
+  const size_t row = (size_t)slot * P + part;
+  for (int k = threadIdx.x; k < M; k += T)
+    SpecT<SPEC>::put(H, row * M + k, make_float2(sm[k].x * inv, sm[k].y * inv));
+}
+
+}  // namespace staged
+
 template <int LOG2M, int SPEC>
 __global__ void __launch_bounds__(RegGroups<LOG2M>::THREADS)
-    eng_ir_kernel(EngChan* __restrict__ chans, const EngUpd* __restrict__ upd, const float2* __restrict__ tw) {
+    eng_ir_kernel(const EngChan* __restrict__ chans, const EngUpd* __restrict__ upd,
+                  const float2* __restrict__ tw) {
   using Sh = RegGroups<LOG2M>;
   extern __shared__ __align__(16) float2 sm[];
   const EngUpd u = upd[blockIdx.y];
   const EngChan ch = chans[u.chan];
-  ir_partitions<LOG2M, SPEC>(ch.H, ch.scale, ch.P, u.slot, blockIdx.x * Sh::G + threadIdx.x / Sh::F::T,
-                             gridDim.x * Sh::G, u.src, 0, u.n, tw, sm);
+  ir_partitions<LOG2M, SPEC>(ch.H, ch.P, u.slot, blockIdx.x * Sh::G + threadIdx.x / Sh::F::T, gridDim.x * Sh::G, u.src,
+                             0, u.n, tw, sm);
 }
 
 // Partitions of non-uniform levels of one size (2^LOG2M): partition `part` of
 // level record u.lvl covers taps [off + part M, off + (part + 1) M).
 template <int LOG2M, int SPEC>
 __global__ void __launch_bounds__(RegGroups<LOG2M>::THREADS)
-    eng_level_ir_kernel(EngLevel* __restrict__ levels, const EngLvlUpd* __restrict__ upd,
+    eng_level_ir_kernel(const EngLevel* __restrict__ levels, const EngLvlUpd* __restrict__ upd,
                         const float2* __restrict__ tw) {
   using Sh = RegGroups<LOG2M>;
   extern __shared__ __align__(16) float2 sm[];
   const EngLvlUpd u = upd[blockIdx.y];
   const EngLevel lv = levels[u.lvl];
-  ir_partitions<LOG2M, SPEC>(lv.H, lv.scale, lv.K, u.slot, blockIdx.x * Sh::G + threadIdx.x / Sh::F::T,
-                             gridDim.x * Sh::G, u.src, lv.off, u.n, tw, sm);
+  ir_partitions<LOG2M, SPEC>(lv.H, lv.K, u.slot, blockIdx.x * Sh::G + threadIdx.x / Sh::F::T, gridDim.x * Sh::G, u.src,
+                             lv.off, u.n, tw, sm);
+}
+
+template <int LOG2M, int SPEC>
+__global__ void __launch_bounds__(FftShape<LOG2M>::T)
+    eng_ir_staged_kernel(const EngChan* __restrict__ chans, const EngUpd* __restrict__ upd,
+                         const float2* __restrict__ tw) {
+  extern __shared__ __align__(16) float2 sm[];
+  const int part = blockIdx.x;
+  const EngUpd u = upd[blockIdx.y];
+  const EngChan ch = chans[u.chan];
+  if (part >= ch.P) return;
+  staged::ir_partition<LOG2M, SPEC>(ch.H, ch.scale, ch.P, u.slot, part, u.src, (long long)part * (1 << LOG2M), u.n, tw,
+                                    sm);
+}
+
+template <int LOG2M, int SPEC>
+__global__ void __launch_bounds__(FftShape<LOG2M>::T)
+    eng_level_ir_staged_kernel(const EngLevel* __restrict__ levels, const EngLvlUpd* __restrict__ upd,
+                               const float2* __restrict__ tw) {
+  extern __shared__ __align__(16) float2 sm[];
+  const int part = blockIdx.x;
+  const EngLvlUpd u = upd[blockIdx.y];
+  const EngLevel lv = levels[u.lvl];
+  if (part >= lv.K) return;
+  staged::ir_partition<LOG2M, SPEC>(lv.H, lv.scale, lv.K, u.slot, part, u.src, lv.off + (long long)part * (1 << LOG2M),
+                                    u.n, tw, sm);
 }
 
 // ---------------------------------------------------------------------------
@@ -1514,8 +1670,12 @@ cudaError_t attrs_t() {
   cudaError_t e = cudaFuncSetAttribute(eng_block_kernel<LOG2M, SPEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        eng_block_smem<LOG2M>(true));
   if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(eng_ir_kernel<LOG2M, SPEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              RegGroups<LOG2M>::SMEM);
+  if constexpr (kScaled<SPEC>)
+    return cudaFuncSetAttribute(eng_ir_staged_kernel<LOG2M, SPEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (1 << LOG2M) * (int)sizeof(float2));
+  else
+    return cudaFuncSetAttribute(eng_ir_kernel<LOG2M, SPEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                RegGroups<LOG2M>::SMEM);
 }
 
 template <int LOG2M>
@@ -1542,8 +1702,12 @@ cudaError_t lattrs_t() {
   e = cudaFuncSetAttribute(eng_level_commit_out_kernel<LOG2M, SPEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            smem);
   if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(eng_level_ir_kernel<LOG2M, SPEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              RegGroups<LOG2M>::SMEM);
+  if constexpr (kScaled<SPEC>)
+    return cudaFuncSetAttribute(eng_level_ir_staged_kernel<LOG2M, SPEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (1 << LOG2M) * (int)sizeof(float2));
+  else
+    return cudaFuncSetAttribute(eng_level_ir_kernel<LOG2M, SPEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                RegGroups<LOG2M>::SMEM);
 }
 
 template <int LOG2M>
@@ -1565,17 +1729,27 @@ int ir_grid(int parts, int nupd, int groups) {
 
 template <int LOG2M, int SPEC>
 cudaError_t ir_t(EngChan* chans, const EngUpd* upd, int nupd, int maxP, const float2* tw, cudaStream_t st) {
-  using Sh = RegGroups<LOG2M>;
-  eng_ir_kernel<LOG2M, SPEC><<<dim3(ir_grid(maxP, nupd, Sh::G), nupd), Sh::THREADS, Sh::SMEM, st>>>(chans, upd, tw);
+  if constexpr (kScaled<SPEC>) {
+    using S = FftShape<LOG2M>;
+    eng_ir_staged_kernel<LOG2M, SPEC><<<dim3(maxP, nupd), S::T, S::M * sizeof(float2), st>>>(chans, upd, tw);
+  } else {
+    using Sh = RegGroups<LOG2M>;
+    eng_ir_kernel<LOG2M, SPEC><<<dim3(ir_grid(maxP, nupd, Sh::G), nupd), Sh::THREADS, Sh::SMEM, st>>>(chans, upd, tw);
+  }
   return cudaGetLastError();
 }
 
 template <int LOG2M, int SPEC>
 cudaError_t level_ir_t(EngLevel* levels, const EngLvlUpd* upd, int nupd, int maxK, const float2* tw,
                        cudaStream_t st) {
-  using Sh = RegGroups<LOG2M>;
-  eng_level_ir_kernel<LOG2M, SPEC><<<dim3(ir_grid(maxK, nupd, Sh::G), nupd), Sh::THREADS, Sh::SMEM, st>>>(levels, upd,
-                                                                                                        tw);
+  if constexpr (kScaled<SPEC>) {
+    using S = FftShape<LOG2M>;
+    eng_level_ir_staged_kernel<LOG2M, SPEC><<<dim3(maxK, nupd), S::T, S::M * sizeof(float2), st>>>(levels, upd, tw);
+  } else {
+    using Sh = RegGroups<LOG2M>;
+    eng_level_ir_kernel<LOG2M, SPEC>
+        <<<dim3(ir_grid(maxK, nupd, Sh::G), nupd), Sh::THREADS, Sh::SMEM, st>>>(levels, upd, tw);
+  }
   return cudaGetLastError();
 }
 
