@@ -136,7 +136,7 @@ struct tanb_convolution {
   float* d_ir = nullptr;
   int* h_err = nullptr;  // host-mapped error word written by kernels (DevState::err)
   // head completion for host-row calls (tanb::HeadSignal): the count lives in
-  // device memory, the flag in mapped host memory; head_seq numbers launches
+  // device memory, the flags in mapped host memory; head_seq numbers launches
   unsigned* d_head_count = nullptr;
   long long* h_head_flag = nullptr;
   long long* d_head_flag = nullptr;
@@ -623,21 +623,30 @@ int channel_flags(tanb_convolution* v, const uint32_t* flags, std::vector<uint8_
   return nrun;
 }
 
-// Waits until the head launch numbered `seq` has signalled (tanb::HeadSignal).
-// Spins on the mapped flag; every 256 polls it also asks whether ev_out (behind
+// Waits until the launch of signal `sig` has signalled (tanb::HeadSignal).
+// Spins on the mapped flags; every 256 polls it also asks whether ev_out (behind
 // the tail launched after that head) has completed, so a failed launch or a
 // missing signal ends the wait with an error instead of spinning on.
-int32_t wait_heads(tanb_convolution* v, long long seq) {
-  volatile long long* flag = v->h_head_flag;
+int32_t wait_heads(tanb_convolution* v, const tanb::HeadSignal& sig) {
+  volatile long long* flag = v->h_head_flag + (sig.each ? 1 : 0);
+  const long long seq = sig.seq;
+  int left = sig.each ? v->C : 1;  // flags still to see, in order
+  auto seen = [&] {
+    while (left && *flag >= seq) {
+      --left;
+      ++flag;
+    }
+    return left == 0;
+  };
   for (unsigned n = 1;; ++n) {
-    if (*flag >= seq) {
+    if (seen()) {
       std::atomic_thread_fence(std::memory_order_acquire);
       return TANB_OK;
     }
     if ((n & 255) == 0) {
       const cudaError_t e = cudaEventQuery(v->ev_out);
       if (e == cudaSuccess) {
-        if (*flag >= seq) continue;
+        if (seen()) continue;
         return fail(TANB_FAIL, "head launch %lld completed without signalling", seq);
       }
       if (e != cudaErrorNotReady) return fail(TANB_FAIL, "head wait: %s", cudaGetErrorString(e));
@@ -874,7 +883,7 @@ int32_t run_blocks(tanb_convolution* v, const RunCall& q, int nb, int* done, dou
   r.trow = (int)((v->blocks + nb) & 1);
   tanb::HeadSignal sig;
   const bool host_out = q.out_mem == Mem::Host;
-  if (host_out) sig = tanb::HeadSignal{v->d_head_count, v->d_head_flag, ++v->head_seq};
+  if (host_out) sig = tanb::HeadSignal{v->d_head_count, v->d_head_flag, ++v->head_seq, 0};
   v->launches[tanb_convolution::kHead] += 1;  // the inverse transforms; the forward ones count with the launch
   v->launches[tanb_convolution::kTail] += 1;
   TANB_CUDA(counted(v, tanb_convolution::kHead, [&] { return tanb::launch_run(v->ds, ref, r, v->stream, sig); }));
@@ -890,7 +899,7 @@ int32_t run_blocks(tanb_convolution* v, const RunCall& q, int nb, int* done, dou
   if (ir_stage) TANB_CUDA(cudaEventRecord(v->ev_ir, v->stream));
   if (host_out) {
     const auto t0 = std::chrono::steady_clock::now();
-    if (wait_heads(v, v->head_seq) != TANB_OK) return TANB_FAIL;
+    if (wait_heads(v, sig) != TANB_OK) return TANB_FAIL;
     *t_wait += std::chrono::duration<double, std::micro>(std::chrono::steady_clock::now() - t0).count();
     v->staging_busy = false;
     if (stage_out)
@@ -1085,6 +1094,7 @@ int32_t process_common(tanb_convolution* v, Mem in_mem, const float* const* in, 
       TANB_CUDA(cudaMemcpyAsync(v->d_stage, v->h_stage, nb * v->desc_bytes, cudaMemcpyHostToDevice, v->stream));
       TANB_CUDA(cudaEventRecord(v->ev_stage, v->stream));
     }
+    tanb::HeadSignal last_sig;
     for (int b = 0; b < nb; ++b) {
       for (int c : flush_b[b]) TANB_CUDA(flush_channel(v, c));
       const ChanCtl* dctl = v->desc_ctl(v->d_stage, b);
@@ -1101,7 +1111,8 @@ int32_t process_common(tanb_convolution* v, Mem in_mem, const float* const* in, 
       if (pcm) epi.out16 = reinterpret_cast<int16_t*>(v->h_out + (size_t)b * C * B);  // [ngroups][B] of block b
       const int parity = (int)((v->blocks + b) & 1);
       tanb::HeadSignal sig;
-      if (host_out) sig = tanb::HeadSignal{v->d_head_count, v->d_head_flag, ++v->head_seq};
+      if (host_out) sig = tanb::HeadSignal{v->d_head_count, v->d_head_flag, ++v->head_seq, param ? 1 : 0};
+      last_sig = sig;
       TANB_CUDA(counted(v, tanb_convolution::kHead,
                         [&] { return tanb::launch_head(v->ds, ref, cur_b[b], parity, v->stream, epi, sig); }));
       const bool last = (b == nb - 1);
@@ -1134,7 +1145,7 @@ int32_t process_common(tanb_convolution* v, Mem in_mem, const float* const* in, 
     if (host_out) {
       // the outputs are final once the last head has signalled; the tail
       // launched behind it keeps running while they are scattered
-      if (wait_heads(v, v->head_seq) != TANB_OK) return TANB_FAIL;
+      if (wait_heads(v, last_sig) != TANB_OK) return TANB_FAIL;
       const Clock::time_point t3 = Clock::now();
       t_wait += us(t2, t3);
       v->staging_busy = false;
@@ -1716,7 +1727,7 @@ int32_t init_impl(tanb_convolution* v, uint32_t method, uint32_t L, uint32_t B, 
     if ((e = cudaMallocHost(&v->h_ir, Cs * Ps * Bs * sizeof(float))) != cudaSuccess) break;
     if ((e = cudaMallocHost(&v->h_uctl, uctl_bytes(C))) != cudaSuccess) break;
     if ((e = cudaHostAlloc(&v->h_err, sizeof(int), cudaHostAllocMapped)) != cudaSuccess) break;
-    if ((e = cudaHostAlloc(&v->h_head_flag, sizeof(long long), cudaHostAllocMapped)) != cudaSuccess) break;
+    if ((e = cudaHostAlloc(&v->h_head_flag, (1 + tanb::kParamChannels) * sizeof(long long), cudaHostAllocMapped)) != cudaSuccess) break;
     if ((e = cudaEventCreateWithFlags(&v->ev_stage, cudaEventDisableTiming)) != cudaSuccess) break;
     if ((e = cudaEventCreateWithFlags(&v->ev_ir, cudaEventDisableTiming)) != cudaSuccess) break;
     if ((e = cudaEventCreateWithFlags(&v->ev_out, cudaEventDisableTiming)) != cudaSuccess) break;
@@ -1745,7 +1756,7 @@ int32_t init_impl(tanb_convolution* v, uint32_t method, uint32_t L, uint32_t B, 
   v->ds.C = C;
   v->ds.tw = v->d_tw;
   *v->h_err = tanb::kErrNone;
-  *v->h_head_flag = 0;
+  std::memset(v->h_head_flag, 0, (1 + tanb::kParamChannels) * sizeof(long long));
   v->head_seq = 0;
   if ((e = cudaHostGetDevicePointer(reinterpret_cast<void**>(&v->ds.err), v->h_err, 0)) != cudaSuccess ||
       (e = cudaHostGetDevicePointer(reinterpret_cast<void**>(&v->d_head_flag), v->h_head_flag, 0)) != cudaSuccess) {

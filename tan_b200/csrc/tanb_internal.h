@@ -180,15 +180,19 @@ struct MixEpi {
   int* clip = nullptr;             // set when a sample was clamped
 };
 
-// Completion signal of a head launch for host-row calls: every CTA fences its
-// output stores system-wide and counts itself in `count` (device memory, zero
-// between launches); the last one resets the count and stores `seq` into
-// `flag` (mapped host memory). The host then reads the outputs without waiting
-// for the tail launched behind the head. seq == 0: no signal.
+// Completion signal of a launch for host-row calls, in mapped host memory, so that
+// the host reads the outputs without waiting for the tail launched behind.
+// A head launch of up to kParamChannels CTAs: each CTA, its output stores fenced
+// system-wide, stores `seq` into flag[1 + channel] (`each`); the host waits for
+// every one. Other launches: each CTA counts itself in `count` (device memory,
+// zero between launches); the last one resets the count and stores `seq` into
+// flag[0], a counter's and a second fence's round trip later (2 us of a 64-channel
+// block's 25). seq == 0: no signal.
 struct HeadSignal {
   unsigned* count = nullptr;
   long long* flag = nullptr;
   long long seq = 0;
+  int each = 0;
 };
 
 // Where the IR-spectrum kernel reads row j (the IR of channel chans[j]):

@@ -447,11 +447,18 @@ __device__ __forceinline__ void head_body(const DevState& s, const D& desc, int 
   if (epi.active) mix_epilogue<M, T>(epi, c);
 }
 
-// Completion signal of a launch of `total` CTAs: every CTA, running or not,
-// counts itself once its output stores are visible to the host; the last one
-// raises the flag.
+// Completion signal of a launch of `total` CTAs (HeadSignal): every CTA, running
+// or not, once its output stores are visible to the host.
 __device__ __forceinline__ void signal_heads(const HeadSignal& sig, unsigned total) {
   if (sig.seq == 0) return;
+  if (sig.each) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence_system();  // behind the barrier: the whole CTA's stores
+      *reinterpret_cast<volatile long long*>(sig.flag + 1 + blockIdx.x) = sig.seq;
+    }
+    return;
+  }
   __threadfence_system();
   __syncthreads();
   if (threadIdx.x == 0 && atomicAdd(sig.count, 1u) == total - 1) {
