@@ -1049,6 +1049,9 @@ __device__ __forceinline__ void lv_split(float2 (&v)[RegFft<LOG2M>::E], float2* 
 #pragma unroll
   for (int i = 0; i < E; ++i)
     if (i % RL >= RL / 2) buf[F::pad(reg_out_index<LOG2M>(t, i))] = v[i];
+  float2 wk[E / 2];  // loaded side by side, not one behind each branch below
+#pragma unroll
+  for (int p = 0; p < E / 2; ++p) wk[p] = __ldg(tw + reg_out_index<LOG2M>(t, reg_pair<LOG2M>(p)));
   sync();
 #pragma unroll
   for (int p = 0; p < E / 2; ++p) {
@@ -1058,7 +1061,7 @@ __device__ __forceinline__ void lv_split(float2 (&v)[RegFft<LOG2M>::E], float2* 
       v[i] = x_post_dc(a);
       v[i + RL / 2] = x_post_mid(b);
     } else {
-      x_post(a, b, __ldg(tw + k), v[i], v[i + RL / 2]);
+      x_post(a, b, wk[p], v[i], v[i + RL / 2]);
     }
   }
   sync();
@@ -1072,6 +1075,9 @@ __device__ __forceinline__ void lv_inverse(float2 (&v)[RegFft<LOG2M>::E], const 
   using F = RegFft<LOG2M>;
   constexpr int M = F::M, E = F::E, RL = F::RL;
   const float inv_n = 1.0f / (float)(2 * M);
+  float2 wk[E / 2];
+#pragma unroll
+  for (int p = 0; p < E / 2; ++p) wk[p] = __ldg(tw + reg_out_index<LOG2M>(t, reg_pair<LOG2M>(p)));
 #pragma unroll
   for (int p = 0; p < E / 2; ++p) {
     const int i = reg_pair<LOG2M>(p), k = reg_out_index<LOG2M>(t, i), km = k == 0 ? M / 2 : M - k;
@@ -1080,7 +1086,7 @@ __device__ __forceinline__ void lv_inverse(float2 (&v)[RegFft<LOG2M>::E], const 
       zk = x_pre_dc(v[i], inv_n);
       zm = x_pre_mid(v[i + RL / 2], inv_n);
     } else {
-      x_pre(v[i], v[i + RL / 2], __ldg(tw + k), inv_n, zk, zm);
+      x_pre(v[i], v[i + RL / 2], wk[p], inv_n, zk, zm);
     }
     if constexpr (F::SYM) v[i] = zk;
     else buf[F::pad(k)] = zk;
@@ -1428,16 +1434,21 @@ __global__ void __launch_bounds__(RegGroups<LOG2M>::THREADS, run_level_ctas<LOG2
   float* ring = lv.ring + (size_t)ch.active * lv.R;
   const int rmask = lv.R - 1, slot = ch.active;
   const long long tb = k0 << log2B, te = (k0 + nb) << log2B;
-  auto add = [&](long long at, float2 o) {  // samples at, at + 1 of the stream, both inside the call or both after it
+  auto load = [&](const float* q) {
+    return y_vec ? *reinterpret_cast<const float2*>(q) : make_float2(q[0], q[1]);
+  };
+  // samples at, at + 1 of the stream, both inside the call (added to the row's
+  // `old`) or both after it
+  auto put = [&](long long at, float2 old, float2 o) {
     if (at < te) {
       if (!y) return;
       float* q = y + (at - tb);
+      const float2 s = c_add(old, o);
       if (y_vec) {
-        float2* q2 = reinterpret_cast<float2*>(q);
-        *q2 = c_add(*q2, o);
+        *reinterpret_cast<float2*>(q) = s;
       } else {
-        q[0] = __fadd_rn(q[0], o.x);
-        q[1] = __fadd_rn(q[1], o.y);
+        q[0] = s.x;
+        q[1] = s.y;
       }
     } else {
       *reinterpret_cast<float2*>(ring + (at & rmask)) = o;
@@ -1448,7 +1459,7 @@ __global__ void __launch_bounds__(RegGroups<LOG2M>::THREADS, run_level_ctas<LOG2
     const long long e = min(te, max(tb, lv.off + j0 * M));
     for (long long a = tb + 2 * (blockIdx.x * (long long)blockDim.x + threadIdx.x); a < e;
          a += 2LL * gridDim.x * blockDim.x)
-      add(a, *reinterpret_cast<const float2*>(ring + (a & rmask)));
+      if (y) put(a, load(y + (a - tb)), *reinterpret_cast<const float2*>(ring + (a & rmask)));
   }
   const int r = blockIdx.x * G + grp;
   if (r >= m) return;
@@ -1467,24 +1478,51 @@ __global__ void __launch_bounds__(RegGroups<LOG2M>::THREADS, run_level_ctas<LOG2
     const float2* Xj = m > 1 ? W + ((size_t)blockIdx.y * (m + 1) + r + 1) * M : lv.fdl + (size_t)lv_slot(j, lv.Kr) * M;
     const float2* Xp = m > 1 ? Xj - M : lv.fdl + (size_t)lv_slot(j - 1, lv.Kr) * M;
     const float2* H0 = reinterpret_cast<const float2*>(lv.H) + (size_t)slot * lv.K * M;
+    const bool two = lv.K > 1;
+    constexpr int D = E > 8 ? 1 : 2;  // bin pairs whose loads are in flight together
 #pragma unroll
-    for (int p = 0; p < E / 2; ++p) {
-      const int i = reg_pair<LOG2M>(p), k = reg_out_index<LOG2M>(t, i), km = k == 0 ? M / 2 : M - k;
-      float2 tk = make_float2(0.f, 0.f), tm = tk;
-      if (lv.K > 1) {
-        tk = k == 0 ? c_mac_dc(tk, Xp[k], H0[M + k]) : c_mac(tk, Xp[k], H0[M + k]);
-        tm = c_mac(tm, Xp[km], H0[M + km]);
+    for (int p0 = 0; p0 < E / 2; p0 += D) {
+      float2 x[D][4], h[D][4];  // X_{j-1}, X_j and H_1, H_0 at bins k and M - k
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        const int k = reg_out_index<LOG2M>(t, reg_pair<LOG2M>(p0 + d)), km = k == 0 ? M / 2 : M - k;
+        x[d][0] = two ? __ldg(Xp + k) : make_float2(0.f, 0.f);
+        x[d][1] = two ? __ldg(Xp + km) : make_float2(0.f, 0.f);
+        h[d][0] = two ? __ldg(H0 + M + k) : make_float2(0.f, 0.f);
+        h[d][1] = two ? __ldg(H0 + M + km) : make_float2(0.f, 0.f);
+        x[d][2] = __ldg(Xj + k);
+        x[d][3] = __ldg(Xj + km);
+        h[d][2] = __ldg(H0 + k);
+        h[d][3] = __ldg(H0 + km);
       }
-      v[i] = k == 0 ? c_mac_dc(tk, Xj[k], H0[k]) : c_mac(tk, Xj[k], H0[k]);
-      v[i + RL / 2] = c_mac(tm, Xj[km], H0[km]);
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        const int i = reg_pair<LOG2M>(p0 + d), k = reg_out_index<LOG2M>(t, i);
+        float2 tk = make_float2(0.f, 0.f), tm = tk;
+        if (two) {
+          tk = k == 0 ? c_mac_dc(tk, x[d][0], h[d][0]) : c_mac(tk, x[d][0], h[d][0]);
+          tm = c_mac(tm, x[d][1], h[d][1]);
+        }
+        v[i] = k == 0 ? c_mac_dc(tk, x[d][2], h[d][2]) : c_mac(tk, x[d][2], h[d][2]);
+        v[i + RL / 2] = c_mac(tm, x[d][3], h[d][3]);
+      }
     }
   }
   lv_inverse<LOG2M, false>(v, nullptr, buf, tw, t, bar);
+  // the samples of the rows so far, read together before the first is written (the
+  // compiler must take a store for one that the next load could see; with that, and
+  // the loads above, 38.9 -> 35.5 us at N = 256, 70.8 -> 62.9 at N = 8192)
   const long long base = lv.off + j * M;
+  float2 old[E / 2];
+#pragma unroll
+  for (int p = 0; p < E / 2; ++p) {
+    const long long at = base + 2 * (reg_out_index<LOG2M>(t, reg_pair<LOG2M>(p) + RL / 2) - M / 2);
+    if (at < te && y) old[p] = load(y + (at - tb));
+  }
 #pragma unroll
   for (int p = 0; p < E / 2; ++p) {
     const int i = reg_pair<LOG2M>(p) + RL / 2;
-    add(base + 2 * (reg_out_index<LOG2M>(t, i) - M / 2), v[i]);
+    put(base + 2 * (reg_out_index<LOG2M>(t, i) - M / 2), old[p], v[i]);
   }
 }
 
@@ -1774,10 +1812,13 @@ cudaError_t level_head_t(int log2B, EngChan* chans, int nslots, const EngLevel* 
 template <int LOG2M>
 cudaError_t run_base_t(const EngChan* chans, int nslots, const EngRows& rows, const float2* tw, long long k0, int nb,
                        cudaStream_t st) {
-  // runs of blocks per CTA (one transform more than its blocks per run): enough
-  // CTAs to fill the GPU at 1024 threads per SM, at most 16 blocks
-  const long long all = (long long)nslots * nb, ctas = 148 * (1024 / FftShape<LOG2M>::T);
-  const int run = (int)(all / ctas < 1 ? 1 : all / ctas > 16 ? 16 : (all + ctas - 1) / ctas);
+  // runs of blocks per CTA (one transform more than its blocks per run): the
+  // shortest whose CTAs are all resident at 1024 threads per SM, at most 16 blocks
+  // (256 channels x 128 blocks of 128: runs of 7 left 128 CTAs for a second wave,
+  // 80 us; runs of 8 take 72)
+  const long long ctas = 148 * (1024 / FftShape<LOG2M>::T);
+  int run = 1;
+  while (run < 16 && (long long)((nb + run - 1) / run) * nslots > ctas) ++run;
   eng_run_base_kernel<LOG2M><<<dim3((nb + run - 1) / run, nslots), FftShape<LOG2M>::T, 2 * (1 << LOG2M) * sizeof(float2),
                                st>>>(chans, rows, tw, k0, nb, run);
   return cudaGetLastError();
