@@ -720,6 +720,18 @@ cudaError_t ensure_mix(tanb_convolution* v, const PcmIO& pcm, tanb::MixEpi* epi)
   return cudaSuccess;
 }
 
+// Blocks from which a call goes through one launch sequence. Three blocks of 64
+// channels of 65536 taps, B = 512, take 56.9 us in it and 58.4 one by one, of 256
+// channels of 32768 150 and 162, of 16 channels of 24000, B = 256, 35.8 and 39.4;
+// two blocks 57.0 and 49.1, 147 and 131, 35.2 and 32.3. One by one, the staging of
+// caller rows runs beside the device's work on the block before, which a large
+// block's copy outweighs longer: at 512 KB of rows per block (256 channels of 512)
+// three blocks take 363 us in one sequence and 330 one by one, six 664 and 637,
+// eight 788 and 840; at 128 KB (64 channels) 108 and 114 at three already.
+constexpr size_t kRunMinBlocks = 3;
+constexpr size_t kRunStagedMinBlocks = 8;
+constexpr size_t kRunStagedBytes = 256u << 10;  // of one block's rows
+
 // Blocks of one many-block launch at most, and the device bytes of its
 // workspace at most (the rest of a call goes through further launches).
 constexpr int kRunMaxBlocks = 64;
@@ -967,13 +979,16 @@ int32_t process_common(tanb_convolution* v, Mem in_mem, const float* const* in, 
   // tail must sum its partitions in the register-load kernel's chunks. A swap
   // takes its block through the one-block path first.
   float2* run_work = nullptr;
-  bool many = nblocks > 1 && !pcm && !v->finalize_mode && v->tiling.kind == 0 && v->tiling.sy >= 8;
+  const size_t from = in_mem == Mem::Host && !direct_in && (size_t)C * B * sizeof(float) >= kRunStagedBytes
+                          ? kRunStagedMinBlocks
+                          : kRunMinBlocks;
+  bool many = nblocks >= from && !pcm && !v->finalize_mode && v->tiling.kind == 0 && v->tiling.sy >= 8;
   for (int c = 0; many && flags && c < C; ++c) many = (flags[c] & kStopInput) == 0;
   if (many) many = rows_apart(in, out, C, nblocks * (size_t)B);
   while (processed < nblocks && status == TANB_OK) {
     const Clock::time_point t0 = Clock::now();
     int nb = (int)std::min<size_t>(kMaxBlocksPerChunk, nblocks - processed);
-    if (many && nblocks - processed > 1) {
+    if (many && nblocks - processed >= from) {
       bool pend = false;
       for (int c = 0; c < C; ++c) pend = pend || v->pending[c];
       if (pend) {
@@ -1373,7 +1388,9 @@ int32_t nu_process(tanb_convolution* v, Mem in_mem, const float* const* in, Mem 
 // TIME_DOMAIN method (ConvolutionImpl.cpp:407-468, 721-762, 2645-2782)
 // ---------------------------------------------------------------------------
 
-// Rows of a direct call of at least this many bytes are staged on the host pool.
+// Rows of a direct call of at least this many bytes are staged on the host pool:
+// a call of 16 channels, 4096 taps and 2048 samples (393 KB) takes 103 us so and 106
+// on the calling thread, of 32 channels 114 and 132; of 8 channels (197 KB) 100 and 94.
 constexpr size_t kTdParallelBytes = 256u << 10;
 
 // Bytes of the call descriptors in front of the rows.

@@ -269,8 +269,10 @@ int level_class(const tanb_engine* e, int log2N) { return log2N - e->log2B - 1; 
 constexpr size_t kMaxRetiredGraphs = 64;
 
 // Blocks from which a launch sequence over several blocks (a launch or two per
-// level, whatever their number) replaces one launch or more per block.
-constexpr size_t kRunMinBlocks = 4;
+// level, whatever their number) replaces one launch or more per block: six blocks
+// of 128 take 90 us so and 99 block by block at 2 channels of 65536 taps, 114 and
+// 132 at 64 channels; four blocks 80 and 70, 102 and 99.
+constexpr size_t kRunMinBlocks = 5;
 constexpr size_t kRunMaxBytes = 256u << 20;  // its workspace at most
 
 void destroy_retired(tanb_engine* e) {

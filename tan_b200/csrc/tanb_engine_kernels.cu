@@ -1,11 +1,11 @@
 // Kernels of the batched engine: every channel of every open session runs in
 // ONE graph launch per audio block.
 //
-//   eng_ir_kernel      one CTA per (IR partition, updated channel): R2C of the
-//                      partition, optional FP16/BF16 quantisation with a
-//                      power-of-two per-partition scale, stored in the idle slot
-//                      (runs on the engine's update stream); eng_level_ir_kernel
-//                      the same for the partitions of a non-uniform level
+//   eng_ir_kernel      R2C of the partitions of an updated channel into the idle
+//                      slot (runs on the engine's update stream);
+//                      eng_ir_staged_kernel for FP16/BF16 spectra, with a
+//                      power-of-two scale per partition; eng_level_ir_* the same
+//                      for the partitions of a non-uniform level
 //   eng_block_kernel   per block: the first CTAs are a persistent grid over
 //                      work items (channel, partition range within [2, P))
 //                      writing the partial sums of the NEXT block; the last
@@ -38,6 +38,7 @@
 //                      partial rows of the level blocks still to come and the
 //                      output of level blocks whose output is still to be
 //                      played, recomputed with the new IR
+//   eng_run_*_kernel   several blocks of a non-uniform session in one call
 //
 // The per-block sums are the reference's head and tail
 // (tan/tanlibrary/src/TrueAudioNext/convolution/ConvolutionImpl.cpp:2380-2643);

@@ -31,16 +31,11 @@ __device__ __forceinline__ float2 c_mul(float2 a, float2 b) {
 __device__ __forceinline__ float2 c_conj(float2 a) { return make_float2(a.x, -a.y); }
 
 // Threads per FFT block and complex values each thread holds per stage.
-// TW_SMEM: the 2M-entry twiddle table is staged in shared memory (it fits
-// beside two M-point work buffers up to M = 2048).
 template <int LOG2M>
 struct FftShape {
   static constexpr int M = 1 << LOG2M;
   static constexpr int T = (M / 4 > 1024) ? 1024 : M / 4;
   static constexpr int E = M / T;
-  static constexpr bool TW_SMEM = LOG2M <= 11;
-  // bin pairs (k, M-k), k in [0, M/2], handled per thread
-  static constexpr int KP = (M / 2 + 1 + T - 1) / T;
 };
 
 // In-place M-point complex FFT of s[0..M) (forward: exp(-i..), inverse:

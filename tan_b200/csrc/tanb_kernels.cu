@@ -1,6 +1,7 @@
 // sm_100a kernels of the uniformly-partitioned overlap-save convolution.
 //
-//   ir_spectrum_kernel  one CTA per (IR partition, channel): R2C of [h_i, 0^B]
+//   ir_spectrum_kernel  R2C of the IR partitions [h_i, 0^B], one per group of
+//                       threads (tanb_fft_reg.cuh)
 //   head_kernel         one CTA per channel: R2C of [x_{k-1}, x_k] into the
 //                       delay line, MAC with partition 0, add the precomputed
 //                       tail, C2R, output the upper B samples (crossfading old
@@ -9,6 +10,7 @@
 //                       (the HBM-bound kernel): float4 loads of the IR spectrum
 //                       and the delay line, partitions split across warps and
 //                       reduced in shared memory in a fixed order
+//   run_*_kernel        the same for a call over several blocks at once
 //
 // The reference computes the same sums on the CPU with an overlap-add form
 // (tan/tanlibrary/src/TrueAudioNext/convolution/ConvolutionImpl.cpp:2380-2643);
@@ -1267,8 +1269,11 @@ cudaError_t launch_head_t(const DevState& s, const BlockRef& d, int cur, int par
 // enough that every SM has work.
 constexpr int kRunMax = 8;
 
-// Warps from which run_mac_line_kernel takes the sums.
-constexpr int kRunLineWarps = 148 * 4;
+// Warps from which run_mac_line_kernel takes the sums. Its CTAs go through all
+// partitions in series: a call of 12 blocks of 512 with 65536 taps takes 34 us with
+// run_mac_kernel and 61 with it at one channel, 58 and 74 at 32 channels (512
+// warps), 90 and 90 at 64 (1024 warps).
+constexpr int kRunLineWarps = 148 * 6;
 
 template <int LOG2M>
 cudaError_t launch_run_t(const DevState& s, const BlockRef& d, const RunShape& r, cudaStream_t st,
