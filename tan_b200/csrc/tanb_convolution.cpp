@@ -1452,17 +1452,10 @@ int32_t td_launch(tanb_convolution* v, int n, size_t rows, bool overlap, float* 
   const size_t C = v->C, len = v->length;
   const tanb::TdChan* h_ch = reinterpret_cast<const tanb::TdChan*>(v->h_td);
   const tanb::TdChan* d_ch = reinterpret_cast<const tanb::TdChan*>(v->d_td);
-  if (overlap) {
-    // the inputs enter the history first, from descriptors that still hold them
-    TANB_CUDA(cudaMemcpyAsync(v->d_td, v->h_td, C * sizeof(tanb::TdChan), cudaMemcpyHostToDevice, v->stream));
-    TANB_CUDA(tanb::launch_td_insert(v->td_hist, (int)len, d_ch, (int)C, n, v->stream));
-    TANB_CUDA(cudaStreamSynchronize(v->stream));
-    for (size_t c = 0; c < C; ++c) reinterpret_cast<tanb::TdChan*>(v->h_td)[c].in = nullptr;
-  }
   const size_t bytes = rows ? td_desc_bytes(C) + rows * sizeof(float) : C * sizeof(tanb::TdChan);
   TANB_CUDA(cudaMemcpyAsync(v->d_td, v->h_td, bytes, cudaMemcpyHostToDevice, v->stream));
   TANB_CUDA(counted(v, tanb_convolution::kTail, [&] {
-    return tanb::launch_td(v->td_hist, (int)len, d_ch, (int)C, n, v->B, v->stream);
+    return tanb::launch_td(v->td_hist, (int)len, d_ch, (int)C, n, v->B, overlap, v->stream);
   }));
   TANB_CUDA(cudaStreamSynchronize(v->stream));
   if (host_out)

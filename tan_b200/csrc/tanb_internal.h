@@ -263,11 +263,10 @@ struct TdChan {
 };
 
 // TIME_DOMAIN: n direct-FIR outputs of each running channel, whose n input
-// samples enter its circular history (len samples, [C][len]). No output row
-// may overlap an input row; launch_td_insert first (and a null `in`) where one does.
-cudaError_t launch_td(float* hist, int len, const TdChan* ch, int C, int n, int fade_len, cudaStream_t st);
-// The history's new samples alone.
-cudaError_t launch_td_insert(float* hist, int len, const TdChan* ch, int C, int n, cudaStream_t st);
+// samples enter its circular history (len samples, [C][len]). `overlap`: output
+// rows may overlap input rows (one launch more).
+cudaError_t launch_td(float* hist, int len, const TdChan* ch, int C, int n, int fade_len, bool overlap,
+                      cudaStream_t st);
 
 // Sets the shared-memory attributes of the kernels of one block size (once per
 // device and size: setting one loads the kernel).

@@ -9,7 +9,9 @@
 // with the call's n inputs already in the history at pos .. pos + n - 1 (mod
 // len). One launch: a sample that this call writes is read from the caller's
 // row, every other one from the history, so that no CTA waits for another's
-// history stores.
+// history stores. Where output rows overlap input rows the inputs enter the
+// history in a launch of their own (td_insert_kernel), and every sample is then
+// read from there.
 //
 // Taps are accumulated in increasing k with fused multiply-adds, the order of
 // the reference's loop (another order differs from it by more than the 1e-5 of
@@ -184,8 +186,9 @@ __device__ __forceinline__ void fir_tile(const float* __restrict__ h, int len, c
   }
 }
 
+// `inserted`: the history already holds the call's inputs.
 __global__ void __launch_bounds__(32 * kWarps) td_fir_kernel(float* hist, int len, const TdChan* __restrict__ ch,
-                                                             int C, int n, int fade_len) {
+                                                             int C, int n, int fade_len, int inserted) {
   __shared__ __align__(16) TdSmem sms[kWarps];
   // output tiles of all channels over the warps in turn
   const int tiles = (n + kTJ - 1) / kTJ, lane = threadIdx.x & 31;
@@ -193,8 +196,9 @@ __global__ void __launch_bounds__(32 * kWarps) td_fir_kernel(float* hist, int le
   const int c = (int)(id / tiles), j0 = (int)(id % tiles) * kTJ;
   if (c >= C) return;
   TdSmem& sm = sms[threadIdx.x >> 5];
-  const TdChan t = ch[c];
+  TdChan t = ch[c];
   if (!t.run) return;
+  if (inserted) t.in = nullptr;
   float* h = hist + (size_t)c * len;
   float a[kOut], b[kOut];
   fir_tile(h, len, t, t.ir, n, j0, sm, a);
@@ -223,8 +227,7 @@ __global__ void __launch_bounds__(32 * kWarps) td_fir_kernel(float* hist, int le
   for (int j = j0 + lane; j < min(n, j0 + kTJ); j += 32) t.out[j] = sm.xs[j - j0];
 }
 
-// hist[c][(pos + i) mod len] = in[c][i], i < n, for calls whose output rows
-// overlap input rows: the FIR launch behind it then reads the history alone.
+// hist[c][(pos + i) mod len] = in[c][i], i < n.
 __global__ void td_insert_kernel(float* hist, int len, const TdChan* __restrict__ ch, int n) {
   const int c = blockIdx.y;
   const TdChan t = ch[c];
@@ -236,16 +239,13 @@ __global__ void td_insert_kernel(float* hist, int len, const TdChan* __restrict_
 
 }  // namespace
 
-cudaError_t launch_td_insert(float* hist, int len, const TdChan* ch, int C, int n, cudaStream_t st) {
+cudaError_t launch_td(float* hist, int len, const TdChan* ch, int C, int n, int fade_len, bool overlap,
+                      cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
-  td_insert_kernel<<<dim3((n + 255) / 256, C), 256, 0, st>>>(hist, len, ch, n);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_td(float* hist, int len, const TdChan* ch, int C, int n, int fade_len, cudaStream_t st) {
-  if (n <= 0) return cudaSuccess;
+  if (overlap) td_insert_kernel<<<dim3((n + 255) / 256, C), 256, 0, st>>>(hist, len, ch, n);
   const long long warps = (long long)C * ((n + kTJ - 1) / kTJ);
-  td_fir_kernel<<<(unsigned)((warps + kWarps - 1) / kWarps), 32 * kWarps, 0, st>>>(hist, len, ch, C, n, fade_len);
+  td_fir_kernel<<<(unsigned)((warps + kWarps - 1) / kWarps), 32 * kWarps, 0, st>>>(hist, len, ch, C, n, fade_len,
+                                                                                overlap ? 1 : 0);
   return cudaGetLastError();
 }
 
