@@ -180,9 +180,9 @@ struct tanb_convolution {
   // one block, pinned (h_td) and on the device (d_td), so that one transfer
   // takes what the call uses of it; host output rows are written in place in
   // pinned memory.
-  char* h_td = nullptr;        // pinned: TdChan[C], then [2][C][length] floats
+  char* h_td = nullptr;        // pinned: TdChan[C], then C rows (td_row_floats)
   char* d_td = nullptr;
-  float* h_td_out = nullptr;   // pinned [C][length]
+  float* h_td_out = nullptr;   // pinned [C][max(length, B)]
   std::vector<int> td_pos;
   int td_fade = -1;            // crossfade sample index, -1 when none
   std::vector<int> td_swapping;
@@ -1396,14 +1396,18 @@ constexpr size_t kTdParallelBytes = 256u << 10;
 // Bytes of the call descriptors in front of the rows.
 size_t td_desc_bytes(size_t C) { return (C * sizeof(tanb::TdChan) + 255) & ~size_t(255); }
 
+// Floats per channel behind the descriptors: ProcessDirect's taps and inputs
+// (length samples each at most) or Process's inputs (a block, which may be longer).
+size_t td_row_floats(const tanb_convolution* v) { return std::max<size_t>(2 * (size_t)v->length, v->B); }
+
 cudaError_t td_alloc(tanb_convolution* v) {
-  const size_t C = v->C, len = v->length, block = td_desc_bytes(C) + 2 * C * len * sizeof(float);
+  const size_t C = v->C, len = v->length, block = td_desc_bytes(C) + C * td_row_floats(v) * sizeof(float);
   cudaError_t e;
   if ((e = dev_alloc(v, &v->td_hist, C * len)) != cudaSuccess) return e;
   if ((e = dev_alloc(v, &v->td_ir, 2 * C * len)) != cudaSuccess) return e;
   if ((e = dev_alloc(v, &v->d_td, block)) != cudaSuccess) return e;
   if ((e = cudaMallocHost(&v->h_td, block)) != cudaSuccess) return e;
-  if ((e = cudaMallocHost(&v->h_td_out, C * len * sizeof(float))) != cudaSuccess) return e;
+  if ((e = cudaMallocHost(&v->h_td_out, C * std::max<size_t>(len, v->B) * sizeof(float))) != cudaSuccess) return e;
   v->td_pos.assign(C, 0);
   v->td_fade = -1;
   v->td_swapping.assign(C, 0);

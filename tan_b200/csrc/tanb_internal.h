@@ -263,8 +263,9 @@ struct TdChan {
 };
 
 // TIME_DOMAIN: n direct-FIR outputs of each running channel, whose n input
-// samples enter its circular history (len samples, [C][len]). `overlap`: output
-// rows may overlap input rows (one launch more).
+// samples enter its circular history (len samples, [C][len]); n above len goes
+// through it in pieces of len. `overlap`: output rows may overlap input rows (one
+// launch more per piece).
 cudaError_t launch_td(float* hist, int len, const TdChan* ch, int C, int n, int fade_len, bool overlap,
                       cudaStream_t st);
 

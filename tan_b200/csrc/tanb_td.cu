@@ -186,9 +186,10 @@ __device__ __forceinline__ void fir_tile(const float* __restrict__ h, int len, c
   }
 }
 
-// `inserted`: the history already holds the call's inputs.
+// The n <= len samples of the rows from `at` on. `inserted`: the history already
+// holds them.
 __global__ void __launch_bounds__(32 * kWarps) td_fir_kernel(float* hist, int len, const TdChan* __restrict__ ch,
-                                                             int C, int n, int fade_len, int inserted) {
+                                                             int C, int n, int at, int fade_len, int inserted) {
   __shared__ __align__(16) TdSmem sms[kWarps];
   // output tiles of all channels over the warps in turn
   const int tiles = (n + kTJ - 1) / kTJ, lane = threadIdx.x & 31;
@@ -198,7 +199,9 @@ __global__ void __launch_bounds__(32 * kWarps) td_fir_kernel(float* hist, int le
   TdSmem& sm = sms[threadIdx.x >> 5];
   TdChan t = ch[c];
   if (!t.run) return;
-  if (inserted) t.in = nullptr;
+  t.in = (t.in && !inserted) ? t.in + at : nullptr;
+  t.out = t.out ? t.out + at : nullptr;
+  t.fade0 += at;
   float* h = hist + (size_t)c * len;
   float a[kOut], b[kOut];
   fir_tile(h, len, t, t.ir, n, j0, sm, a);
@@ -227,26 +230,33 @@ __global__ void __launch_bounds__(32 * kWarps) td_fir_kernel(float* hist, int le
   for (int j = j0 + lane; j < min(n, j0 + kTJ); j += 32) t.out[j] = sm.xs[j - j0];
 }
 
-// hist[c][(pos + i) mod len] = in[c][i], i < n.
-__global__ void td_insert_kernel(float* hist, int len, const TdChan* __restrict__ ch, int n) {
+// hist[c][(pos + i) mod len] = in[c][at + i], i < n <= len.
+__global__ void td_insert_kernel(float* hist, int len, const TdChan* __restrict__ ch, int n, int at) {
   const int c = blockIdx.y;
   const TdChan t = ch[c];
   if (!t.run || !t.in) return;
   float* h = hist + (size_t)c * len;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    h[wrap(t.pos, i, len)] = t.in[i];
+    h[wrap(t.pos, i, len)] = t.in[at + i];
 }
 
 }  // namespace
 
 cudaError_t launch_td(float* hist, int len, const TdChan* ch, int C, int n, int fade_len, bool overlap,
                       cudaStream_t st) {
-  if (n <= 0) return cudaSuccess;
-  if (overlap) td_insert_kernel<<<dim3((n + 255) / 256, C), 256, 0, st>>>(hist, len, ch, n);
-  const long long warps = (long long)C * ((n + kTJ - 1) / kTJ);
-  td_fir_kernel<<<(unsigned)((warps + kWarps - 1) / kWarps), 32 * kWarps, 0, st>>>(hist, len, ch, C, n, fade_len,
-                                                                                overlap ? 1 : 0);
-  return cudaGetLastError();
+  // The history takes len samples at a time, after which its position is the same
+  // again: a longer call (a block above the response's length rounded up) goes
+  // through it in pieces, each with the samples and results of a call of its own.
+  for (int at = 0; at < n; at += len) {
+    const int m = n - at < len ? n - at : len;
+    if (overlap) td_insert_kernel<<<dim3((m + 255) / 256, C), 256, 0, st>>>(hist, len, ch, m, at);
+    const long long warps = (long long)C * ((m + kTJ - 1) / kTJ);
+    td_fir_kernel<<<(unsigned)((warps + kWarps - 1) / kWarps), 32 * kWarps, 0, st>>>(hist, len, ch, C, m, at, fade_len,
+                                                                                  overlap ? 1 : 0);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 }  // namespace tanb
