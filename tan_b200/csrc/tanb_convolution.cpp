@@ -128,6 +128,7 @@ struct tanb_convolution {
   std::vector<std::vector<uint8_t>> scr_run_b;
   std::vector<std::vector<int>> scr_flush_b;
   std::vector<int> scr_cur_b;
+  std::vector<std::pair<uintptr_t, int>> scr_rows;  // row_relation
   tanb::CtlParam last_ctlp{};
   bool last_is_param = false;
 
@@ -363,22 +364,43 @@ int32_t run_pending_finalize(tanb_convolution* v) {
   return TANB_OK;
 }
 
-// True when no input row of n samples touches a byte between the first and the
-// last output row (null rows aside).
-bool spans_apart(const float* const* in, float* const* out, int C, size_t n) {
+// How the output rows of a call lie to its input rows of n samples each (null
+// rows aside): no byte in common; in common only where a channel's output is its
+// own input row; or otherwise. Exact, so that rows that take turns in one buffer
+// count as apart; only rows whose address ranges meet are looked at one by one.
+enum class Rows { Apart, InPlace, Overlap };
+
+Rows row_relation(tanb_convolution* v, const float* const* in, float* const* out, int C, size_t n) {
+  const uintptr_t w = n * sizeof(float);
   uintptr_t il = UINTPTR_MAX, ih = 0, ol = UINTPTR_MAX, oh = 0;
   for (int c = 0; c < C; ++c) {
     const uintptr_t a = reinterpret_cast<uintptr_t>(in[c]), b = reinterpret_cast<uintptr_t>(out[c]);
     if (a) {
       il = std::min(il, a);
-      ih = std::max(ih, a + n * sizeof(float));
+      ih = std::max(ih, a + w);
     }
     if (b) {
       ol = std::min(ol, b);
-      oh = std::max(oh, b + n * sizeof(float));
+      oh = std::max(oh, b + w);
     }
   }
-  return il >= oh || ol >= ih;
+  if (il >= oh || ol >= ih) return Rows::Apart;
+  auto& rows = v->scr_rows;  // input rows by address
+  rows.clear();
+  for (int c = 0; c < C; ++c)
+    if (in[c]) rows.emplace_back(reinterpret_cast<uintptr_t>(in[c]), c);
+  std::sort(rows.begin(), rows.end());
+  Rows r = Rows::Apart;
+  for (int c = 0; c < C; ++c) {
+    if (!out[c]) continue;
+    const uintptr_t b = reinterpret_cast<uintptr_t>(out[c]);
+    auto q = std::partition_point(rows.begin(), rows.end(), [&](const auto& a) { return a.first + w <= b; });
+    for (; q != rows.end() && q->first < b + w; ++q) {
+      if (q->first != b || q->second != c) return Rows::Overlap;
+      r = Rows::InPlace;
+    }
+  }
+  return r;
 }
 
 int32_t td_update(tanb_convolution* v, Mem mem, const float* const* ir, size_t n, const uint32_t* flags,
@@ -773,24 +795,6 @@ int ensure_run(tanb_convolution* v, size_t nb, float2** work) {
   return v->run_blocks;
 }
 
-// True when the input and output rows of a call over n samples per row are
-// apart, or every channel's output is its own input row: reading all inputs
-// before writing any output then gives what block-by-block processing gives.
-bool rows_apart(const float* const* in, float* const* out, int C, size_t n) {
-  if (spans_apart(in, out, C, n)) return true;
-  bool same = true;
-  for (int c = 0; c < C; ++c) same = same && in[c] == out[c];
-  if (!same) return false;
-  // in place: the rows must not overlap one another
-  std::vector<uintptr_t> r;
-  for (int c = 0; c < C; ++c)
-    if (in[c]) r.push_back(reinterpret_cast<uintptr_t>(in[c]));
-  std::sort(r.begin(), r.end());
-  for (size_t j = 1; j < r.size(); ++j)
-    if (r[j] - r[j - 1] < n * sizeof(float)) return false;
-  return true;
-}
-
 // Blocks of the next of as few launches as `left` blocks need, alike in size.
 int even_share(size_t left, int cap) {
   const size_t parts = (left + cap - 1) / cap;
@@ -984,7 +988,9 @@ int32_t process_common(tanb_convolution* v, Mem in_mem, const float* const* in, 
                           : kRunMinBlocks;
   bool many = nblocks >= from && !pcm && !v->finalize_mode && v->tiling.kind == 0 && v->tiling.sy >= 8;
   for (int c = 0; many && flags && c < C; ++c) many = (flags[c] & kStopInput) == 0;
-  if (many) many = rows_apart(in, out, C, nblocks * (size_t)B);
+  // all inputs are read before any output is written: as block by block where the
+  // rows are apart or in place
+  if (many) many = row_relation(v, in, out, C, nblocks * (size_t)B) != Rows::Overlap;
   while (processed < nblocks && status == TANB_OK) {
     const Clock::time_point t0 = Clock::now();
     int nb = (int)std::min<size_t>(kMaxBlocksPerChunk, nblocks - processed);
@@ -1294,8 +1300,9 @@ int32_t nu_process(tanb_convolution* v, Mem in_mem, const float* const* in, Mem 
   // block goes one by one first).
   bool many = !host_io && nblocks > 1;
   for (int c = 0; many && flags && c < C; ++c) many = (flags[c] & kStopInput) == 0;
-  many = many && rows_apart(in, out, C, nblocks * (size_t)B);
-  const int overlap = !host_io && !spans_apart(in, out, C, nblocks * (size_t)B);
+  const Rows rel = host_io ? Rows::Apart : row_relation(v, in, out, C, nblocks * (size_t)B);
+  many = many && rel != Rows::Overlap;
+  const int overlap = rel != Rows::Apart;
   while (processed < nblocks && status == TANB_OK) {
     const int next = many ? tanb::engine_run_fit(v->nu_eng, v->nu_sess, nblocks - processed) : -1;
     const int fit = std::max(next, 0);
@@ -1511,7 +1518,8 @@ int32_t td_process(tanb_convolution* v, Mem in_mem, const float* const* in, Mem 
     }
     t.out = out_mem == Mem::Host ? v->h_td_out + c * ns : out[c];
   }
-  const bool overlap = in_mem == Mem::Device && out_mem == Mem::Device && !spans_apart(in, out, (int)C, ns);
+  const bool overlap =
+      in_mem == Mem::Device && out_mem == Mem::Device && row_relation(v, in, out, (int)C, ns) != Rows::Apart;
   int32_t r = td_launch(v, ns, in_mem == Mem::Host ? C * ns : 0, overlap,
                         out_mem == Mem::Host ? out : nullptr);
   if (r != TANB_OK) return r;
@@ -1671,6 +1679,7 @@ int32_t init_impl(tanb_convolution* v, uint32_t method, uint32_t L, uint32_t B, 
 
   cudaError_t e = cudaSetDevice(v->ctx->device);
   if (e != cudaSuccess) return fail(TANB_NO_DEVICE, "cudaSetDevice: %s", cudaGetErrorString(e));
+  v->scr_rows.reserve(C);
   auto host_state = [&] {
     v->active.assign(C, 0);
     v->pending.assign(C, 0);

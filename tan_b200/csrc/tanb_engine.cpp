@@ -1532,6 +1532,27 @@ int32_t tanb_engine_process(tanb_engine* e) {
   return TANB_OK;
 }
 
+}  // extern "C"
+
+namespace {
+
+// True when one of n rows of B samples from `in` on, ld apart, shares a byte with
+// one of n such rows from `out` on (always where such rows share bytes themselves).
+bool rows_meet(const float* in, const float* out, long long ld, size_t n, int B) {
+  if (ld < B) return true;
+  const long long d = (long long)(reinterpret_cast<uintptr_t>(out) - reinterpret_cast<uintptr_t>(in)), step = ld * 4,
+                  w = B * 4LL;
+  // output row j lies d + (j - i) step past input row i: of these distances the two
+  // next to zero are m and m - step
+  const long long m = ((d % step) + step) % step, q = (d - m) / step;
+  auto in_range = [&](long long k) { return (k < 0 ? -k : k) < (long long)n; };
+  return (m < w && in_range(-q)) || (step - m < w && in_range(-q - 1));
+}
+
+}  // namespace
+
+extern "C" {
+
 int32_t tanb_engine_process_device(tanb_engine* e, const float* in, float* out, uint32_t ld) {
   tanb::NvtxRange range("tanb engine block (device rows)");
   if (!e) return efail(TANB_INVALID_POINTER, "null engine");
@@ -1543,9 +1564,7 @@ int32_t tanb_engine_process_device(tanb_engine* e, const float* in, float* out, 
   rows.in_base = in;
   rows.out_base = out;
   rows.ld = ld ? (int)ld : e->B;
-  const uintptr_t span = ((uintptr_t)rows.ld * (e->nslots_hwm ? e->nslots_hwm - 1 : 0) + e->B) * sizeof(float);
-  const uintptr_t a = reinterpret_cast<uintptr_t>(in), b = reinterpret_cast<uintptr_t>(out);
-  rows.overlap = in && a < b + span && b < a + span;
+  rows.overlap = in && rows_meet(in, out, rows.ld, e->nslots_hwm, e->B);
   return run_block(e, &rows);
 }
 
