@@ -150,9 +150,8 @@ struct tanb_convolution {
 
   cudaEvent_t ev_stage = nullptr, ev_ir = nullptr, ev_out = nullptr;
 
-  // calls over several blocks: spectra of the new blocks and of their outputs,
-  // [2][C][run_blocks][B] float2, allocated by the first such call
-  float2* d_run = nullptr;
+  // blocks of one launch over several: spectra of the new blocks and of their
+  // outputs, [2][C][run_blocks][B] float2, in d_ir
   int run_blocks = 0;
 
   // fused PCM pipeline (tanb_convolution_process_mix_pcm16), allocated on first use
@@ -276,8 +275,6 @@ void free_all(tanb_convolution* v) {
   v->d_head_count = nullptr;
   cudaFree(v->d_ir);
   cudaFree(v->d_uctl);
-  cudaFree(v->d_run);
-  v->d_run = nullptr;
   v->run_blocks = 0;
   cudaFree(v->d_mix_scratch);
   cudaFree(v->d_mix_table);
@@ -761,38 +758,26 @@ constexpr int kRunIrBlocks = 16;
 constexpr size_t kRunSmallBytes = 8u << 20;
 constexpr size_t kRunMaxBytes = 64u << 20;
 
-// Workspace for launches over up to `nb` blocks; returns the blocks it holds
-// (0: too large for the bound, or no memory: the call then runs block by block).
-// The device rows of IR updates (C x P x B floats, used by copies and transforms
-// on the same stream only) serve where they hold the whole launch, or enough
-// blocks of a large one (kRunIrBlocks) that a second launch sequence costs little;
-// calls of a few small channels are bound by the sequence's latency (two
-// sequences for 64 blocks of two channels took 93 us instead of 56).
-int ensure_run(tanb_convolution* v, size_t nb, float2** work) {
-  const int ir = std::min(v->P / 4, kRunMaxBlocks);  // 4 B floats per block and channel
-  const size_t per = 2 * (size_t)v->C * v->B * sizeof(float2);  // bytes per block
-  const int want = (int)std::min<size_t>({nb, (size_t)kRunMaxBlocks, kRunMaxBytes / per});
-  if (ir >= 2 && (want <= ir || (ir >= kRunIrBlocks && per * want > kRunSmallBytes))) {
-    *work = reinterpret_cast<float2*>(v->d_ir);
-    return ir;
+// The device rows of IR updates (C x P x B floats, used by copies and transforms on
+// the same stream only) are the workspace too, made larger by Init where they hold
+// fewer blocks (4 B floats per block and channel) than a call can use well; a call
+// allocates nothing. Calls of a few small channels are bound by the sequence's
+// latency (two sequences for 64 blocks of two channels took 93 us instead of 56),
+// so up to kRunSmallBytes hold all kRunMaxBlocks; beyond, kRunIrBlocks are enough
+// that a second launch sequence costs little.
+cudaError_t alloc_ir_rows(tanb_convolution* v) {
+  const size_t block = 4 * (size_t)v->C * v->B, bytes = block * sizeof(float), rows = (size_t)v->C * v->P * v->B;
+  size_t most = std::min<size_t>({(size_t)kRunMaxBlocks, kRunMaxBytes / bytes,
+                                  std::max<size_t>(kRunIrBlocks, kRunSmallBytes / bytes)});
+  if (v->finalize_mode || most < 2) most = 0;
+  size_t n = std::max(rows, most * block);
+  cudaError_t e = dev_alloc(v, &v->d_ir, n);
+  if (e != cudaSuccess && n > rows) {
+    (void)cudaGetLastError();
+    e = dev_alloc(v, &v->d_ir, n = rows);
   }
-  if (want < 2) return 0;
-  if (want > v->run_blocks) {
-    // the old one may be in use by a launch in flight: freed after it
-    if (v->d_run && cudaStreamSynchronize(v->stream) != cudaSuccess) return 0;
-    cudaFree(v->d_run);
-    v->dev_bytes -= per * v->run_blocks;
-    v->d_run = nullptr;
-    v->run_blocks = 0;
-    if (cudaMalloc(&v->d_run, per * want) != cudaSuccess) {
-      (void)cudaGetLastError();
-      return 0;
-    }
-    v->run_blocks = want;
-    v->dev_bytes += per * want;
-  }
-  *work = v->d_run;
-  return v->run_blocks;
+  v->run_blocks = n / block < 2 ? 0 : (int)std::min<size_t>(n / block, kRunMaxBlocks);
+  return e;
 }
 
 // Blocks of the next of as few launches as `left` blocks need, alike in size.
@@ -811,7 +796,6 @@ struct RunCall {
   const PinnedRows* pin_in;   // caller rows addressed in place
   const PinnedRows* pin_out;
   bool param, staged;
-  float2* work;             // X and Y of RunShape
 };
 
 // Up to `nb` blocks of a call as one launch sequence; *done: how many. Host rows
@@ -891,8 +875,8 @@ int32_t run_blocks(tanb_convolution* v, const RunCall& q, int nb, int* done, dou
     ref.out = v->desc_out(v->d_stage, 0);
   }
   tanb::RunShape r;
-  r.X = q.work;
-  r.Y = q.work + (size_t)C * nb * B;
+  r.X = reinterpret_cast<float2*>(v->d_ir);
+  r.Y = r.X + (size_t)C * nb * B;
   r.nb = nb;
   r.sy = v->tiling.sy;
   r.cur = v->cur;
@@ -982,7 +966,6 @@ int32_t process_common(tanb_convolution* v, Mem in_mem, const float* const* in, 
   // then runs, and a flush can only fall on the call's first block), and the
   // tail must sum its partitions in the register-load kernel's chunks. A swap
   // takes its block through the one-block path first.
-  float2* run_work = nullptr;
   const size_t from = in_mem == Mem::Host && !direct_in && (size_t)C * B * sizeof(float) >= kRunStagedBytes
                           ? kRunStagedMinBlocks
                           : kRunMinBlocks;
@@ -999,10 +982,10 @@ int32_t process_common(tanb_convolution* v, Mem in_mem, const float* const* in, 
       for (int c = 0; c < C; ++c) pend = pend || v->pending[c];
       if (pend) {
         nb = 1;
-      } else if (const int cap = ensure_run(v, nblocks - processed, &run_work)) {
+      } else if (v->run_blocks) {
         const int32_t r = run_blocks(v, RunCall{in_mem, in, out_mem, out, flags, processed, direct_in ? &pin_in : nullptr,
-                                                direct_out ? &pin_out : nullptr, param, staged, run_work},
-                                     even_share(nblocks - processed, cap), &nb, &t_wait);
+                                                direct_out ? &pin_out : nullptr, param, staged},
+                                     even_share(nblocks - processed, v->run_blocks), &nb, &t_wait);
         if (r != TANB_OK) return r;
         processed += nb;
         v->blocks += nb;
@@ -1262,7 +1245,7 @@ int32_t nu_init(tanb_convolution* v, uint32_t L, uint32_t B, uint32_t C, uint32_
   }
   int64_t info[8];
   tanb_engine_info(v->nu_eng, info);
-  v->dev_bytes = (size_t)info[4];
+  v->dev_bytes = (size_t)info[4] + tanb::engine_run_reserve(v->nu_eng, v->nu_sess);
   return TANB_OK;
 }
 
@@ -1743,7 +1726,7 @@ int32_t init_impl(tanb_convolution* v, uint32_t method, uint32_t L, uint32_t B, 
     if ((e = dev_alloc(v, &v->d_tw, 2 * Bs)) != cudaSuccess) break;
     if ((e = dev_alloc(v, &v->d_stage, kMaxBlocksPerChunk * v->desc_bytes)) != cudaSuccess) break;
     if ((e = dev_alloc(v, &v->d_head_count, 1)) != cudaSuccess) break;
-    if ((e = dev_alloc(v, &v->d_ir, Cs * Ps * Bs)) != cudaSuccess) break;
+    if ((e = alloc_ir_rows(v)) != cudaSuccess) break;
     if ((e = dev_alloc(v, &v->d_uctl, uctl_bytes(C))) != cudaSuccess) break;
     if ((e = cudaMallocHost(&v->h_stage, stage_bytes)) != cudaSuccess) break;
     if ((e = cudaMallocHost(&v->h_out, out_floats * sizeof(float))) != cudaSuccess) break;

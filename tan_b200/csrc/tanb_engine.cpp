@@ -193,7 +193,7 @@ struct tanb_engine {
   EngLvlUpd* d_lupd = nullptr;
   float2* d_tw = nullptr;     // the block kernel's twiddles (2B entries)
   float2* d_tw_ir = nullptr;  // the IR transforms' (the register passes' table, 2B entries)
-  float2* d_run = nullptr;    // workspace of calls over several blocks (run_blocks)
+  float2* d_run = nullptr;    // workspace of calls over several blocks (engine_run_reserve)
   size_t run_bytes = 0;
   int tail_grid = 0;
   int sms = 148;  // SMs of the device
@@ -931,51 +931,45 @@ int32_t run_block(tanb_engine* e, const tanb::EngRows* rows) {
   return TANB_OK;
 }
 
-// Workspace of a launch sequence over nb blocks: every level's spectra in turn
-// (at most one level block more than the call's samples), one level after the
-// other. Allocated by the first such call and kept; false without memory for it.
-bool ensure_run(tanb_engine* e, const Session& s, int nb) {
+// Bytes of the workspace of a launch sequence over nb blocks: every level's
+// spectra in turn (at most one level block more than the call's samples).
+size_t run_space(const tanb_engine* e, const Session& s, int nb) {
   size_t per = 0;  // complex values per channel
   for (const LevelSpec& l : s.lv) {
     const size_t N = (size_t)1 << l.log2N, m = ((size_t)nb << e->log2B) / N + 1;
     per = std::max(per, m > 1 ? (m + 1) * N : N);
   }
-  const size_t need = per * e->max_channels * sizeof(float2);
-  if (need <= e->run_bytes) return true;
-  if (need > kRunMaxBytes) return false;
-  if (e->d_run && cudaStreamSynchronize(e->stream) != cudaSuccess) return false;
-  cudaFree(e->d_run);
-  e->d_run = nullptr;
-  e->run_bytes = 0;
-  if (cudaMalloc(&e->d_run, need) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return false;
-  }
-  e->run_bytes = need;
-  return true;
+  return per * e->max_channels * sizeof(float2);
+}
+
+// Blocks of a launch sequence over several blocks at most (tanb_engine_kernels.cu,
+// eng_run_*), 0 where the session takes none: non-uniform, FP32 spectra, at most
+// two partitions in the base level; within one period of the largest level and of
+// every level with work items, so that each of those has at most one head in it
+// and its partial rows are those of two level blocks (two parities).
+int run_blocks_most(const tanb_engine* e, const Session& s) {
+  if (e->spec != tanb::kSpecFP32 || s.lv.empty() || s.nitem) return 0;
+  // a level takes up to two level blocks more than the call's samples
+  size_t most = kRunMaxBytes / (sizeof(float2) * e->B * e->max_channels) / 3;
+  for (const LevelSpec& l : s.lv)
+    if (l.ngroup || &l == &s.lv.back()) most = std::min(most, (size_t)1 << (l.log2N - e->log2B));
+  return most >= kRunMinBlocks ? (int)most : 0;
 }
 
 // Blocks of the next launch sequence over several blocks of the engine's only
-// session (tanb_engine_kernels.cu, eng_run_*), of at most `nb`: 0 when the next
-// block has to go by itself (an update takes effect on it), -1 when all do.
-// Non-uniform, FP32 spectra, at most two partitions in the base level; a sequence
-// stays within one
-// period of the largest level and of every level with work items, so that each
-// of those has at most one head in it and its partial rows are those of two
-// level blocks (two parities).
+// session, of at most `nb`: 0 when the next block has to go by itself (an update
+// takes effect on it), -1 when all do.
 int run_blocks_fit(tanb_engine* e, const Session& s, size_t nb) {
-  if (e->spec != tanb::kSpecFP32 || s.lv.empty() || s.nitem || nb < kRunMinBlocks) return -1;
-  for (const LevelSpec& l : s.lv)
-    if (l.ngroup && (1u << (l.log2N - e->log2B)) < kRunMinBlocks) return -1;
+  const int most = run_blocks_most(e, s);
+  if (!most || nb < kRunMinBlocks) return -1;
   if (s.staged) return 0;
   for (int j = 0; j < s.C; ++j)
     if (e->h_chans[s.slot0 + j].pending) return 0;
+  const int fit = (int)std::min(nb, (size_t)most);
   const long long t0 = e->k_host << e->log2B;
-  size_t fit = nb;
   long long off = 0, reach = 0;
   for (const LevelSpec& l : s.lv) {
     const long long N = 1LL << l.log2N;
-    if (l.ngroup || &l == &s.lv.back()) fit = std::min(fit, (size_t)(N >> e->log2B));
     // a sample's sum takes the levels in order, those with a head for it in this
     // sequence before those whose rings hold it: where the latter begin has to
     // grow with the level
@@ -983,9 +977,7 @@ int run_blocks_fit(tanb_engine* e, const Session& s, size_t nb) {
     if (off < reach) return 0;
     reach = off;
   }
-  const size_t most = kRunMaxBytes / (sizeof(float2) * e->B * e->max_channels);  // blocks of workspace
-  fit = std::min(fit, most / 3);  // a level takes up to two level blocks more than the call's samples
-  return fit >= kRunMinBlocks && ensure_run(e, s, (int)fit) ? (int)fit : -1;
+  return run_space(e, s, fit) <= e->run_bytes ? fit : -1;
 }
 
 // One launch sequence over nb blocks (as run_blocks_fit allows) of the engine's
@@ -1070,6 +1062,21 @@ int32_t engine_process_rows(tanb_engine* e, const EngRows& rows) {
   ENG_CUDA(cudaSetDevice(e->ctx->device));
   if (e->sessions.empty()) return efail(TANB_WRONG_STATE, "no open sessions");
   return run_block(e, &rows);
+}
+
+size_t engine_run_reserve(tanb_engine* e, int32_t session) {
+  std::lock_guard<std::mutex> lock(e->mu);
+  auto it = e->sessions.find(session);
+  const int most = it == e->sessions.end() ? 0 : run_blocks_most(e, it->second);
+  if (!most || e->d_run || cudaSetDevice(e->ctx->device) != cudaSuccess) return 0;
+  const size_t need = run_space(e, it->second, most);
+  if (need > kRunMaxBytes) return 0;  // level blocks above the call's bound
+  if (cudaMalloc(&e->d_run, need) != cudaSuccess) {
+    (void)cudaGetLastError();
+    e->d_run = nullptr;
+    return 0;
+  }
+  return e->run_bytes = need;
 }
 
 int32_t engine_run_blocks(tanb_engine* e, int32_t session, const EngRows& rows, size_t nb, int* done) {

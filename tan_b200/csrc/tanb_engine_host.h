@@ -23,6 +23,9 @@ size_t engine_nu_session_bytes(int block, int spectrum, int channels, uint32_t i
                                const uint32_t* level_block, const uint32_t* level_parts);
 // One block with the given rows (direct launches on the audio stream).
 int32_t engine_process_rows(tanb_engine* e, const EngRows& rows);
+// Allocates the workspace of engine_run_blocks for the session and returns its
+// bytes (0: the session takes none, or no memory; its blocks then go one by one).
+size_t engine_run_reserve(tanb_engine* e, int32_t session);
 // Up to nb blocks of the engine's only session as one launch sequence, rows
 // holding the blocks back to back: *done of them (0: they have to go one by one).
 // Same samples as engine_process_rows bit for bit.
