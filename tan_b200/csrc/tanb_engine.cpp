@@ -966,22 +966,13 @@ int run_blocks_fit(tanb_engine* e, const Session& s, size_t nb) {
   for (int j = 0; j < s.C; ++j)
     if (e->h_chans[s.slot0 + j].pending) return 0;
   const int fit = (int)std::min(nb, (size_t)most);
-  const long long t0 = e->k_host << e->log2B;
-  long long off = 0, reach = 0;
-  for (const LevelSpec& l : s.lv) {
-    const long long N = 1LL << l.log2N;
-    // a sample's sum takes the levels in order, those with a head for it in this
-    // sequence before those whose rings hold it: where the latter begin has to
-    // grow with the level
-    off = l.off + t0 / N * N;
-    if (off < reach) return 0;
-    reach = off;
-  }
   return run_space(e, s, fit) <= e->run_bytes ? fit : -1;
 }
 
 // One launch sequence over nb blocks (as run_blocks_fit allows) of the engine's
-// only session: rows hold the blocks back to back. Caller holds mu.
+// only session: rows hold the blocks back to back. Every sample takes the levels in
+// order, from each one either what its ring holds or the head in this sequence that
+// covers it, as block by block. Caller holds mu.
 cudaError_t run_blocks(tanb_engine* e, Session& s, const tanb::EngRows& rows, int nb) {
   const int ns = (int)e->nslots_hwm;
   tanb::EngRunLevel p;

@@ -92,3 +92,22 @@ def test_many_blocks_rows_and_flags(tan_ctx, place, nulls):
     assert np.array_equal(stream(many, x, B, plan, events, f_many, place, nulls), y1)
     one.Release()
     many.Release()
+
+
+@pytest.mark.parametrize("B,levels", [(128, [(128, 2), (256, 1), (512, 1), (1024, 7), (2048, 1), (8192, 3)]),
+                                      (256, [(256, 2), (512, 1), (1024, 1), (2048, 7), (4096, 1), (16384, 2)])])
+def test_levels_that_grow_by_more_than_two(tan_ctx, B, levels):
+    """Calls that start where a small level's next output lies behind a larger
+    one's: the larger one's rings hold samples that the smaller one's heads of the
+    same call also add to."""
+    g = H.rng(780 + levels[-1][0])
+    C, L = 2, sum(b * k for b, k in levels)
+    plan = [9, 14, 6, 17, 5, 30, 11, 8, 23, 7, 13, 64, 19, 12]
+    n = sum(plan)
+    x = H.noise(g, C, n * B)
+    events = {0: H.irs(g, C, L), plan[0] + plan[1]: H.irs(g, C, L)}
+    one, many = make(tan_ctx, L, B, C, levels), make(tan_ctx, L, B, C, levels)
+    y1 = stream(one, x, B, [1] * n, events, {})
+    assert np.array_equal(stream(many, x, B, plan, events, {}), y1)
+    one.Release()
+    many.Release()
