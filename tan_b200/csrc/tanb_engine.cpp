@@ -196,7 +196,7 @@ struct tanb_engine {
   float2* d_run = nullptr;    // workspace of calls over several blocks (engine_run_reserve)
   size_t run_bytes = 0;
   int tail_grid = 0;
-  int sms = 148;  // SMs of the device
+  int sms = tanb::kSms;  // SMs of the device
   size_t nslots_hwm = 0, nitems_hwm = 0;
   // graphs of the host-buffer block, one per set of due level size classes,
   // each valid for the high-water marks in its key; executable graphs

@@ -1762,7 +1762,7 @@ cudaError_t lattrs_all() {
 // twiddles, few enough that every SM has several CTAs.
 int ir_grid(int parts, int nupd, int groups) {
   const long long ctas = ((long long)parts * nupd + groups - 1) / groups;  // at one partition per group
-  const int turns = (int)(ctas / (148 * 2) < 1 ? 1 : ctas / (148 * 2) > 4 ? 4 : ctas / (148 * 2));
+  const int turns = (int)(ctas / (kSms * 2) < 1 ? 1 : ctas / (kSms * 2) > 4 ? 4 : ctas / (kSms * 2));
   return (parts + groups * turns - 1) / (groups * turns);
 }
 
@@ -1817,7 +1817,7 @@ cudaError_t run_base_t(const EngChan* chans, int nslots, const EngRows& rows, co
   // shortest whose CTAs are all resident at 1024 threads per SM, at most 16 blocks
   // (256 channels x 128 blocks of 128: runs of 7 left 128 CTAs for a second wave,
   // 80 us; runs of 8 take 72)
-  const long long ctas = 148 * (1024 / FftShape<LOG2M>::T);
+  const long long ctas = kSms * (1024 / FftShape<LOG2M>::T);
   int run = 1;
   while (run < 16 && (long long)((nb + run - 1) / run) * nslots > ctas) ++run;
   eng_run_base_kernel<LOG2M><<<dim3((nb + run - 1) / run, nslots), FftShape<LOG2M>::T, 2 * (1 << LOG2M) * sizeof(float2),

@@ -70,6 +70,9 @@ struct ChanCtl {
 // Error codes a kernel writes to DevState::err.
 enum : int { kErrNone = 0, kErrBulkWaitTimeout = 1 };
 
+// SMs of the GPU that the launch rules are laid out for. Results do not depend on it.
+constexpr int kSms = 148;
+
 // Polls of an mbarrier before a bounded wait gives up (about a second).
 constexpr int kBulkWaitLimit = 1 << 20;
 
@@ -84,7 +87,7 @@ struct DevState {
   float2* H;      // IR spectra      [C][2 slots][P][B]
   float2* fdl;    // delay line      [C][P][B]  (slot (cur + i) mod P holds X_{k-i})
   float* prev;    // previous input  [C][B]     (overlap-save history)
-  float2* tail;   // tails           [C][2][B]  ([0]: active IR, [1]: pending IR)
+  float2* tail;   // tails           [C][3][B]  ([0], [1]: active IR, by block parity; [2]: pending IR)
   const float2* tw;  // twiddles of the B-point register transform (2B entries)
   int* err;       // device-visible error word (host-mapped); nonzero after a
                   // bounded wait in a kernel gave up (kErr* codes)

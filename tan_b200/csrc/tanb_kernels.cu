@@ -1242,7 +1242,7 @@ cudaError_t launch_ir_t(const DevState& s, const IrRows& ir, const int* chans, i
                         cudaStream_t st) {
   using R = RegGroups<LOG2M>;
   const long long groups = ((long long)s.P * nch + R::G - 1) / R::G;  // CTAs at one partition per group
-  const int iters = (int)std::max<long long>(1, std::min<long long>(kIrPartsPerGroup, groups / (148 * 2)));
+  const int iters = (int)std::max<long long>(1, std::min<long long>(kIrPartsPerGroup, groups / (kSms * 2)));
   const int gx = (s.P + R::G * iters - 1) / (R::G * iters);
   ir_spectrum_kernel<LOG2M><<<dim3(gx, nch), R::THREADS, R::SMEM, st>>>(s, ir, chans, ctl);
   return cudaGetLastError();
@@ -1273,13 +1273,13 @@ constexpr int kRunMax = 8;
 // partitions in series: a call of 12 blocks of 512 with 65536 taps takes 34 us with
 // run_mac_kernel and 61 with it at one channel, 58 and 74 at 32 channels (512
 // warps), 90 and 90 at 64 (1024 warps).
-constexpr int kRunLineWarps = 148 * 6;
+constexpr int kRunLineWarps = kSms * 6;
 
 template <int LOG2M>
 cudaError_t launch_run_t(const DevState& s, const BlockRef& d, const RunShape& r, cudaStream_t st,
                          const HeadSignal& sig) {
   using Sh = RegGroups<LOG2M>;
-  const int run = (int)std::max<long long>(1, std::min<long long>(kRunMax, (long long)s.C * r.nb / (Sh::G * 148LL * 2)));
+  const int run = (int)std::max<long long>(1, std::min<long long>(kRunMax, (long long)s.C * r.nb / ((long long)Sh::G * kSms * 2)));
   const dim3 gf((r.nb + Sh::G * run - 1) / (Sh::G * run), s.C);
   const int groups = (r.nb + 1 + kRunBlocks - 1) / kRunBlocks, per = (r.nb + 1 + groups - 1) / groups;
   const dim3 gm(s.B / kRunBins, s.C, groups), bm(kRunBins, kRunRows);

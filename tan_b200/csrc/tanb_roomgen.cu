@@ -358,12 +358,12 @@ int32_t tanb_room_response(tanb_room_generator* g, const tanb_room* room, const 
   if (smem <= tanb::kRoomTableBytes) {
     const int fast = a.cx >= a.cy && a.cx >= a.cz ? 0 : a.cy >= a.cz ? 1 : 2;
     const long long rows = images / (fast == 0 ? a.cx : fast == 1 ? a.cy : a.cz);
-    const unsigned blocks = (unsigned)std::max<long long>(1, std::min<long long>((rows + 7) / 8, 148 * 4));
+    const unsigned blocks = (unsigned)std::max<long long>(1, std::min<long long>((rows + 7) / 8, tanb::kSms * 4));
     auto kernel = fast == 0 ? tanb::room_images_kernel<0> : fast == 1 ? tanb::room_images_kernel<1>
                                                                       : tanb::room_images_kernel<2>;
     kernel<<<blocks, 256, smem, st>>>(a, g->acc, (size_t)g->max_length);
   } else {
-    const unsigned blocks = (unsigned)std::max<long long>(1, std::min<long long>((images + 255) / 256, 16LL * 148));
+    const unsigned blocks = (unsigned)std::max<long long>(1, std::min<long long>((images + 255) / 256, 16LL * tanb::kSms));
     tanb::room_images_any_kernel<<<blocks, 256, 0, st>>>(a, g->acc, (size_t)g->max_length, images);
   }
   const unsigned fill = (unsigned)std::min(1024, (length + 255) / 256);
