@@ -3,10 +3,10 @@
 //   ir_spectrum_kernel  R2C of the IR partitions [h_i, 0^B], one per group of
 //                       threads (tanb_fft_reg.cuh)
 //   head_kernel         one CTA per channel: R2C of [x_{k-1}, x_k] into the
-//                       delay line, MAC with partition 0, add the precomputed
-//                       tail, C2R, output the upper B samples (crossfading old
-//                       and new IR on a swap block)
-//   tail_kernel         streaming MAC over partitions 1..P-1 for the next block
+//                       delay line, MAC with partitions 0 and 1, add the
+//                       precomputed tail, C2R, output the upper B samples
+//                       (crossfading old and new IR on a swap block)
+//   tail_kernel         streaming MAC over partitions 2..P-1 for the next block
 //                       (the HBM-bound kernel): float4 loads of the IR spectrum
 //                       and the delay line, partitions split across warps and
 //                       reduced in shared memory in a fixed order
@@ -246,8 +246,8 @@ __device__ __forceinline__ void mix_epilogue(const MixEpi& epi, int c) {
 // any of them is used, so the block waits for one memory round trip: the frame
 // (caller rows may sit in pinned host memory, the longest latency), the
 // twiddles, the tail, partitions 0 and 1 and X_{k-1}. The transforms run as
-// register passes (tanb_fft_reg.cuh): a block of 512 meets six barriers, where
-// radix-4 stages in shared memory met 24.
+// register passes (tanb_fft_reg.cuh): a block of 512 meets seven barriers (one
+// more where it signals the host), where radix-4 stages in shared memory met 24.
 template <int LOG2M>
 struct HeadShape {
   using F = RegFft<LOG2M>;
