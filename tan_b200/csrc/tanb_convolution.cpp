@@ -878,7 +878,7 @@ int32_t run_blocks(tanb_convolution* v, const RunCall& q, int nb, int* done, dou
   r.X = reinterpret_cast<float2*>(v->d_ir);
   r.Y = r.X + (size_t)C * nb * B;
   r.nb = nb;
-  r.sy = v->tiling.sy;
+  r.sy = v->tiling.kind == 0 ? v->tiling.sy : 1;  // a bulk pipeline sums in one chunk
   r.cur = v->cur;
   r.trow = (int)((v->blocks + nb) & 1);
   tanb::HeadSignal sig;
@@ -963,13 +963,16 @@ int32_t process_common(tanb_convolution* v, Mem in_mem, const float* const* in, 
   double t_stage = 0, t_launch = 0, t_wait = 0, t_copy = 0;
   // Several blocks in one launch sequence (launch_run): no channel may change
   // state inside the call, which only STOP_INPUT makes happen (every channel
-  // then runs, and a flush can only fall on the call's first block), and the
-  // tail must sum its partitions in the register-load kernel's chunks. A swap
-  // takes its block through the one-block path first.
+  // then runs, and a flush can only fall on the call's first block). The sums take
+  // the chunks of the tail tiling, whichever it is; one that the block size does not
+  // allow fails as block by block. A swap takes its block through the one-block path
+  // first. (Tilings of 4 or 2 chunks and bulk pipelines, 32 blocks of 256, 16
+  // channels of 24000 taps: 263, 394 and 656 us block by block, 26, 33 and 44 so.)
   const size_t from = in_mem == Mem::Host && !direct_in && (size_t)C * B * sizeof(float) >= kRunStagedBytes
                           ? kRunStagedMinBlocks
                           : kRunMinBlocks;
-  bool many = nblocks >= from && !pcm && !v->finalize_mode && v->tiling.kind == 0 && v->tiling.sy >= 8;
+  bool many = nblocks >= from && !pcm && !v->finalize_mode &&
+              (v->tiling.kind == 0 || B % (2 * v->tiling.ux) == 0);
   for (int c = 0; many && flags && c < C; ++c) many = (flags[c] & kStopInput) == 0;
   // all inputs are read before any output is written: as block by block where the
   // rows are apart or in place

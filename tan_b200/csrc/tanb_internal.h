@@ -238,8 +238,8 @@ cudaError_t launch_tail(const DevState& s, const BlockRef& d, int which, int cur
 // One call over nb blocks of every channel: all channels run, none swaps, the
 // descriptor's rows hold the nb blocks back to back. X and Y are workspaces of
 // [C][nb][B] float2; `cur` is the delay-line slot of the newest spectrum before
-// the call, `sy` the partition chunks of the object's tail tiling (kind 0, at
-// least 8), `trow` the tail row of the block after the call.
+// the call, `sy` the partition chunks of the object's tail tiling (1: a bulk
+// pipeline's), `trow` the tail row of the block after the call.
 struct RunShape {
   float2* X = nullptr;
   float2* Y = nullptr;
