@@ -19,7 +19,8 @@ ours (default):
          tail kernel; p50/p99/p99.9 of the per-block latency (Process return).
 reference: the oracle's C++ restatement of TAN's CPU path on all host cores.
 Under torchrun each rank runs its own 64-channel replica (weak scaling, no
-data-path collective); rank 0 prints one JSON line.
+data-path collective); rank 0 prints one JSON line, a few KB long (--record FILE
+keeps the whole record that it is taken from).
 """
 from __future__ import annotations
 
@@ -54,6 +55,7 @@ def parse():
     p.add_argument("--warmup", type=int, default=32)
     p.add_argument("--impl", choices=["ours", "reference"], default="ours")
     p.add_argument("--cpu-sample-s", type=float, default=10.0)
+    p.add_argument("--record", default="", help="file for the whole record, per-channel errors included")
     p.add_argument("--no-cpu-baseline", action="store_true")
     p.add_argument("--no-capacity", action="store_true")
     p.add_argument("--no-configs", action="store_true",
@@ -327,6 +329,33 @@ def run_reference(args):
         "e2e": {"value": value, "unit": "GSamples/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
     }
     print(json.dumps(line), flush=True)
+
+
+# Of the other configurations' records the line keeps these figures.
+CONFIG_KEYS = {"p99", "max", "deadline_misses", "deadline_misses_host", "nonfinite_channels"}
+
+
+def stdout_line(record):
+    """The JSON line's form of a record: every key and figure of the measurement itself, without
+    explanations and lists per channel or per grid, the configuration as it is, and of the other
+    configurations the key figures. Floats to 7 digits."""
+    def figures(v, keys):
+        if isinstance(v, dict):
+            d = {k: figures(x, keys) for k, x in v.items() if isinstance(x, dict) or k in keys}
+            return {k: x for k, x in d.items() if x != {}}
+        return plain(v)
+
+    def plain(v):
+        if isinstance(v, dict):
+            return {k: plain(x) for k, x in v.items() if k not in ("what", "grids_us", "fit") and not k.endswith("_what")}
+        if isinstance(v, list):
+            return [plain(x) for x in v[:8]]
+        return float(f"{v:.7g}") if isinstance(v, float) else v
+
+    line = {k: v if k == "config" else plain(v) for k, v in record.items() if k != "configs"}
+    if record.get("configs"):
+        line["configs"] = figures(record["configs"], CONFIG_KEYS)
+    return line
 
 
 def read_traffic(name="tail_kernel_64ch_b512_ir65536.txt"):
@@ -767,7 +796,10 @@ def run_ours(args):
             line["configs"] = configs
         if sharded:
             line["serving_sharded"] = sharded
-        print(json.dumps(line), flush=True)
+        if args.record:
+            with open(args.record, "w") as f:
+                json.dump(line, f)
+        print(json.dumps(stdout_line(line)), flush=True)
     ctx.Release()
     if pg:
         pg.barrier()
