@@ -930,9 +930,11 @@ __device__ __forceinline__ void run_mac_body(const DevState& s, const D& desc, c
 // CTA meets, so that group g's row for partition i is q = (G - 1 - g) NB + NB - 3
 // + i. The inner loop is one copy of code for every bin, stage and chunk: the
 // kernel runs for some twenty stages, and with the loop doubled for the packed
-// bin 0 and for chunk ends it waited for instructions (64 us at 64 channels of
-// 128 partitions of 512 and 32 blocks; with each warp loading its own rows into
-// registers 86 us).
+// bin 0 and for chunk ends it waited for instructions. At 64 channels of 128
+// partitions of 512 and 32 blocks a launch takes 79 us alone: 512 CTAs of six warps
+// are 0.86 of a wave at four per SM, and their dependent FP32 operations and the
+// barriers between stages keep the issue slots 65% busy. (The width of six outputs
+// spills 64 bytes a thread, 128 with device tables, at the 80 registers that allows.)
 constexpr int kLineStage = 8, kLineDepth = 2, kLineGroups = 6, kLineBins = 64, kLineXRows = 64, kLineHRows = 32;
 
 // acc + x h for two bins; (h0, nh0, g0, k0): of the first bin, h.x, -h.y and
