@@ -902,6 +902,7 @@ int32_t run_blocks(tanb_convolution* v, const RunCall& q, int nb, int* done, dou
     if (wait_heads(v, sig) != TANB_OK) return TANB_FAIL;
     *t_wait += std::chrono::duration<double, std::micro>(std::chrono::steady_clock::now() - t0).count();
     v->staging_busy = false;
+    if (*v->h_err != tanb::kErrNone) return fail(TANB_FAIL, "device wait timed out (error %d)", *v->h_err);
     if (stage_out)
       for (int c = 0; c < C; ++c)
         if (q.out[c]) std::memcpy(q.out[c] + off, hout + c * row, row * sizeof(float));

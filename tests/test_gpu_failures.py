@@ -75,6 +75,24 @@ def test_bulk_wait_timeout_is_reported_and_a_fresh_object_works(tan_ctx):
     assert H.rel_err(y, yr) < TOL
 
 
+def test_bulk_wait_timeout_is_reported_by_calls_over_several_blocks(tan_ctx):
+    """The recorded error also fails the launch sequence of a several-block call,
+    which starts no bulk pipeline itself."""
+    g = H.rng(20261203 + 43)
+    C, B, L = 2, 256, 20000
+    conv = cv.TANConvolution(tan_ctx)
+    assert conv.Init(cv.TAN_CONVOLUTION_METHOD_FFT_PARTITIONED_UNIFORM, L, B, C) == 0
+    assert conv.tiling(bulk_tiling_index(tan_ctx, B))[0] == cv.AMF_OK
+    assert cv.lib().tanb_convolution_set_wait_limit(conv._h, 0) == cv.AMF_OK
+    assert conv.UpdateResponseTD(H.irs(g, C, L), L) == 0
+    x = H.noise(g, C, 8 * B)
+    rc1, _ = conv.Process(np.ascontiguousarray(x[:, :B]), np.zeros((C, B), np.float32), B)
+    conv.Synchronize()
+    rc, _ = conv.Process(x, np.zeros_like(x), 8 * B)
+    assert rc == cv.AMF_FAIL and "timed out" in cv.last_error()
+    conv.Release()
+
+
 def alone(ctx, x, B, events):
     C = x.shape[0]
     L = max(ir.shape[1] for ir in events.values())
